@@ -159,6 +159,7 @@ struct Level {
     std::vector<int> ext;    // exterior port -> matrix index
     std::vector<int> seams;  // 6 ints per seam candidate
     int nseams = 0;
+    int cap_inc = 0;  // most seam candidates that touch one child
     DevBuf<int> d_ext, d_seams, d_ext_inv;
     DevBuf<uint16_t> mat;
     DevBuf<uint8_t> kflag;
@@ -276,7 +277,11 @@ struct UpdateArena {
     PoolBuf<uint16_t> panel;
     PoolBuf<uint8_t> pflags;
     HostBuf stage, rb;
-    cudaEvent_t ev_cnt = nullptr;  // an opening level's pivot counts reached the host
+    cudaEvent_t ev_cnt = nullptr;  // an opening level's pivot counts / a build's seam counts reached the host
+    // node builds: the staged node lists with the seam counts, and the
+    // scratch of the launches (hb::node_build_layout)
+    HostBuf nstage;
+    PoolBuf<unsigned char> nlist, nscratch;
     int open_grid = 0;             // CTAs of the persistent opening kernel
     // phase time stamps of the last device-driven opening launch (device,
     // and where they are in the arena)
@@ -289,6 +294,9 @@ struct UpdateArena {
         pflags.release();
         stage.release();
         rb.release();
+        nstage.release();
+        nlist.release();
+        nscratch.release();
         if (ev_cnt) cudaEventDestroy(ev_cnt);
         ev_cnt = nullptr;
         trace_valid = 0;
@@ -435,6 +443,12 @@ void make_levels(htrip_index* h) {
             }
         }
         Lv.nseams = (int)Lv.seams.size() / 6;
+        std::vector<int> touch((size_t)g * g, 0);
+        for (int s = 0; s < Lv.nseams; ++s) {
+            ++touch[Lv.seams[6 * s] / Lv.nP];
+            ++touch[Lv.seams[6 * s + 1] / Lv.nP];
+        }
+        Lv.cap_inc = *std::max_element(touch.begin(), touch.end());
         cs *= g;
     }
 }
@@ -495,44 +509,10 @@ std::vector<int> weighted_leaves(const htrip_index* h, const std::vector<int>& l
     return out;
 }
 
-void close_matrices(htrip_index* h, Level& Lv, const std::vector<int>& act);
-
-// Leaf matrices of the listed leaves (all when `leaves` is null) from the
-// passability mirror: bit-parallel BFS, then, for leaves with non-unit
-// weights, the weighted adjacency closed over its passable cells.
-void build_leaves(htrip_index* h, const std::vector<int>* leaves, const uint8_t* obs, int rows, int cols) {
-    cudaStream_t st = h->stream;
-    Level& L0 = h->L[0];
-    DevBuf<int> list;
-    std::vector<int> all;
-    if (!leaves) {
-        all.resize(L0.nnodes);
-        std::iota(all.begin(), all.end(), 0);
-        hb::launch_leaf_bfs(h->pass.p, h->S, h->b, h->leaves_x, L0.nnodes, L0.ms(), st);
-    } else if (!leaves->empty()) {
-        list.reserve(leaves->size());
-        ck(cudaMemcpyAsync(list.p, leaves->data(), leaves->size() * sizeof(int), cudaMemcpyHostToDevice, st), "list");
-        hb::launch_leaf_bfs(h->pass.p, h->S, h->b, h->leaves_x, (int)leaves->size(), L0.ms(), st, list.p);
-    }
-    ck(cudaGetLastError(), "leaf bfs");
-    const std::vector<int> wl = weighted_leaves(h, leaves ? *leaves : all, obs, rows, cols);
-    if (!wl.empty()) {
-        DevBuf<int> wlist;
-        wlist.reserve(wl.size());
-        ck(cudaMemcpyAsync(wlist.p, wl.data(), wl.size() * sizeof(int), cudaMemcpyHostToDevice, st), "list");
-        hb::launch_leaf_weight_init(h->pass.p, h->wts.p, h->S, h->b, h->leaves_x, (int)wl.size(), L0.ms(),
-                                    L0.kflag.p, wlist.p, st);
-        ck(cudaGetLastError(), "weighted leaf init");
-        close_matrices(h, L0, wl);  // synchronises before returning
-        wlist.release();
-    }
-    ck(cudaStreamSynchronize(st), "leaf sync");
-    list.release();
-}
-
 void alloc_levels(htrip_index* h) {
     for (auto& Lv : h->L) {
         Lv.mat.reserve((size_t)Lv.nnodes * Lv.NP * Lv.NP);
+        if (Lv.lvl >= 1) hb::launch_pad_fill(Lv.ms(), Lv.nnodes, h->stream);  // node builds write the logical part only
         Lv.d_ext.reserve(std::max(1, Lv.nExt));
         ck(cudaMemcpyAsync(Lv.d_ext.p, Lv.ext.data(), Lv.nExt * sizeof(int), cudaMemcpyHostToDevice, h->stream), "ext");
         if (Lv.nseams) {
@@ -644,6 +624,156 @@ void close_matrices(htrip_index* h, Level& Lv, const std::vector<int>& act) {
 }
 
 // ---------------------------------------------------------------------------
+// Matrices from the grid: leaves from the passability mirror (and weights),
+// nodes from their children and seams, level by level.
+// ---------------------------------------------------------------------------
+// What a build covers.  all: every leaf and node.  Otherwise leaves and, per
+// level l >= 1, nodes[l]; with `track` a node above level 1 is built only
+// if the exterior block of a built child changed (decided on the device), and
+// parent[l][i] is the place of nodes[l][i]'s parent in nodes[l + 1].
+struct BuildSet {
+    bool all = false, track = false;
+    std::vector<int> leaves;
+    std::vector<std::vector<int>> nodes, parent;
+};
+
+// Scratch of one launch of the general node build (bounds the nodes a launch takes).
+constexpr size_t kNodeScratch = (size_t)192 << 20;
+
+// Everything is issued on the index's stream; the host waits once, early, for the
+// levels' seam counts (they set the number of closure rounds), while the
+// leaf kernel runs.  Not waited for at the end.
+void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int rows, int cols) {
+    cudaStream_t st = h->stream;
+    UpdateArena& A = h->u;
+    const int H = h->H;
+    auto count = [&](int l) {
+        return l == 0 ? (bs.all ? h->L[0].nnodes : (int)bs.leaves.size())
+                      : (bs.all ? h->L[l].nnodes : (int)bs.nodes[l].size());
+    };
+    std::vector<int> every;
+    if (bs.all && !h->wgrid.empty()) {
+        every.resize(h->L[0].nnodes);
+        std::iota(every.begin(), every.end(), 0);
+    }
+    const std::vector<int> wl = weighted_leaves(h, bs.all ? every : bs.leaves, obs, rows, cols);
+    // one upload: {seam counts | leaves, weighted leaves, node lists, parents, active flags}
+    size_t bytes = 0;
+    auto take = [&](size_t n) {
+        const size_t o = bytes;
+        bytes += align256(std::max<size_t>(n, 1));
+        return o;
+    };
+    const size_t o_most = take((H + 1) * sizeof(int));
+    const size_t o_leaves = take((bs.all ? 0 : bs.leaves.size()) * sizeof(int)), o_wl = take(wl.size() * sizeof(int));
+    std::vector<size_t> o_list(H + 1), o_parent(H + 1), o_active(H + 1);
+    if (!bs.all)
+        for (int l = 1; l <= H; ++l) {
+            o_list[l] = take(bs.nodes[l].size() * sizeof(int));
+            if (!bs.track) continue;
+            o_parent[l] = take(bs.nodes[l].size() * sizeof(int));
+            o_active[l] = take(bs.nodes[l].size());
+        }
+    A.nstage.reserve(bytes);
+    A.nlist.reserve(bytes, st);
+    unsigned char *hs = A.nstage.p, *ds = A.nlist.p;
+    std::memset(hs, 0, bytes);
+    auto put = [&](size_t o, const std::vector<int>& v) { std::memcpy(hs + o, v.data(), v.size() * sizeof(int)); };
+    put(o_wl, wl);
+    if (!bs.all) {
+        put(o_leaves, bs.leaves);
+        for (int l = 1; l <= H; ++l) {
+            put(o_list[l], bs.nodes[l]);
+            if (!bs.track) continue;
+            if (l < H) put(o_parent[l], bs.parent[l]);
+            if (l == 1) std::memset(hs + o_active[1], 1, bs.nodes[1].size());
+        }
+    }
+    ck(cudaMemcpyAsync(ds, hs, bytes, cudaMemcpyHostToDevice, st), "build lists");
+    std::vector<hb::NodeBuild> nb(H + 1);
+    bool wait = false;
+    for (int l = 1; l <= H; ++l) {
+        Level& Lv = h->L[l];
+        Level& Lc = h->L[l - 1];
+        hb::NodeBuild& P = nb[l];
+        P = hb::NodeBuild{};
+        P.N = Lv.ms();
+        P.C = Lc.ms();
+        P.cext = Lc.d_ext.p;
+        P.isext = Lv.d_isext.p;
+        P.nP = Lv.nP;
+        P.g = h->g;
+        P.nodes_x = Lv.nodes_x;
+        P.child_nodes_x = Lc.nodes_x;
+        P.side = Lv.side;
+        P.S = h->S;
+        P.seams = Lv.d_seams.p;
+        P.n_seams = Lv.nseams;
+        P.capI = Lv.cap_inc;
+        P.pass = h->pass.p;
+        P.wts = h->wts.p;
+        if (!bs.all) {
+            P.list = reinterpret_cast<const int*>(ds + o_list[l]);
+            if (bs.track) {
+                P.active = ds + o_active[l];
+                if (l < H) {
+                    P.parent = reinterpret_cast<const int*>(ds + o_parent[l]);
+                    P.changed = ds + o_active[l + 1];
+                }
+            }
+        }
+        if (count(l) && !hb::node_build_small(P)) {
+            hb::launch_seam_count(P, count(l), reinterpret_cast<int*>(ds + o_most) + l, st);
+            wait = true;
+        }
+    }
+    ck(cudaGetLastError(), "seam counts");
+    if (wait) {
+        ck(cudaMemcpyAsync(hs + o_most, ds + o_most, (H + 1) * sizeof(int), cudaMemcpyDeviceToHost, st), "seam counts");
+        if (!A.ev_cnt) ck(cudaEventCreateWithFlags(&A.ev_cnt, cudaEventDisableTiming), "event");
+        ck(cudaEventRecord(A.ev_cnt, st), "seam counts");
+    }
+    // leaves: bit-parallel BFS, then, for leaves with non-unit weights, the
+    // weighted adjacency closed over its passable cells
+    if (count(0))
+        hb::launch_leaf_bfs(h->pass.p, h->S, h->b, h->leaves_x, count(0), h->L[0].ms(), st,
+                            bs.all ? nullptr : reinterpret_cast<const int*>(ds + o_leaves));
+    ck(cudaGetLastError(), "leaf bfs");
+    if (wait) ck(cudaEventSynchronize(A.ev_cnt), "seam counts");
+    if (!wl.empty()) {
+        hb::launch_leaf_weight_init(h->pass.p, h->wts.p, h->S, h->b, h->leaves_x, (int)wl.size(), h->L[0].ms(),
+                                    h->L[0].kflag.p, reinterpret_cast<const int*>(ds + o_wl), st);
+        ck(cudaGetLastError(), "weighted leaf init");
+        close_matrices(h, h->L[0], wl);
+    }
+    const int* most = reinterpret_cast<const int*>(hs + o_most);
+    size_t scratch = 0;
+    std::vector<int> chunk(H + 1, 0);
+    for (int l = 1; l <= H; ++l) {
+        if (!count(l)) continue;
+        chunk[l] = count(l);
+        if (hb::node_build_small(nb[l])) continue;
+        hb::NodeBuild P = nb[l];
+        const size_t per = hb::node_build_layout(P, 1, nullptr);
+        chunk[l] = (int)std::min<size_t>({(size_t)count(l), std::max<size_t>(1, kNodeScratch / per), (size_t)65535});
+        scratch = std::max(scratch, hb::node_build_layout(P, chunk[l], nullptr));
+    }
+    if (scratch) A.nscratch.reserve(scratch, st);
+    for (int l = 1; l <= H; ++l)
+        for (int c0 = 0; c0 < count(l); c0 += chunk[l]) {
+            hb::NodeBuild P = nb[l];
+            const int n = std::min(chunk[l], count(l) - c0);
+            P.first = c0;
+            if (P.list) P.list += c0;
+            if (P.active) P.active += c0;
+            if (P.parent) P.parent += c0;
+            if (!hb::node_build_small(P)) hb::node_build_layout(P, n, A.nscratch.p);
+            hb::launch_node_build(P, n, most[l], st);
+            ck(cudaGetLastError(), "node build");
+        }
+}
+
+// ---------------------------------------------------------------------------
 // Build (reference MinPlusOracle::build, minplus_oracle.cpp:48-137)
 // ---------------------------------------------------------------------------
 void do_build(htrip_index* h, const uint8_t* observed, int rows, int cols) {
@@ -672,19 +802,9 @@ void do_build(htrip_index* h, const uint8_t* observed, int rows, int cols) {
     h->pass.reserve(pass.size());
     ck(cudaMemcpyAsync(h->pass.p, pass.data(), pass.size(), cudaMemcpyHostToDevice, st), "pass");
     upload_weights(h);
-    build_leaves(h, nullptr, observed, rows, cols);
-    for (int l = 1; l <= H; ++l) {
-        Level& Lv = h->L[l];
-        Level& Lc = h->L[l - 1];
-        hb::launch_node_init(Lv.ms(), Lc.ms(), Lc.d_ext.p, Lv.nP, g, Lv.nodes_x, Lc.nodes_x, Lv.nnodes, st);
-        ck(cudaGetLastError(), "node init");
-        hb::launch_seams_build(Lv.ms(), Lv.d_seams.p, Lv.nseams, h->pass.p, S, Lv.side, Lv.nodes_x, Lv.nnodes,
-                               Lv.kflag.p, st, nullptr, h->wts.p);
-        ck(cudaGetLastError(), "seams build");
-        std::vector<int> act(Lv.nnodes);
-        std::iota(act.begin(), act.end(), 0);
-        close_matrices(h, Lv, act);
-    }
+    BuildSet bs;
+    bs.all = true;
+    build_matrices(h, bs, observed, rows, cols);
     ck(cudaStreamSynchronize(st), "build sync");
     h->built = true;
     h->epoch++;
@@ -751,27 +871,13 @@ void do_lift_root(htrip_index* h, const uint8_t* observed, int rows, int cols) {
                 if (tx >= old_nodes_x || ty >= old_nodes_x) v.push_back(ty * nodes_x + tx);
         return v;
     };
-    DevBuf<int> list;
-    {
-        const std::vector<int> nl = fresh(h->L[0].nodes_x, old_S / b);
-        build_leaves(h, &nl, observed, rows, cols);
-    }
-    for (int l = 1; l <= h->H; ++l) {
-        Level& Lv = h->L[l];
-        Level& Lc = h->L[l - 1];
-        const std::vector<int> nn = l < h->H ? fresh(Lv.nodes_x, old_S / Lv.side) : std::vector<int>{0};
-        list.reserve(nn.size());
-        ck(cudaMemcpyAsync(list.p, nn.data(), nn.size() * sizeof(int), cudaMemcpyHostToDevice, st), "list");
-        hb::launch_node_init(Lv.ms(), Lc.ms(), Lc.d_ext.p, Lv.nP, g, Lv.nodes_x, Lc.nodes_x, (int)nn.size(), st,
-                             list.p);
-        ck(cudaGetLastError(), "node init");
-        hb::launch_seams_build(Lv.ms(), Lv.d_seams.p, Lv.nseams, h->pass.p, S, Lv.side, Lv.nodes_x, (int)nn.size(),
-                               Lv.kflag.p, st, list.p, h->wts.p);
-        ck(cudaGetLastError(), "seams build");
-        close_matrices(h, Lv, nn);
-        ck(cudaStreamSynchronize(st), "sync");
-    }
-    list.release();
+    BuildSet bs;
+    bs.leaves = fresh(h->L[0].nodes_x, old_S / b);
+    bs.nodes.resize(h->H + 1);
+    for (int l = 1; l <= h->H; ++l)
+        bs.nodes[l] = l < h->H ? fresh(h->L[l].nodes_x, old_S / h->L[l].side) : std::vector<int>{0};
+    build_matrices(h, bs, observed, rows, cols);
+    ck(cudaStreamSynchronize(st), "root growth");
     h->epoch++;
 }
 
@@ -805,59 +911,30 @@ void do_rebuild_leaves(htrip_index* h, const std::vector<int>& leaves_in, const 
     for (int r = 0; r < std::min(rows, S); ++r)
         for (int c = 0; c < std::min(cols, S); ++c) pass[(size_t)r * S + c] = observed[(size_t)r * cols + c] == 1;
     ck(cudaMemcpyAsync(h->pass.p, pass.data(), pass.size(), cudaMemcpyHostToDevice, st), "pass");
-    DevBuf<int> list;
-    DevBuf<hb::Slot> slots;
-    DevBuf<uint8_t> changed;
-    build_leaves(h, &cur, observed, rows, cols);
-    for (int l = 1; l <= h->H && !cur.empty(); ++l) {
-        Level& Lv = h->L[l];
-        Level& Lc = h->L[l - 1];
-        std::vector<int> parents;
-        std::vector<uint8_t> seen(Lv.nnodes, 0);
+    // every ancestor of a listed leaf, per level; the device skips those that
+    // `track` leaves unchanged
+    BuildSet bs;
+    bs.track = !propagate_all;
+    bs.leaves = cur;
+    bs.nodes.resize(h->H + 1);
+    bs.parent.resize(h->H + 1);
+    for (int l = 1; l <= h->H; ++l) {
+        const Level& Lv = h->L[l];
+        const Level& Lc = h->L[l - 1];
+        std::vector<int> at(Lv.nnodes, -1), place;
         for (int c : cur) {
             const int p = (c / Lc.nodes_x / g) * Lv.nodes_x + (c % Lc.nodes_x) / g;
-            if (!seen[p]) { seen[p] = 1; parents.push_back(p); }
+            if (at[p] < 0) {
+                at[p] = (int)bs.nodes[l].size();
+                bs.nodes[l].push_back(p);
+            }
+            place.push_back(at[p]);
         }
-        const int n = (int)parents.size();
-        const bool track = !propagate_all && l < h->H;  // does the next level depend on S_U changes?
-        std::vector<hb::Slot> hs;
-        if (track) {
-            hs.resize(n);
-            for (int i = 0; i < n; ++i) hs[i] = level_slot(Lv, nullptr, parents[i], 0, 0);
-            slots.reserve(n);
-            ck(cudaMemcpyAsync(slots.p, hs.data(), n * sizeof(hb::Slot), cudaMemcpyHostToDevice, st), "slots");
-            h->u.snap.reserve((size_t)n * Lv.nExt * Lv.nExt);
-            hb::launch_ext_snapshot(slots.p, n, Lv.d_ext.p, Lv.nExt, Lv.NP, h->u.snap.p, st);
-            ck(cudaGetLastError(), "snapshot");
-        }
-        list.reserve(n);
-        ck(cudaMemcpyAsync(list.p, parents.data(), n * sizeof(int), cudaMemcpyHostToDevice, st), "list");
-        hb::launch_node_init(Lv.ms(), Lc.ms(), Lc.d_ext.p, Lv.nP, g, Lv.nodes_x, Lc.nodes_x, n, st, list.p);
-        ck(cudaGetLastError(), "node init");
-        hb::launch_seams_build(Lv.ms(), Lv.d_seams.p, Lv.nseams, h->pass.p, S, Lv.side, Lv.nodes_x, n, Lv.kflag.p,
-                               st, list.p, h->wts.p);
-        ck(cudaGetLastError(), "seams build");
-        close_matrices(h, Lv, parents);
-        if (track) {
-            changed.reserve(n);
-            ck(cudaMemsetAsync(changed.p, 0, n, st), "changed");
-            hb::launch_ext_compare(slots.p, n, Lv.d_ext.p, Lv.nExt, Lv.NP, h->u.snap.p, changed.p, g, st, 1);
-            ck(cudaGetLastError(), "compare");
-            std::vector<uint8_t> ch(n);
-            ck(cudaMemcpyAsync(ch.data(), changed.p, n, cudaMemcpyDeviceToHost, st), "changed d2h");
-            ck(cudaStreamSynchronize(st), "sync");
-            std::vector<int> next;
-            for (int i = 0; i < n; ++i)
-                if (ch[i]) next.push_back(parents[i]);
-            cur = std::move(next);
-        } else {
-            ck(cudaStreamSynchronize(st), "sync");
-            cur = std::move(parents);
-        }
+        bs.parent[l - 1] = std::move(place);
+        cur = bs.nodes[l];
     }
-    list.release();
-    slots.release();
-    changed.release();
+    build_matrices(h, bs, observed, rows, cols);
+    ck(cudaStreamSynchronize(st), "rebuild");
 }
 
 // ---------------------------------------------------------------------------
@@ -3414,6 +3491,7 @@ htrip_status htrip_memory_bytes(const htrip_index* h, uint64_t* reference_bytes,
         for (const auto& Lv : h->L)
             dev += (Lv.mat.n + Lv.klist.n * 2 + Lv.kcnt.n * 2) * sizeof(uint16_t) + Lv.kflag.n + Lv.dec.n +
                    (Lv.d_ext.n + Lv.d_seams.n) * sizeof(int);
+        dev += h->u.nlist.n + h->u.nscratch.n;
         dev += h->pass.n + h->u.dev.n + h->u.snap.n * 2 + h->u.panel.n * 2 + h->u.pflags.n + h->q.dev.n +
                h->wts.n * sizeof(uint16_t);
     }

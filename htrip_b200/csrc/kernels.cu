@@ -83,66 +83,6 @@ leaf_bfs_kernel(const uint8_t* __restrict__ pass, int S, int b, int leaves_x, Ma
 }
 
 // ---------------------------------------------------------------------------
-// Node initial D_U (internal_node.cpp:98-145): entry (i, j) of node n is the
-// child summary S_q[p][p'] when i = q*nP + p and j = q*nP + p' lie in the
-// same child block q, INF otherwise (and in the padding).  S_q is the child
-// matrix restricted to its exterior ports: child[ext[p]][ext[p']].
-// ---------------------------------------------------------------------------
-__global__ void node_init_kernel(MatSet N, MatSet Cm, const int* __restrict__ cext, int nP, int g,
-                                 int nodes_x, int child_nodes_x, const int* __restrict__ list, int y0) {
-    const int node = list ? list[y0 + blockIdx.y] : y0 + blockIdx.y;
-    const int NP = N.NP, nV = N.n;
-    const size_t chunk = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // 8 entries
-    const size_t per_row = NP / 8;
-    if (chunk >= (size_t)NP * per_row) return;
-    const int i = (int)(chunk / per_row);
-    const int j0 = (int)(chunk % per_row) * 8;
-    uint16_t v[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) v[t] = INF;
-    if (i < nV) {
-        const int q = i / nP, p = i - q * nP;
-        const int tx = node % nodes_x, ty = node / nodes_x;
-        const int cx = q % g, cy = q / g;
-        const int child = (ty * g + cy) * child_nodes_x + (tx * g + cx);
-        const uint16_t* crow = mat_ptr(Cm, child) + (size_t)cext[p] * Cm.NP;
-        const int lo = q * nP, hi = lo + nP;
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            const int j = j0 + t;
-            if (j >= lo && j < hi) v[t] = crow[cext[j - lo]];
-        }
-    }
-    uint4 o;
-    o.x = v[0] | ((uint32_t)v[1] << 16);
-    o.y = v[2] | ((uint32_t)v[3] << 16);
-    o.z = v[4] | ((uint32_t)v[5] << 16);
-    o.w = v[6] | ((uint32_t)v[7] << 16);
-    reinterpret_cast<uint4*>(mat_ptr(N, node) + (size_t)i * NP)[j0 / 8] = o;
-}
-
-// Build-time seams: both cells Free -> unit edge, both endpoints are pivots.
-__global__ void seams_build_kernel(MatSet N, const int* __restrict__ seams, int n_seams,
-                                   const uint8_t* __restrict__ pass, const uint16_t* __restrict__ wts, int S,
-                                   int side, int nodes_x, uint8_t* kflag, const int* __restrict__ list, int y0) {
-    const int node = list ? list[y0 + blockIdx.y] : y0 + blockIdx.y;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n_seams) return;
-    const int* e = seams + 6 * s;
-    const int R0 = (node / nodes_x) * side, C0 = (node % nodes_x) * side;
-    const size_t a = (size_t)(R0 + e[2]) * S + C0 + e[3], c = (size_t)(R0 + e[4]) * S + C0 + e[5];
-    if (!pass[a] || !pass[c]) return;
-    const uint16_t w = wts ? edge_weight(wts[a], wts[c]) : (uint16_t)1;  // internal_node.cpp:160-161
-    if (w >= INF) return;
-    uint16_t* D = mat_ptr(N, node);
-    const int NP = N.NP;
-    D[(size_t)e[0] * NP + e[1]] = min(D[(size_t)e[0] * NP + e[1]], w);
-    D[(size_t)e[1] * NP + e[0]] = min(D[(size_t)e[1] * NP + e[0]], w);
-    kflag[(size_t)node * NP + e[0]] = 1;
-    kflag[(size_t)node * NP + e[1]] = 1;
-}
-
-// ---------------------------------------------------------------------------
 // Weighted leaf (LeafTile::recomputeFromGrid's Dijkstra branch,
 // leaf_tile.cpp:154-192): D starts as the tile's weighted adjacency - 0 on
 // the diagonal, w(u, v) between 4-adjacent passable cells, INF elsewhere and
@@ -491,19 +431,9 @@ __global__ void ext_snapshot_kernel(const Slot* __restrict__ S, const int* __res
 // clears its children's decrease flags, which its insert stage has consumed:
 // outside an opening call all decrease flags are zero.
 __global__ void ext_compare_kernel(const Slot* __restrict__ S, const int* __restrict__ ext, int nExt, int NP,
-                                   const uint16_t* __restrict__ snap, uint8_t* slot_dec, int g, int any_change) {
+                                   const uint16_t* __restrict__ snap, uint8_t* slot_dec, int g) {
     const int slot = blockIdx.y;
     const Slot& sl = S[slot];
-    if (any_change) {  // rebuilds: slot_dec[slot] = 1 when any exterior entry differs, nothing else
-        const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-        bool d = false;
-        if (idx < (size_t)nExt * nExt) {
-            const int a = (int)(idx / nExt), c = (int)(idx % nExt);
-            d = sl.mat[(size_t)ext[a] * NP + ext[c]] != snap[(size_t)slot * nExt * nExt + idx];
-        }
-        if (__any_sync(FULL, d) && (threadIdx.x & 31) == 0) slot_dec[slot] = 1;
-        return;
-    }
     if (sl.child_dec && blockIdx.x == 0 && threadIdx.x < g * g) {
         const int q = threadIdx.x;
         const int tx = sl.node % sl.nodes_x, ty = sl.node / sl.nodes_x;
@@ -614,25 +544,6 @@ void launch_leaf_bfs(const uint8_t* pass, int S, int b, int leaves_x, int n_leav
     }
 }
 
-void launch_node_init(MatSet node, MatSet child, const int* child_ext, int nP, int g, int nodes_x,
-                      int child_nodes_x, int n_nodes, cudaStream_t st, const int* list) {
-    const size_t chunks = (size_t)node.NP * (node.NP / 8);
-    for (int y0 = 0; y0 < n_nodes; y0 += kMaxGridY) {
-        dim3 grid(blocks_for(chunks, 256), std::min(kMaxGridY, n_nodes - y0));
-        node_init_kernel<<<grid, 256, 0, st>>>(node, child, child_ext, nP, g, nodes_x, child_nodes_x, list, y0);
-    }
-}
-
-void launch_seams_build(MatSet node, const int* seams, int n_seams, const uint8_t* pass, int S, int side,
-                        int nodes_x, int n_nodes, uint8_t* kflag, cudaStream_t st, const int* list,
-                        const uint16_t* wts) {
-    if (n_seams == 0) return;
-    for (int y0 = 0; y0 < n_nodes; y0 += kMaxGridY) {
-        dim3 grid(blocks_for(n_seams, 128), std::min(kMaxGridY, n_nodes - y0));
-        seams_build_kernel<<<grid, 128, 0, st>>>(node, seams, n_seams, pass, wts, S, side, nodes_x, kflag, list, y0);
-    }
-}
-
 void launch_leaf_weight_init(const uint8_t* pass, const uint16_t* wts, int S, int b, int leaves_x, int n_leaves,
                              MatSet leaves, uint8_t* kflag, const int* list, cudaStream_t st) {
     constexpr int kWarps = 8;
@@ -710,11 +621,11 @@ void launch_ext_snapshot(const Slot* S, int n, const int* ext, int nExt, int NP,
 }
 
 void launch_ext_compare(const Slot* S, int n, const int* ext, int nExt, int NP, const uint16_t* snap,
-                        uint8_t* slot_dec, int g, cudaStream_t st, int any_change) {
+                        uint8_t* slot_dec, int g, cudaStream_t st) {
     for (int y0 = 0; y0 < n; y0 += kMaxGridY) {
         dim3 grid(blocks_for((size_t)nExt * nExt, 256), std::min(kMaxGridY, n - y0));
         ext_compare_kernel<<<grid, 256, 0, st>>>(S + y0, ext, nExt, NP, snap + (size_t)y0 * nExt * nExt,
-                                                 slot_dec + y0, g, any_change);
+                                                 slot_dec + y0, g);
     }
 }
 

@@ -25,19 +25,42 @@ constexpr int kFlagTile = 64;     // column granularity of panel "finite" flags
 void launch_leaf_bfs(const uint8_t* pass, int S, int b, int leaves_x, int n_leaves, MatSet leaves,
                      cudaStream_t st, const int* list = nullptr);
 
-// Internal-node initial D_U: block diagonal of child summaries, INF
-// elsewhere (internal_node.cpp:98-145).  child_ext: the child level's
-// port -> matrix-index table (nP entries).
-void launch_node_init(MatSet node, MatSet child, const int* child_ext, int nP, int g, int nodes_x,
-                      int child_nodes_x, int n_nodes, cudaStream_t st, const int* list = nullptr);
-
-// Seam edges of the build (internal_node.cpp:155-173): seams = 6 ints per
-// candidate {u, v, ur, uc, vr, vc} (node-relative coordinates).
-// wts (optional): per-cell traversal weights (S x S); a seam gets the edge
-// weight w(u, v) = max(1, (w_u + w_v) / 2) (GridMap::edgeWeight), else 1.
-void launch_seams_build(MatSet node, const int* seams, int n_seams, const uint8_t* pass, int S,
-                        int side, int nodes_x, int n_nodes, uint8_t* kflag, cudaStream_t st,
-                        const int* list = nullptr, const uint16_t* wts = nullptr);
+// Internal-node matrices of one level from their children and seams
+// (node_build.cu; internal_node.cpp:94-245).
+struct NodeBuild {
+    MatSet N, C;            // the level's and the child level's matrices
+    const int* cext;        // child port -> child matrix index (nP entries)
+    const uint8_t* isext;   // [NP] 1 = exterior port of the node
+    int nP, g, nodes_x, child_nodes_x, side, S;
+    const int* seams;       // candidates: 6 ints {u, v, ur, uc, vr, vc}, node-relative
+    int n_seams;
+    int capI;               // most candidates that touch one child
+    const uint8_t* pass;    // S x S, 1 = Free
+    const uint16_t* wts;    // S x S traversal weights or null: an edge costs
+                            // max(1, (w_u + w_v) / 2) (GridMap::edgeWeight), else 1
+    const int* list;        // nodes of the launch, or null: first, first + 1, ...
+    int first;
+    const uint8_t* active;  // or null: node i of the launch is built when active[i]
+    const int* parent;      // with `changed`: position of node i's parent in the next level's list
+    uint8_t* changed;       // or null: set to 1 for the parent of a node whose exterior block changed
+    // scratch of the launch, per node (node_build_layout)
+    int n, TP, RP;          // nodes, padded seam count, row stride of R and U
+    int* cnt;               // [n][1 + g^2] active seams, incidences per child
+    int* vmax;              // [n][4] largest finite values of R, T, U
+    int4* edge;             // [n][TP]
+    uint2* inc;             // [n][g^2][capI]
+    uint16_t *R, *T, *P, *U;
+};
+bool node_build_small(const NodeBuild& P);  // the level needs no scratch
+// Scratch pointers for n nodes at `base` (any base: only the size counts);
+// returns the bytes.
+size_t node_build_layout(NodeBuild& P, int n, unsigned char* base);
+// *most = max(*most, active seams of each of the n nodes).
+void launch_seam_count(const NodeBuild& P, int n, int* most, cudaStream_t st);
+// most_seams: at least the active seams of every node of the launch.
+void launch_node_build(const NodeBuild& P, int n, int most_seams, cudaStream_t st);
+// INF in the padding of the first `count` matrices of M.
+void launch_pad_fill(MatSet M, int count, cudaStream_t st);
 
 // Weighted leaves (the reference's Dijkstra leaf build): D = the tile's
 // weighted adjacency with a zero diagonal, pivot flags = its passable cells;
@@ -93,11 +116,10 @@ void launch_node_seams(const Slot* S, int n, const int* seams, int NP, cudaStrea
 // S_U): snap holds nExt*nExt entries per slot; compare sets *dec and
 // slot_dec[slot] when any entry decreased (refreshBoundarySummary,
 // leaf_tile.cpp:253-273, internal_node.cpp:415-433) and clears the node
-// slots' children's decrease flags.  With any_change != 0 (rebuilds) it only
-// sets slot_dec[slot] when any exterior entry differs from the snapshot.
+// slots' children's decrease flags.
 void launch_ext_snapshot(const Slot* S, int n, const int* ext, int nExt, int NP, uint16_t* snap, cudaStream_t st);
 void launch_ext_compare(const Slot* S, int n, const int* ext, int nExt, int NP, const uint16_t* snap,
-                        uint8_t* slot_dec, int g, cudaStream_t st, int any_change = 0);
+                        uint8_t* slot_dec, int g, cudaStream_t st);
 
 // --- device-driven openings (open.cu) -----------------------------------------
 // One onBatchCellsOpened call (or several, on indexes of equal b and g) as ONE
