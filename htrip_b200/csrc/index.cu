@@ -146,6 +146,13 @@ struct PoolBuf {
     }
 };
 
+// A piece of an index's device arena.
+template <class T>
+struct Span {
+    T* p = nullptr;
+    size_t n = 0;
+};
+
 struct Level {
     int lvl = 0;
     int side = 0;      // tile side (b for leaves, s for nodes)
@@ -160,22 +167,19 @@ struct Level {
     std::vector<int> seams;  // 6 ints per seam candidate
     int nseams = 0;
     int cap_inc = 0;  // most seam candidates that touch one child
-    DevBuf<int> d_ext, d_seams, d_ext_inv;
-    DevBuf<uint16_t> mat;
-    DevBuf<uint8_t> kflag;
-    DevBuf<int> klist, kcnt;
-    DevBuf<uint8_t> dec;
+    // device-side tables and state (pieces of htrip_index::arena)
+    Span<int> d_ext, d_seams, d_ext_inv;
+    Span<uint16_t> mat;
+    Span<uint8_t> kflag;
+    Span<int> klist, kcnt;
+    Span<uint8_t> dec;
     // device-driven openings: per matrix index, 1 = an exterior port (leaf
     // perimeter cell / node exterior port); per node, the stamp of the last
     // opening call whose update decreased its exterior block (dstamp) and of
     // the last call that put it on the level's work list (mstamp)
-    DevBuf<uint8_t> d_isext;
-    DevBuf<uint32_t> dstamp, mstamp;
+    Span<uint8_t> d_isext;
+    Span<uint32_t> dstamp, mstamp;
     MatSet ms() const { return MatSet{mat.p, n, NP}; }
-    void release() {
-        d_ext.release(); d_seams.release(); d_ext_inv.release(); mat.release(); kflag.release();
-        klist.release(); kcnt.release(); dec.release(); d_isext.release(); dstamp.release(); mstamp.release();
-    }
 };
 
 inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
@@ -336,6 +340,7 @@ struct htrip_index {
     uint64_t update_counter = 0;  // opening calls since creation
     int S = 0, H = 0, rows = 0, cols = 0, leaves_x = 0;
     std::vector<Level> L;
+    DevBuf<unsigned char> arena;  // every level's tables, state and matrices
     DevBuf<uint8_t> pass;
     // scratch of the index's own build / opening launches
     UpdateArena u;
@@ -356,8 +361,8 @@ struct htrip_index {
         wts.release();
     }
     void release() {
-        for (auto& l : L) l.release();
         L.clear();
+        arena.release();
         pass.release();
         u.release();
         q.release();
@@ -474,6 +479,19 @@ uint16_t host_cell_weight(const htrip_index* h, int r, int c, const uint8_t* obs
     return h->wgrid[(size_t)r * h->wcols + c];
 }
 
+// The passability mirror over the index's S x S cells (outside the grid: not
+// passable) from the caller's grid: its cell states go out as they are and a
+// kernel writes the mirror.
+void upload_passable(htrip_index* h, const uint8_t* observed, int rows, int cols) {
+    cudaStream_t st = h->stream;
+    const size_t n = (size_t)rows * cols;
+    h->pass.reserve((size_t)h->S * h->S);
+    h->u.dev.reserve(std::max<size_t>(1, n), st);
+    if (n) ck(cudaMemcpyAsync(h->u.dev.p, observed, n, cudaMemcpyHostToDevice, st), "grid");
+    hb::launch_passable(h->u.dev.p, rows, cols, h->pass.p, h->S, st);
+    ck(cudaGetLastError(), "passability");
+}
+
 // The weights' device mirror over the index's S x S (1 outside the grid,
 // where no cell is passable).
 void upload_weights(htrip_index* h) {
@@ -509,41 +527,73 @@ std::vector<int> weighted_leaves(const htrip_index* h, const std::vector<int>& l
     return out;
 }
 
+// One device allocation for all levels: the static tables (one upload), the
+// per-node state that starts at zero (one memset), the pivot lists, then the
+// matrices.  Separate allocations, nine per level, cost a small map's
+// build more than its kernels do (256 x 256: 3 of 6 ms).
 void alloc_levels(htrip_index* h) {
+    size_t off = 0;
+    auto take = [&](auto& span, size_t n) {
+        span.n = n;
+        span.p = reinterpret_cast<decltype(span.p)>(off);  // offset until the arena exists
+        off += align256(std::max<size_t>(1, n) * sizeof(*span.p));
+    };
     for (auto& Lv : h->L) {
-        Lv.mat.reserve((size_t)Lv.nnodes * Lv.NP * Lv.NP);
-        if (Lv.lvl >= 1) hb::launch_pad_fill(Lv.ms(), Lv.nnodes, h->stream);  // node builds write the logical part only
-        Lv.d_ext.reserve(std::max(1, Lv.nExt));
-        ck(cudaMemcpyAsync(Lv.d_ext.p, Lv.ext.data(), Lv.nExt * sizeof(int), cudaMemcpyHostToDevice, h->stream), "ext");
-        if (Lv.nseams) {
-            Lv.d_seams.reserve(Lv.seams.size());
-            ck(cudaMemcpyAsync(Lv.d_seams.p, Lv.seams.data(), Lv.seams.size() * sizeof(int), cudaMemcpyHostToDevice,
-                               h->stream), "seams");
-        }
-        if (Lv.lvl >= 1) {
-            std::vector<int> inv(Lv.NP, -1);
-            for (int e = 0; e < Lv.nExt; ++e) inv[Lv.ext[e]] = e;
-            Lv.d_ext_inv.reserve(Lv.NP);
-            ck(cudaMemcpyAsync(Lv.d_ext_inv.p, inv.data(), Lv.NP * sizeof(int), cudaMemcpyHostToDevice, h->stream),
-               "ext_inv");
-        }
-        Lv.kflag.reserve((size_t)Lv.nnodes * Lv.NP);
-        ck(cudaMemsetAsync(Lv.kflag.p, 0, (size_t)Lv.nnodes * Lv.NP, h->stream), "kflag");
-        Lv.klist.reserve((size_t)Lv.nnodes * Lv.NP);
-        Lv.kcnt.reserve(Lv.nnodes);
-        Lv.dec.reserve(Lv.nnodes);
-        // decrease flags are zero outside an opening call (each level's flags
-        // are cleared by the level above once it has read them)
-        ck(cudaMemsetAsync(Lv.dec.p, 0, Lv.nnodes, h->stream), "dec");
-        std::vector<uint8_t> isext(Lv.NP, 0);
-        for (int e = 0; e < Lv.nExt; ++e) isext[Lv.ext[e]] = 1;
-        Lv.d_isext.reserve(Lv.NP);
-        ck(cudaMemcpyAsync(Lv.d_isext.p, isext.data(), Lv.NP, cudaMemcpyHostToDevice, h->stream), "isext");
-        Lv.dstamp.reserve(Lv.nnodes);
-        Lv.mstamp.reserve(Lv.nnodes);
-        ck(cudaMemsetAsync(Lv.dstamp.p, 0, Lv.nnodes * sizeof(uint32_t), h->stream), "dstamp");
-        ck(cudaMemsetAsync(Lv.mstamp.p, 0, Lv.nnodes * sizeof(uint32_t), h->stream), "mstamp");
+        take(Lv.d_ext, std::max(1, Lv.nExt));
+        take(Lv.d_seams, Lv.seams.size());
+        take(Lv.d_ext_inv, Lv.NP);
+        take(Lv.d_isext, Lv.NP);
     }
+    const size_t tables = off;
+    for (auto& Lv : h->L) {
+        // pivot and decrease flags are zero outside an opening call (an
+        // opening clears the ones it set)
+        take(Lv.kflag, (size_t)Lv.nnodes * Lv.NP);
+        take(Lv.dec, Lv.nnodes);
+        take(Lv.dstamp, Lv.nnodes);
+        take(Lv.mstamp, Lv.nnodes);
+    }
+    const size_t zeros = off;
+    for (auto& Lv : h->L) {
+        take(Lv.klist, (size_t)Lv.nnodes * Lv.NP);
+        take(Lv.kcnt, Lv.nnodes);
+    }
+    for (auto& Lv : h->L) take(Lv.mat, (size_t)Lv.nnodes * Lv.NP * Lv.NP);
+    h->arena.reserve(off);
+    std::vector<unsigned char> host(tables, 0);
+    unsigned char* base = h->arena.p;
+    auto place = [&](auto& span) {
+        span.p = reinterpret_cast<decltype(span.p)>(base + reinterpret_cast<size_t>(span.p));
+    };
+    for (auto& Lv : h->L) {
+        auto* ext = reinterpret_cast<int*>(host.data() + reinterpret_cast<size_t>(Lv.d_ext.p));
+        auto* seams = reinterpret_cast<int*>(host.data() + reinterpret_cast<size_t>(Lv.d_seams.p));
+        auto* inv = reinterpret_cast<int*>(host.data() + reinterpret_cast<size_t>(Lv.d_ext_inv.p));
+        auto* isext = host.data() + reinterpret_cast<size_t>(Lv.d_isext.p);
+        std::copy(Lv.ext.begin(), Lv.ext.end(), ext);
+        std::copy(Lv.seams.begin(), Lv.seams.end(), seams);
+        std::fill(inv, inv + Lv.NP, -1);
+        for (int e = 0; e < Lv.nExt; ++e) {
+            inv[Lv.ext[e]] = e;
+            isext[Lv.ext[e]] = 1;
+        }
+        place(Lv.d_ext);
+        place(Lv.d_seams);
+        place(Lv.d_ext_inv);
+        place(Lv.d_isext);
+        place(Lv.kflag);
+        place(Lv.dec);
+        place(Lv.dstamp);
+        place(Lv.mstamp);
+        place(Lv.klist);
+        place(Lv.kcnt);
+        place(Lv.mat);
+    }
+    ck(cudaMemcpyAsync(base, host.data(), tables, cudaMemcpyHostToDevice, h->stream), "level tables");
+    ck(cudaMemsetAsync(base + tables, 0, zeros - tables, h->stream), "level state");
+    for (auto& Lv : h->L)  // node builds write the logical part of a matrix only
+        if (Lv.lvl >= 1) hb::launch_pad_fill(Lv.ms(), Lv.nnodes, h->stream);
+    ck(cudaGetLastError(), "padding");
     h->stamp_epoch++;
 }
 
@@ -782,8 +832,11 @@ void do_build(htrip_index* h, const uint8_t* observed, int rows, int cols) {
     while (S < std::max(rows, cols)) S *= g;
     int H = 0;
     for (int t = S / b; t > 1; t /= g) ++H;
-    h->release();
+    // a map of the same padded side is rebuilt in place: the tables are the same,
+    // and every matrix is written anew
+    const bool in_place = h->built && !h->offloaded && h->S == S;
     h->built = false;
+    if (!in_place) h->release();
     h->offloaded = false;
     h->parked.clear();
     h->S = S;
@@ -791,16 +844,13 @@ void do_build(htrip_index* h, const uint8_t* observed, int rows, int cols) {
     h->rows = rows;
     h->cols = cols;
     h->leaves_x = S / b;
-    make_levels(h);
-    h->ref_bytes = reference_bytes(h);
-    alloc_levels(h);
+    if (!in_place) {
+        make_levels(h);
+        h->ref_bytes = reference_bytes(h);
+        alloc_levels(h);
+    }
     cudaStream_t st = h->stream;
-    // Passability mirror, padded to S x S (outside the grid = not passable).
-    std::vector<uint8_t> pass((size_t)S * S, 0);
-    for (int r = 0; r < rows; ++r)
-        for (int c = 0; c < cols; ++c) pass[(size_t)r * S + c] = observed[(size_t)r * cols + c] == 1;
-    h->pass.reserve(pass.size());
-    ck(cudaMemcpyAsync(h->pass.p, pass.data(), pass.size(), cudaMemcpyHostToDevice, st), "pass");
+    upload_passable(h, observed, rows, cols);
     upload_weights(h);
     BuildSet bs;
     bs.all = true;
@@ -823,7 +873,9 @@ void do_lift_root(htrip_index* h, const uint8_t* observed, int rows, int cols) {
     cudaStream_t st = h->stream;
     ck(cudaStreamSynchronize(st), "sync");
     std::vector<Level> old = std::move(h->L);
+    DevBuf<unsigned char> old_arena = h->arena;
     h->L.clear();
+    h->arena = DevBuf<unsigned char>();
     const int old_rows = h->rows, old_cols = h->cols;
     const uint64_t old_ref = h->ref_bytes;
     h->S = old_S * g;
@@ -844,7 +896,8 @@ void do_lift_root(htrip_index* h, const uint8_t* observed, int rows, int cols) {
                                  cudaMemcpyDeviceToDevice, st), "move matrices");
         }
     } catch (...) {
-        for (auto& l : h->L) l.release();
+        h->arena.release();
+        h->arena = old_arena;
         h->L = std::move(old);  // the old matrices are intact
         h->S = old_S;
         h->H = old_H;
@@ -854,14 +907,9 @@ void do_lift_root(htrip_index* h, const uint8_t* observed, int rows, int cols) {
         h->ref_bytes = old_ref;
         throw;
     }
-    for (auto& l : old) l.release();
+    old_arena.release();
     old.clear();
-    const int S = h->S;
-    std::vector<uint8_t> pass((size_t)S * S, 0);
-    for (int r = 0; r < std::min(rows, S); ++r)
-        for (int c = 0; c < std::min(cols, S); ++c) pass[(size_t)r * S + c] = observed[(size_t)r * cols + c] == 1;
-    h->pass.reserve(pass.size());
-    ck(cudaMemcpyAsync(h->pass.p, pass.data(), pass.size(), cudaMemcpyHostToDevice, st), "pass");
+    upload_passable(h, observed, rows, cols);
     upload_weights(h);
     // the new area of every level below the new root
     auto fresh = [&](int nodes_x, int old_nodes_x) {
@@ -897,7 +945,7 @@ void do_lift_root(htrip_index* h, const uint8_t* observed, int rows, int cols) {
 void do_rebuild_leaves(htrip_index* h, const std::vector<int>& leaves_in, const uint8_t* observed, int rows,
                        int cols, bool propagate_all) {
     cudaStream_t st = h->stream;
-    const int S = h->S, g = h->g;
+    const int g = h->g;
     std::vector<int> cur;
     {
         std::vector<uint8_t> seen(h->L[0].nnodes, 0);
@@ -907,10 +955,7 @@ void do_rebuild_leaves(htrip_index* h, const std::vector<int>& leaves_in, const 
     if (cur.empty()) return;
     h->update_counter++;
     // the passability mirror follows the caller's grid (leaf BFS and seams read it)
-    std::vector<uint8_t> pass((size_t)S * S, 0);
-    for (int r = 0; r < std::min(rows, S); ++r)
-        for (int c = 0; c < std::min(cols, S); ++c) pass[(size_t)r * S + c] = observed[(size_t)r * cols + c] == 1;
-    ck(cudaMemcpyAsync(h->pass.p, pass.data(), pass.size(), cudaMemcpyHostToDevice, st), "pass");
+    upload_passable(h, observed, rows, cols);
     // every ancestor of a listed leaf, per level; the device skips those that
     // `track` leaves unchanged
     BuildSet bs;
@@ -3488,10 +3533,7 @@ htrip_status htrip_memory_bytes(const htrip_index* h, uint64_t* reference_bytes,
     uint64_t ref = 0, dev = 0;
     if (h->built) {
         ref = h->ref_bytes;
-        for (const auto& Lv : h->L)
-            dev += (Lv.mat.n + Lv.klist.n * 2 + Lv.kcnt.n * 2) * sizeof(uint16_t) + Lv.kflag.n + Lv.dec.n +
-                   (Lv.d_ext.n + Lv.d_seams.n) * sizeof(int);
-        dev += h->u.nlist.n + h->u.nscratch.n;
+        dev += h->arena.n + h->u.nlist.n + h->u.nscratch.n;
         dev += h->pass.n + h->u.dev.n + h->u.snap.n * 2 + h->u.panel.n * 2 + h->u.pflags.n + h->q.dev.n +
                h->wts.n * sizeof(uint16_t);
     }

@@ -23,6 +23,12 @@ __device__ __forceinline__ uint16_t* mat_ptr(const MatSet& M, int m) {
     return M.base + (size_t)m * M.NP * M.NP;
 }
 
+__global__ void passable_kernel(const uint8_t* __restrict__ observed, int rows, int cols, uint8_t* pass, int S) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y * blockDim.y + threadIdx.y;
+    if (r >= S || c >= S) return;
+    pass[(size_t)r * S + c] = r < rows && c < cols && observed[(size_t)r * cols + c] == 1;
+}
+
 // ---------------------------------------------------------------------------
 // Leaf APSP: one warp per source cell, bit-parallel BFS.  Lane r owns row r
 // of the b x b leaf as a bitmask; a BFS level is one shift/shuffle step, so
@@ -534,6 +540,11 @@ inline unsigned blocks_for(size_t n, unsigned t) { return (unsigned)((n + t - 1)
 // ---------------------------------------------------------------------------
 // Launch wrappers
 // ---------------------------------------------------------------------------
+
+void launch_passable(const uint8_t* observed, int rows, int cols, uint8_t* pass, int S, cudaStream_t st) {
+    const dim3 block(64, 4);
+    passable_kernel<<<dim3(blocks_for(S, 64), blocks_for(S, 4)), block, 0, st>>>(observed, rows, cols, pass, S);
+}
 
 void launch_leaf_bfs(const uint8_t* pass, int S, int b, int leaves_x, int n_leaves, MatSet leaves,
                      cudaStream_t st, const int* list) {

@@ -19,6 +19,9 @@ constexpr int kPivotChunk = 64;   // pivots closed per round (B)
 constexpr int kFlagTile = 64;     // column granularity of panel "finite" flags
 
 // --- build ------------------------------------------------------------------
+// pass[r * S + c] = 1 where the rows x cols grid has a Free cell, else 0 (S x S).
+void launch_passable(const uint8_t* observed, int rows, int cols, uint8_t* pass, int S, cudaStream_t st);
+
 // Leaf APSP by bit-parallel BFS (reference LeafTile::recomputeFromGrid,
 // leaf_tile.cpp:96-153).  pass: S*S bytes, 1 = Free.
 // With `list`, the n_leaves leaves list[0..n_leaves) instead of 0..n_leaves.
