@@ -281,9 +281,8 @@ struct UpdateArena {
     PoolBuf<uint16_t> panel;
     PoolBuf<uint8_t> pflags;
     HostBuf stage, rb;
-    cudaEvent_t ev_cnt = nullptr;  // an opening level's pivot counts / a build's seam counts reached the host
-    // node builds: the staged node lists with the seam counts, and the
-    // scratch of the launches (hb::node_build_layout)
+    cudaEvent_t ev_cnt = nullptr;  // an opening level's pivot counts reached the host
+    // node builds: the staged node lists and the scratch of the launches (hb::node_build_layout)
     HostBuf nstage;
     PoolBuf<unsigned char> nlist, nscratch;
     int open_grid = 0;             // CTAs of the persistent opening kernel
@@ -690,9 +689,7 @@ struct BuildSet {
 // Scratch of one launch of the general node build (bounds the nodes a launch takes).
 constexpr size_t kNodeScratch = (size_t)192 << 20;
 
-// Everything is issued on the index's stream; the host waits once, early, for the
-// levels' seam counts (they set the number of closure rounds), while the
-// leaf kernel runs.  Not waited for at the end.
+// Everything is issued on the index's stream and not waited for.
 void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int rows, int cols) {
     cudaStream_t st = h->stream;
     UpdateArena& A = h->u;
@@ -707,14 +704,13 @@ void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int 
         std::iota(every.begin(), every.end(), 0);
     }
     const std::vector<int> wl = weighted_leaves(h, bs.all ? every : bs.leaves, obs, rows, cols);
-    // one upload: {seam counts | leaves, weighted leaves, node lists, parents, active flags}
+    // one upload: {leaves, weighted leaves, node lists, parents, active flags}
     size_t bytes = 0;
     auto take = [&](size_t n) {
         const size_t o = bytes;
         bytes += align256(std::max<size_t>(n, 1));
         return o;
     };
-    const size_t o_most = take((H + 1) * sizeof(int));
     const size_t o_leaves = take((bs.all ? 0 : bs.leaves.size()) * sizeof(int)), o_wl = take(wl.size() * sizeof(int));
     std::vector<size_t> o_list(H + 1), o_parent(H + 1), o_active(H + 1);
     if (!bs.all)
@@ -741,7 +737,6 @@ void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int 
     }
     ck(cudaMemcpyAsync(ds, hs, bytes, cudaMemcpyHostToDevice, st), "build lists");
     std::vector<hb::NodeBuild> nb(H + 1);
-    bool wait = false;
     for (int l = 1; l <= H; ++l) {
         Level& Lv = h->L[l];
         Level& Lc = h->L[l - 1];
@@ -772,16 +767,6 @@ void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int 
                 }
             }
         }
-        if (count(l) && !hb::node_build_small(P)) {
-            hb::launch_seam_count(P, count(l), reinterpret_cast<int*>(ds + o_most) + l, st);
-            wait = true;
-        }
-    }
-    ck(cudaGetLastError(), "seam counts");
-    if (wait) {
-        ck(cudaMemcpyAsync(hs + o_most, ds + o_most, (H + 1) * sizeof(int), cudaMemcpyDeviceToHost, st), "seam counts");
-        if (!A.ev_cnt) ck(cudaEventCreateWithFlags(&A.ev_cnt, cudaEventDisableTiming), "event");
-        ck(cudaEventRecord(A.ev_cnt, st), "seam counts");
     }
     // leaves: bit-parallel BFS, then, for leaves with non-unit weights, the
     // weighted adjacency closed over its passable cells
@@ -789,14 +774,12 @@ void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int 
         hb::launch_leaf_bfs(h->pass.p, h->S, h->b, h->leaves_x, count(0), h->L[0].ms(), st,
                             bs.all ? nullptr : reinterpret_cast<const int*>(ds + o_leaves));
     ck(cudaGetLastError(), "leaf bfs");
-    if (wait) ck(cudaEventSynchronize(A.ev_cnt), "seam counts");
     if (!wl.empty()) {
         hb::launch_leaf_weight_init(h->pass.p, h->wts.p, h->S, h->b, h->leaves_x, (int)wl.size(), h->L[0].ms(),
                                     h->L[0].kflag.p, reinterpret_cast<const int*>(ds + o_wl), st);
         ck(cudaGetLastError(), "weighted leaf init");
         close_matrices(h, h->L[0], wl);
     }
-    const int* most = reinterpret_cast<const int*>(hs + o_most);
     size_t scratch = 0;
     std::vector<int> chunk(H + 1, 0);
     for (int l = 1; l <= H; ++l) {
@@ -818,7 +801,7 @@ void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int 
             if (P.active) P.active += c0;
             if (P.parent) P.parent += c0;
             if (!hb::node_build_small(P)) hb::node_build_layout(P, n, A.nscratch.p);
-            hb::launch_node_build(P, n, most[l], st);
+            hb::launch_node_build(P, n, st);
             ck(cudaGetLastError(), "node build");
         }
 }

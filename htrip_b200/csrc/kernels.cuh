@@ -30,6 +30,7 @@ void launch_leaf_bfs(const uint8_t* pass, int S, int b, int leaves_x, int n_leav
 
 // Internal-node matrices of one level from their children and seams
 // (node_build.cu; internal_node.cpp:94-245).
+constexpr int kNodeState = 32, kNodeChanged = 4;
 struct NodeBuild {
     MatSet N, C;            // the level's and the child level's matrices
     const int* cext;        // child port -> child matrix index (nP entries)
@@ -49,19 +50,17 @@ struct NodeBuild {
     // scratch of the launch, per node (node_build_layout)
     int n, TP, RP;          // nodes, padded seam count, row stride of R and U
     int* cnt;               // [n][1 + g^2] active seams, incidences per child
-    int* vmax;              // [n][4] largest finite values of R, T, U
+    int* state;             // [n][kNodeState]: largest finite values of R, T, U; from
+                            // kNodeChanged on, whether each closure pass changed T
     int4* edge;             // [n][TP]
     uint2* inc;             // [n][g^2][capI]
-    uint16_t *R, *T, *P, *U;
+    uint16_t *R, *T, *U;
 };
 bool node_build_small(const NodeBuild& P);  // the level needs no scratch
 // Scratch pointers for n nodes at `base` (any base: only the size counts);
 // returns the bytes.
 size_t node_build_layout(NodeBuild& P, int n, unsigned char* base);
-// *most = max(*most, active seams of each of the n nodes).
-void launch_seam_count(const NodeBuild& P, int n, int* most, cudaStream_t st);
-// most_seams: at least the active seams of every node of the launch.
-void launch_node_build(const NodeBuild& P, int n, int most_seams, cudaStream_t st);
+void launch_node_build(const NodeBuild& P, int n, cudaStream_t st);
 // INF in the padding of the first `count` matrices of M.
 void launch_pad_fill(MatSet M, int count, cudaStream_t st);
 

@@ -11,7 +11,7 @@
 // to u's child with offset 0 and to v's child with offset w.  With R_q[k][j] =
 // o_k (+) S_q[x_k][j] for the incidences k = (x_k, e_k, o_k) of child q:
 //   T0[e][e'] = min over common children q of R_q[e][x_e'] (+) o_e'
-//   T  = closure of T0 (blocked Floyd-Warshall, 64 pivots a round)
+//   T  = closure of T0 (repeated squaring)
 //   U_p[e][i]  = min_k T[e][e_k] (+) R_p[k][i]            (k over child p's)
 //   D[i][j]    = min([p == q] S_p[i][j], min_k U_p[e_k][i] (+) R_q[k][j])
 //                for i in child p, j in child q, p <= q, and transposed.
@@ -20,7 +20,7 @@
 // bit for bit; each matrix is written once instead of once per 64 pivots.
 // Measured against the blocked closure over the seam endpoints that it
 // replaces (device time, B200): building a 1024 x 1024 street map, b = 8, 22.8 ->
-// 5.9 ms; one weight change on a 256 x 256 map, b = 8, 2.45 -> 0.75 ms.
+// 5.2 ms; one weight change on a 256 x 256 map, b = 8, 2.45 -> 0.53 ms.
 #include "closure.cuh"
 #include "kernels.cuh"
 
@@ -64,36 +64,24 @@ __device__ __forceinline__ uint16_t seam_weight(const NodeBuild& P, int node, in
     return P.wts ? edge_weight(P.wts[a], P.wts[c]) : (uint16_t)1;  // internal_node.cpp:160-161
 }
 
-// Largest number of active seams of the launch's nodes into *most.
-__global__ void __launch_bounds__(128) seam_count_kernel(const NodeBuild P, int* most) {
-    const int node = node_id(P, blockIdx.x);
-    int c = 0;
-    for (int s = threadIdx.x; s < P.n_seams; s += blockDim.x) c += seam_weight(P, node, s) < INF;
-    c = __reduce_add_sync(FULL, c);
-    __shared__ int w[4];
-    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) atomicMax(most, w[0] + w[1] + w[2] + w[3]);
-}
-
 // Seam edge record: x = qu | qv << 8, y = iu | iv << 16 (incidence rows in the
 // two children), z = xu | xv << 16 (ports in the two children), w = weight.
 // Incidence record: x = port | offset << 16, y = edge.
 
 // Active seams of every node: its edges and each child's incidences.
-__global__ void __launch_bounds__(256) seam_list_kernel(const NodeBuild P) {
+__global__ void __launch_bounds__(1024) seam_list_kernel(const NodeBuild P) {
     __shared__ int q_cnt[256];
-    __shared__ int wtot[8];
+    __shared__ int wtot[32];
     __shared__ int base;
-    const int i = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int i = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
     if (P.active && !P.active[i]) return;
     const int node = node_id(P, i), g2 = P.g * P.g;
-    if (tid < g2) q_cnt[tid] = 0;
+    for (int q = tid; q < g2; q += blockDim.x) q_cnt[q] = 0;
     if (tid == 0) base = 0;
     __syncthreads();
     int4* edge = P.edge + (size_t)i * P.TP;
     uint2* inc = P.inc + (size_t)i * g2 * P.capI;
-    for (int s0 = 0; s0 < P.n_seams; s0 += 256) {
+    for (int s0 = 0; s0 < P.n_seams; s0 += blockDim.x) {
         const int s = s0 + tid;
         const uint16_t w = s < P.n_seams ? seam_weight(P, node, s) : INF;
         const bool on = w < INF;
@@ -112,13 +100,13 @@ __global__ void __launch_bounds__(256) seam_list_kernel(const NodeBuild P) {
         }
         __syncthreads();
         if (tid == 0)
-            for (int k = 0; k < 8; ++k) base += wtot[k];
+            for (int k = 0; k < nw; ++k) base += wtot[k];
         __syncthreads();
     }
     int* cnt = P.cnt + (size_t)i * (1 + g2);
     if (tid == 0) cnt[0] = base;
-    if (tid < g2) cnt[1 + tid] = q_cnt[tid];
-    if (tid < 4) P.vmax[4 * i + tid] = 0;
+    for (int q = tid; q < g2; q += blockDim.x) cnt[1 + q] = q_cnt[q];
+    if (tid < kNodeState) P.state[kNodeState * i + tid] = 0;
 }
 
 // R_q rows of every incidence (one warp per row) and the largest finite one.
@@ -151,31 +139,36 @@ __global__ void __launch_bounds__(kThreads) lift_rows_kernel(const NodeBuild P) 
         if (lane == 0) atomicMax(&s_max, (int)mx);
     }
     __syncthreads();
-    if (threadIdx.x == 0 && s_max) atomicMax(P.vmax + 4 * i, s_max);
+    if (threadIdx.x == 0 && s_max) atomicMax(P.state + kNodeState * i, s_max);
 }
 
-// T0 in 64 x 64 tiles (INF beyond the node's edges, up to the 128-tile edge).
+// T0 in 16 x 64 tiles (INF beyond the node's edges, up to the 128-tile edge)
+// and its largest finite value.
 __global__ void __launch_bounds__(kThreads) seam_block_kernel(const NodeBuild P) {
-    __shared__ int4 er[64], ec[64];
+    __shared__ int4 er[16], ec[64];
+    __shared__ int s_max;
     const int i = blockIdx.y, g2 = P.g * P.g, tid = threadIdx.x;
     if (P.active && !P.active[i]) return;
     const int nE = P.cnt[(size_t)i * (1 + g2)];
     const int tiles = P.TP / 64, I = blockIdx.x / tiles, J = blockIdx.x % tiles;
-    const int used = (nE + 127) / 128 * 128;
-    if (I * 64 >= used || J * 64 >= used) return;
+    const int used = min(P.TP, (nE + 127) / 128 * 128);
+    if (I * 16 >= used || J * 64 >= used) return;
     const int4* edge = P.edge + (size_t)i * P.TP;
-    if (tid < 64) {
-        if (I * 64 + tid < nE) er[tid] = edge[I * 64 + tid];
-    } else if (tid < 128) {
+    if (tid < 16) {
+        if (I * 16 + tid < nE) er[tid] = edge[I * 16 + tid];
+    } else if (tid >= 64 && tid < 128) {
         if (J * 64 + tid - 64 < nE) ec[tid - 64] = edge[J * 64 + tid - 64];
     }
+    if (tid == 0) s_max = 0;
     __syncthreads();
     const uint16_t* R = P.R + (size_t)i * g2 * P.capI * P.RP;
     uint16_t* T = P.T + (size_t)i * P.TP * P.TP;
-    for (int idx = tid; idx < 64 * 64; idx += kThreads) {
-        const int a = idx >> 6, c = idx & 63;
+    uint32_t mx = 0;
+#pragma unroll
+    for (int x4 = 0; x4 < 4; ++x4) {
+        const int a = (tid >> 6) + 4 * x4, c = tid & 63;
         uint32_t v = INF;
-        if (I * 64 + a < nE && J * 64 + c < nE) {
+        if (I * 16 + a < nE && J * 64 + c < nE) {
             const int4 r = er[a], k = ec[c];
             const int qr[2] = {r.x & 255, r.x >> 8}, qc[2] = {k.x & 255, k.x >> 8};
             const int ir[2] = {r.y & 0xffff, (int)((unsigned)r.y >> 16)};
@@ -187,65 +180,105 @@ __global__ void __launch_bounds__(kThreads) seam_block_kernel(const NodeBuild P)
                     if (qr[x] == qc[y])
                         v = min(v, sat_add(R[((size_t)qr[x] * P.capI + ir[x]) * P.RP + xc[y]], y ? (uint32_t)k.w : 0u));
         }
-        T[(size_t)(I * 64 + a) * P.TP + J * 64 + c] = (uint16_t)v;
+        T[(size_t)(I * 16 + a) * P.TP + J * 64 + c] = (uint16_t)v;
+        if (v < INF) mx = max(mx, v);
     }
+    mx = __reduce_max_sync(FULL, mx);
+    if ((tid & 31) == 0 && mx) atomicMax(&s_max, (int)mx);
+    __syncthreads();
+    if (tid == 0 && s_max) atomicMax(P.state + kNodeState * i + 1, s_max);
 }
 
 // ---------------------------------------------------------------------------
-// Min-plus product of one TM x TN tile (TM = 8 RW, TN = 64 CP, 8 warps):
-//   acc[r][c] = min(acc[r][c], min_k A_k[row r] (+) B_k[column pair c]),  k < K
-// A_k = arow(k) (8-column chunks from a_lim on are taken from the row's start:
-// their results are not used), B_k = Bp + k ldb (b_lim alike).  Warp w owns
-// rows RW w .. RW w + RW - 1, a lane CP column pairs.  Steps come in chunks of
-// kKC, double-buffered: the A rows through registers, splatted so that a row
-// value is one broadcast word, the B rows by cp.async.
+// Min-plus product of one TM x TN tile (TM = W RW, TN = 64 CP, W warps):
+//   acc[r][c] = min(acc[r][c], min_k A[arow(k)][row r] (+) Bp[k][column pair c]),  k < K
+// (8-column chunks of an operand row from a_lim / b_lim on are taken from its
+// start: their results are not used).  Warp w owns rows RW w .. RW w + RW - 1, a
+// lane CP column pairs.  Steps come in chunks of kKC rows; kDepth chunks are in
+// flight by cp.async (one chunk takes about 1000 cycles to use, less than its
+// L2 round trip), and the gather index of a row is loaded a chunk before its row.
+// Each thread splats the A values it copied itself, so that a row value is one
+// broadcast word of 32 bits: no barrier between arrival and splat.
 // half: every finite operand is <= kHalfMax, INF is taken as kHalfInf and no
 // sum needs a clamp (results >= kHalfInf mean INF).  Otherwise each step of a
 // warp is skipped (its rows all INF), unclamped (all <= INF_HEADROOM) or clamped.
+// KS = 2: two groups of W warps take half of every chunk's steps each and trade
+// halves of their rows at the end, so 64 x 64 tiles (of which there are few
+// when a closure or a single node is all there is to do) have 8 warps to hide
+// latencies: a closure pass over 390 seams, 16 nodes, 48 -> 44 us, over 195, 64 nodes, 33 -> 25 us.
+// Ends with this warp's rows of the result in out: rows first_row() and on.
 // ---------------------------------------------------------------------------
 constexpr int kKC = 32;
+constexpr int kDepth = 3;
 
-template <int RW, int CP>
+template <int RW, int CP, int W>
 constexpr size_t tile_smem_bytes() {
-    return 2 * (size_t)kKC * (8 * RW * sizeof(uint32_t) + 64 * CP * sizeof(uint16_t) + kWarps);
+    return (size_t)kKC * (2 * W * RW * sizeof(uint32_t) + kDepth * (W * RW + 64 * CP) * sizeof(uint16_t) + 2 * W);
 }
 
-template <int RW, int CP, class ARow>
-__device__ __forceinline__ void tile_minplus(uint32_t (&acc)[RW][CP], ARow arow, int a_lim, const uint16_t* Bp,
-                                             size_t ldb, int b_lim, int K, bool half, unsigned char* smem) {
-    constexpr int TM = 8 * RW, TN = 64 * CP;
-    constexpr int NA = kKC * (TM / 8) / kThreads, NB = kKC * (TN / 8) / kThreads;
-    static_assert(NA * kThreads == kKC * (TM / 8) && NB * kThreads == kKC * (TN / 8), "whole chunks per thread");
-    uint32_t* As = reinterpret_cast<uint32_t*>(smem);
-    uint16_t* Bs = reinterpret_cast<uint16_t*>(As + 2 * kKC * TM);
-    uint8_t* cls = reinterpret_cast<uint8_t*>(Bs + 2 * kKC * TN);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+template <int RW, int W, int KS>
+__device__ __forceinline__ int first_row() {
+    const int warp = threadIdx.x >> 5;
+    return (warp % W) * RW + (warp / W) * (RW / KS);
+}
+
+template <int RW, int CP, int W, int KS, class ARow>
+__device__ __forceinline__ void tile_minplus(uint32_t (&out)[RW / KS][CP], ARow arow, const uint16_t* A, size_t lda,
+                                             int a_lim, const uint16_t* Bp, size_t ldb, int b_lim, int K, bool half,
+                                             unsigned char* smem) {
+    constexpr int TM = W * RW, TN = 64 * CP, NT = 32 * W * KS;
+    constexpr int NA = kKC * (TM / 8) / NT, NB = kKC * (TN / 8) / NT;
+    static_assert(NA * NT == kKC * (TM / 8) && NB * NT == kKC * (TN / 8), "whole chunks per thread");
+    uint32_t* As = reinterpret_cast<uint32_t*>(smem);                // [2][kKC][TM] splatted
+    uint16_t* Ar = reinterpret_cast<uint16_t*>(As + 2 * kKC * TM);   // [kDepth][kKC][TM] as read
+    uint16_t* Bs = Ar + kDepth * kKC * TM;                           // [kDepth][kKC][TN]
+    uint8_t* cls = reinterpret_cast<uint8_t*>(Bs + kDepth * kKC * TN);  // [2][kKC][W]
+    const int tid = threadIdx.x, warp = (tid >> 5) % W, lane = tid & 31, group = tid / (32 * W);
     const int n_c = (K + kKC - 1) / kKC;
-    uint4 va[NA];
-    auto load = [&](int c) {
+    uint32_t acc[RW][CP];
+#pragma unroll
+    for (int r = 0; r < RW; ++r)
+#pragma unroll
+        for (int c = 0; c < CP; ++c) acc[r][c] = INF2;
+    int at[NA];  // rows of the next chunk to load
+    auto index = [&](int c) {
 #pragma unroll
         for (int x = 0; x < NA; ++x) {
-            const int idx = tid + x * kThreads, k = c * kKC + idx / (TM / 8), c8 = (idx % (TM / 8)) * 8;
-            va[x] = make_uint4(INF2, INF2, INF2, INF2);
-            if (k < K) va[x] = *reinterpret_cast<const uint4*>(arow(k) + (c8 < a_lim ? c8 : 0));
+            const int k = c * kKC + (tid + x * NT) / (TM / 8);
+            at[x] = k < K ? arow(k) : 0;
         }
+    };
+    auto load = [&](int c) {
+        if (c < n_c) {
+            const int st = c % kDepth;
 #pragma unroll
-        for (int x = 0; x < NB; ++x) {
-            const int idx = tid + x * kThreads, kk = idx / (TN / 8), c8 = (idx % (TN / 8)) * 8;
-            if (c * kKC + kk < K)
-                cp_async16(Bs + (size_t)((c & 1) * kKC + kk) * TN + c8,
-                           Bp + (size_t)(c * kKC + kk) * ldb + (c8 < b_lim ? c8 : 0));
+            for (int x = 0; x < NA; ++x) {
+                const int idx = tid + x * NT, c8 = (idx % (TM / 8)) * 8;
+                if (c * kKC + idx / (TM / 8) < K)
+                    cp_async16(Ar + st * kKC * TM + idx * 8, A + (size_t)at[x] * lda + (c8 < a_lim ? c8 : 0));
+            }
+#pragma unroll
+            for (int x = 0; x < NB; ++x) {
+                const int idx = tid + x * NT, kk = idx / (TN / 8), c8 = (idx % (TN / 8)) * 8;
+                if (c * kKC + kk < K)
+                    cp_async16(Bs + st * kKC * TN + idx * 8, Bp + (size_t)(c * kKC + kk) * ldb + (c8 < b_lim ? c8 : 0));
+            }
+            index(c + 1);
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    if (n_c > 0) load(0);
+    index(0);
+#pragma unroll
+    for (int c = 0; c < kDepth - 1; ++c) load(c);
     for (int c = 0; c < n_c; ++c) {
         uint32_t* Ab = As + (c & 1) * kKC * TM;
-        uint8_t* cb = cls + (c & 1) * kKC * kWarps;
+        uint8_t* cb = cls + (c & 1) * kKC * W;
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kDepth - 2) : "memory");
 #pragma unroll
-        for (int x = 0; x < NA; ++x) {
-            const int idx = tid + x * kThreads, kk = idx / (TM / 8), c8 = idx % (TM / 8);
-            uint32_t w[4] = {va[x].x, va[x].y, va[x].z, va[x].w};
+        for (int x = 0; x < NA; ++x) {  // rows beyond K: not read below
+            const int idx = tid + x * NT, kk = idx / (TM / 8), c8 = idx % (TM / 8);
+            const uint4 v = *reinterpret_cast<const uint4*>(Ar + (c % kDepth) * kKC * TM + idx * 8);
+            uint32_t w[4] = {v.x, v.y, v.z, v.w};
             if (half) {
 #pragma unroll
                 for (int t = 0; t < 4; ++t) w[t] = min2(w[t], kHalfInf2);
@@ -262,17 +295,17 @@ __device__ __forceinline__ void tile_minplus(uint32_t (&acc)[RW][CP], ARow arow,
                 }
                 mn = min(mn & 0xffffu, mn >> 16);
                 mx = max(mx & 0xffffu, mx >> 16);
-                cb[kk * kWarps + c8 / (RW / 8)] = mn >= INF ? 0 : (mx <= INF_HEADROOM ? 1 : 2);
+                cb[kk * W + c8 / (RW / 8)] = mn >= INF ? 0 : (mx <= INF_HEADROOM ? 1 : 2);
             }
-            uint4* dst = reinterpret_cast<uint4*>(Ab + kk * TM + c8 * 8);
+            uint4* dst = reinterpret_cast<uint4*>(Ab + idx * 8);
             dst[0] = make_uint4(splat(w[0]), splat(w[0] >> 16), splat(w[1]), splat(w[1] >> 16));
             dst[1] = make_uint4(splat(w[2]), splat(w[2] >> 16), splat(w[3]), splat(w[3] >> 16));
         }
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();  // chunk c is staged; every warp is done with chunk c - 1
-        if (c + 1 < n_c) load(c + 1);
-        const int kn = min(kKC, K - c * kKC);
-        const uint32_t* bp = reinterpret_cast<const uint32_t*>(Bs + (size_t)(c & 1) * kKC * TN) + lane * CP;
+        load(c + kDepth - 1);
+        constexpr int KG = kKC / KS;
+        const int k0 = group * KG, kn = min(k0 + KG, K - c * kKC);
+        const uint32_t* bp = reinterpret_cast<const uint32_t*>(Bs + (c % kDepth) * kKC * TN) + lane * CP;
         const uint32_t* ap = Ab + warp * RW;
         auto step = [&](int k, auto mode) {
             constexpr int M = decltype(mode)::value;  // 0 half range, 1 unclamped, 2 clamped
@@ -303,10 +336,10 @@ __device__ __forceinline__ void tile_minplus(uint32_t (&acc)[RW][CP], ARow arow,
         };
         if (half) {
 #pragma unroll 4
-            for (int k = 0; k < kn; ++k) step(k, std::integral_constant<int, 0>());
+            for (int k = k0; k < kn; ++k) step(k, std::integral_constant<int, 0>());
         } else {
-            for (int k = 0; k < kn; ++k) {
-                const int cl = cb[k * kWarps + warp];
+            for (int k = k0; k < kn; ++k) {
+                const int cl = cb[k * W + warp];
                 if (cl == 0) continue;  // uniform over the warp
                 if (cl == 1) step(k, std::integral_constant<int, 1>());
                 else step(k, std::integral_constant<int, 2>());
@@ -314,13 +347,35 @@ __device__ __forceinline__ void tile_minplus(uint32_t (&acc)[RW][CP], ARow arow,
         }
     }
     __syncthreads();  // the staging buffers are free
-    if (half) {
+    if constexpr (KS == 1) {
 #pragma unroll
         for (int r = 0; r < RW; ++r)
 #pragma unroll
-            for (int cc = 0; cc < CP; ++cc) {
-                const uint32_t lo = acc[r][cc] & 0xffffu, hi = acc[r][cc] >> 16;
-                acc[r][cc] = (lo >= kHalfInf ? (uint32_t)INF : lo) | ((hi >= kHalfInf ? (uint32_t)INF : hi) << 16);
+            for (int c = 0; c < CP; ++c) out[r][c] = acc[r][c];
+    } else {
+        static_assert(KS == 2, "two groups trade halves");
+        constexpr int RH = RW / 2;
+        uint32_t* ex = reinterpret_cast<uint32_t*>(smem) + (tid >> 5) * RH * CP * 32 + lane;
+        const uint32_t* other =
+            reinterpret_cast<const uint32_t*>(smem) + (warp + (1 - group) * W) * RH * CP * 32 + lane;
+#pragma unroll
+        for (int r = 0; r < RH; ++r)
+#pragma unroll
+            for (int c = 0; c < CP; ++c) ex[(r * CP + c) * 32] = group ? acc[r][c] : acc[RH + r][c];
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < RH; ++r)
+#pragma unroll
+            for (int c = 0; c < CP; ++c) out[r][c] = min2(group ? acc[RH + r][c] : acc[r][c], other[(r * CP + c) * 32]);
+        __syncthreads();
+    }
+    if (half) {
+#pragma unroll
+        for (int r = 0; r < RW / KS; ++r)
+#pragma unroll
+            for (int c = 0; c < CP; ++c) {
+                const uint32_t lo = out[r][c] & 0xffffu, hi = out[r][c] >> 16;
+                out[r][c] = (lo >= kHalfInf ? (uint32_t)INF : lo) | ((hi >= kHalfInf ? (uint32_t)INF : hi) << 16);
             }
     }
 }
@@ -329,10 +384,9 @@ __device__ __forceinline__ void tile_minplus(uint32_t (&acc)[RW][CP], ARow arow,
 // 16-byte chunks of 8 rows i.  Chunk q of row j sits at q ^ ((j / (2 CP)) & 7), so
 // the 8 lanes of a 16-byte store phase (8 different rows) hit 8 different
 // bank groups.  transposed_chunk reads chunk q of row j.
-template <int RW, int CP>
-__device__ __forceinline__ void transpose_store(uint16_t* Tt, const uint32_t (&acc)[RW][CP]) {
-    constexpr int TM = 8 * RW;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+template <int TM, int RW, int CP>
+__device__ __forceinline__ void transpose_store(uint16_t* Tt, const uint32_t (&acc)[RW][CP], int row0) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int cc = 0; cc < CP; ++cc)
 #pragma unroll
@@ -345,7 +399,7 @@ __device__ __forceinline__ void transpose_store(uint16_t* Tt, const uint32_t (&a
 #pragma unroll
                 for (int t = 0; t < 4; ++t)
                     w4[t] = __byte_perm(acc[8 * h + 2 * t][cc], acc[8 * h + 2 * t + 1][cc], x ? 0x7632 : 0x5410);
-                const int q = warp * (RW / 8) + h;
+                const int q = row0 / 8 + h;
                 *reinterpret_cast<uint4*>(Tt + j * TM + ((q ^ key) * 8)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
             }
         }
@@ -355,151 +409,85 @@ __device__ __forceinline__ uint4 transposed_chunk(const uint16_t* Tt, int j, int
     return *reinterpret_cast<const uint4*>(Tt + j * TM + ((q ^ ((j / (2 * CP)) & 7)) * 8));
 }
 
-template <int RW, int CP>
-__device__ __forceinline__ void fill_inf(uint32_t (&acc)[RW][CP]) {
-#pragma unroll
-    for (int r = 0; r < RW; ++r)
-#pragma unroll
-        for (int c = 0; c < CP; ++c) acc[r][c] = INF2;
-}
-
 // ---------------------------------------------------------------------------
-// Closure of T, stage t of one launch per stage: the panel units of round t
-// (64-column tiles) and the update units of round t - 1 (upper-triangle tile
-// pairs) side by side; a panel applies round t - 1's update to its own rows
-// itself (from round t - 1's panel), so the two only meet at the next launch.
-// The rows a panel reads may or may not hold that update yet: the minimum is
-// the updated value either way.
+// Closure of T by repeated squaring, in place: pass t takes T = min(T, T (x) T)
+// over the upper-triangle 64 x 64 tiles, each also written transposed,
+// so after t passes T holds every path of 2^t seam crossings.  A tile reads
+// entries that other tiles of the pass may be lowering: an entry is the
+// length of some path either way and at most its value before the pass, which is
+// all a pass needs.  A node whose last pass changed nothing is closed and its later
+// passes return at once: a street map needs 3 or 4 passes (few crossings
+// on any shortest path), the worst case is log2 of the seams.  The blocked
+// Floyd-Warshall this replaces needed a dependent launch per 64 seams at 25 us each
+// whatever the map (1024 x 1024, b = 8: 56 launches, 1.46 ms); a pass over 280
+// seams takes about as long as one of them.
 // ---------------------------------------------------------------------------
-constexpr size_t kStagePanelSmem = ((size_t)3 * B * kTLD + (size_t)B * 64) * sizeof(uint16_t) + (size_t)B * kWarps;
+constexpr int kSquareThreads = 256;
 
-__device__ void stage_panel(const NodeBuild& P, int i, int nE, int j0, int t, unsigned char* smem) {
-    uint16_t (*Ts)[kTLD] = reinterpret_cast<uint16_t (*)[kTLD]>(smem);
-    uint16_t (*Ag)[kTLD] = Ts + B;  // old panel at the pivot columns
-    uint16_t (*Bt)[kTLD] = Ag + B;  // the tile's pivot rows
-    uint16_t* Pj = &Bt[B][0];       // old panel at the tile's columns
-    uint8_t* cls = reinterpret_cast<uint8_t*>(Pj + B * 64);
-    const int tid = threadIdx.x, TP = P.TP, k0 = t * B, mk = min(B, nE - k0);
-    const bool ahead = t > 0;
-    const uint16_t* T = P.T + (size_t)i * TP * TP;
-    const uint16_t* Pp = P.P + ((size_t)((t - 1) & 1) * P.n + i) * B * TP;
-    for (int idx = tid; idx < B * 8; idx += kThreads) {
-        const int a = idx >> 3, c = (idx & 7) * 8;
-        cp_async16(&Ts[a][c], T + (size_t)(k0 + a) * TP + k0 + c);
-        cp_async16(&Bt[a][c], T + (size_t)(k0 + a) * TP + j0 + c);
-        if (ahead) {
-            cp_async16(&Ag[a][c], Pp + (size_t)a * TP + k0 + c);
-            cp_async16(Pj + a * 64 + c, Pp + (size_t)a * TP + j0 + c);
+__global__ void __launch_bounds__(kSquareThreads) seam_square_kernel(const NodeBuild P, int t) {
+    constexpr int TT = 64;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_max, s_chg, s_half;
+    const int i = blockIdx.y;
+    if (P.active && !P.active[i]) return;
+    int* state = P.state + kNodeState * i;
+    if (t > 0 && state[kNodeChanged + t - 1] == 0) return;  // closed
+    const int nE = P.cnt[(size_t)i * (1 + P.g * P.g)], nt = (nE + TT - 1) / TT;
+    if ((int)blockIdx.x >= nt * (nt + 1) / 2) return;
+    int I, J;
+    tri_pair(blockIdx.x, nt, I, J);
+    const int tid = threadIdx.x, lane = tid & 31, row0 = first_row<16, 4, 2>(), TP = P.TP;
+    uint16_t* T = P.T + (size_t)i * TP * TP;
+    // values found in this pass may exceed the maximum read here: their entries
+    // were INF before the pass, so taking a sum with one as INF loses nothing
+    if (tid == 0) {
+        s_max = s_chg = 0;
+        s_half = *(volatile int*)(state + 1) <= kHalfMax;  // one value for the CTA: the pass raises it
+    }
+    __syncthreads();
+    const bool half = s_half != 0;
+    uint32_t acc[8][1], old[8];  // the old tile: no other CTA writes it
+    uint32_t* d0 = reinterpret_cast<uint32_t*>(T + (size_t)(I * TT + row0) * TP + J * TT) + lane;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) old[r] = __ldcg(d0 + (size_t)r * (TP / 2));
+    tile_minplus<16, 1, 4, 2>(acc, [](int k) { return k; }, T + I * TT, TP, TP - I * TT, T + J * TT, TP, TP - J * TT, nE,
+                           half, smem);
+    bool chg = false;
+    uint32_t mx = 0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        acc[r][0] = min2(acc[r][0], old[r]);
+        if (acc[r][0] != old[r]) {
+            d0[(size_t)r * (TP / 2)] = acc[r][0];
+            chg = true;
+            const uint32_t lo = acc[r][0] & 0xffffu, hi = acc[r][0] >> 16;
+            if (lo < INF) mx = max(mx, lo);
+            if (hi < INF) mx = max(mx, hi);
         }
     }
-    cp_async_wait_all();
+    mx = __reduce_max_sync(FULL, mx);
+    if (lane == 0 && mx) atomicMax(&s_max, (int)mx);
+    if (chg) s_chg = 1;
     __syncthreads();
-    if (ahead) {
-        uint32_t acc[2][4];
-        block_classes(Ag, B, cls);
-        __syncthreads();
-        gemm64(Ag, &Ag[0][0], kTLD, B, cls, acc);
-        min_into(&Ts[0][0], kTLD, B, acc);
-        gemm64(Ag, Pj, 64, B, cls, acc);
-        min_into(&Bt[0][0], kTLD, B, acc);
-        __syncthreads();
-    }
-    uint32_t vb[8];
-    close_pivot_panel(Ts, Bt, mk, vb);
-    uint16_t* out = P.P + ((size_t)(t & 1) * P.n + i) * B * TP;
-    const int a = tid >> 2, c0 = (tid & 3) * 16;
-    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)a * TP + j0 + c0);
-    if (a >= mk) {
-#pragma unroll
-        for (int x = 0; x < 8; ++x) vb[x] = INF2;
-    }
-    dst[0] = make_uint4(vb[0], vb[1], vb[2], vb[3]);
-    dst[1] = make_uint4(vb[4], vb[5], vb[6], vb[7]);
-}
-
-template <int RW, int CP>
-__device__ void stage_update(const NodeBuild& P, int i, int nE, int I, int J, int t, unsigned char* smem) {
-    constexpr int TT = 8 * RW;
-    static_assert(TT == 64 * CP, "square tiles");
-    const int TP = P.TP, mk = min(B, nE - t * B);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint16_t* T = P.T + (size_t)i * TP * TP;
-    const uint16_t* Pp = P.P + ((size_t)(t & 1) * P.n + i) * B * TP;
-    uint32_t acc[RW][CP];
-#pragma unroll
-    for (int r = 0; r < RW; ++r) {
-        const uint32_t* row = reinterpret_cast<const uint32_t*>(T + (size_t)(I * TT + warp * RW + r) * TP + J * TT);
-#pragma unroll
-        for (int c = 0; c < CP; ++c) acc[r][c] = row[lane * CP + c];
-    }
-    tile_minplus<RW, CP>(acc, [&](int k) { return Pp + (size_t)k * TP + I * TT; }, TP - I * TT, Pp + J * TT, TP,
-                         TP - J * TT, mk, false, smem);
-#pragma unroll
-    for (int r = 0; r < RW; ++r) {
-        uint32_t* row = reinterpret_cast<uint32_t*>(T + (size_t)(I * TT + warp * RW + r) * TP + J * TT);
-#pragma unroll
-        for (int c = 0; c < CP; ++c) row[lane * CP + c] = acc[r][c];
+    if (!s_chg) return;
+    if (tid == 0) {
+        atomicMax(state + 1, s_max);
+        state[kNodeChanged + t] = 1;
     }
     if (I == J) return;
     uint16_t* Tt = reinterpret_cast<uint16_t*>(smem);
-    transpose_store<RW, CP>(Tt, acc);
+    transpose_store<TT, 8, 1>(Tt, acc, row0);
     __syncthreads();
-    for (int idx = threadIdx.x; idx < TT * (TT / 8); idx += kThreads) {
+    for (int idx = tid; idx < TT * (TT / 8); idx += kSquareThreads) {
         const int j = idx / (TT / 8), q = idx % (TT / 8);
-        reinterpret_cast<uint4*>(T + (size_t)(J * TT + j) * TP + I * TT)[q] = transposed_chunk<TT, CP>(Tt, j, q);
+        reinterpret_cast<uint4*>(T + (size_t)(J * TT + j) * TP + I * TT)[q] = transposed_chunk<TT, 1>(Tt, j, q);
     }
-}
-
-__global__ void __launch_bounds__(kThreads, 2) seam_stage_kernel(const NodeBuild P, int t) {
-    extern __shared__ __align__(16) unsigned char nsm[];
-    const int i = blockIdx.y;
-    if (P.active && !P.active[i]) return;
-    const int nE = P.cnt[(size_t)i * (1 + P.g * P.g)];
-    const int rounds = (nE + B - 1) / B;
-    if (t > rounds) return;
-    // the panel covers whole update tiles
-    const int n_panel = t < rounds ? (P.TP >= 128 ? (nE + 127) / 128 * 2 : 1) : 0;
-    int u = blockIdx.x;
-    if (u < n_panel) {
-        stage_panel(P, i, nE, u * 64, t, nsm);
-        return;
-    }
-    u -= n_panel;
-    const int TT = P.TP >= 128 ? 128 : 64;
-    const int nt = (nE + TT - 1) / TT;
-    if (t == 0 || u >= nt * (nt + 1) / 2) return;
-    int I, J;
-    tri_pair(u, nt, I, J);
-    if (TT == 128) stage_update<16, 2>(P, i, nE, I, J, t - 1, nsm);
-    else stage_update<8, 1>(P, i, nE, I, J, t - 1, nsm);
-}
-
-// Largest finite value of every node's T (one 64-row strip per CTA).
-__global__ void __launch_bounds__(kThreads) seam_max_kernel(const NodeBuild P) {
-    const int i = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (P.active && !P.active[i]) return;
-    const int nE = P.cnt[(size_t)i * (1 + P.g * P.g)];
-    const uint16_t* T = P.T + (size_t)i * P.TP * P.TP;
-    uint32_t mx = 0;
-    for (int r = blockIdx.x * 64 + warp; r < min(nE, (int)blockIdx.x * 64 + 64); r += kWarps)
-        for (int c = lane * 8; c < nE; c += 256) {
-            const uint4 v = *reinterpret_cast<const uint4*>(T + (size_t)r * P.TP + c);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const uint32_t lo = w[t] & 0xffffu, hi = w[t] >> 16;
-                if (lo < INF) mx = max(mx, lo);
-                if (hi < INF) mx = max(mx, hi);
-            }
-        }
-    mx = __reduce_max_sync(FULL, mx);
-    if (lane == 0 && mx) atomicMax(P.vmax + 4 * i + 1, (int)mx);
 }
 
 // U_p tiles: rows = edges, columns = ports of child p.
-template <int RW, int CP>
-__global__ void __launch_bounds__(kThreads, 2) lift_kernel(const NodeBuild P) {
-    constexpr int TM = 8 * RW, TN = 64 * CP;
+template <int RW, int CP, int W, int KS>
+__global__ void __launch_bounds__(32 * W * KS, 2) lift_kernel(const NodeBuild P) {
+    constexpr int TM = W * RW, TN = 64 * CP, NR = RW / KS;
     extern __shared__ __align__(16) unsigned char nsm[];
     __shared__ int s_max;
     const int i = blockIdx.z, p = blockIdx.y, g2 = P.g * P.g;
@@ -508,23 +496,22 @@ __global__ void __launch_bounds__(kThreads, 2) lift_kernel(const NodeBuild P) {
     const int tn = (P.RP + TN - 1) / TN;
     const int m0 = (blockIdx.x / tn) * TM, n0 = (blockIdx.x % tn) * TN;
     if (m0 >= cnt[0]) return;
-    const int* vm = P.vmax + 4 * i;
+    const int* vm = P.state + kNodeState * i;
     const bool half = max(vm[0], vm[1]) <= kHalfMax;
     const uint2* inc = P.inc + ((size_t)i * g2 + p) * P.capI;
     const uint16_t* T = P.T + (size_t)i * P.TP * P.TP;
     const uint16_t* R = P.R + ((size_t)i * g2 + p) * P.capI * P.RP;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t acc[RW][CP];
-    fill_inf<RW, CP>(acc);
+    const int row0 = first_row<RW, W, KS>(), lane = threadIdx.x & 31;
+    uint32_t acc[NR][CP];
     if (threadIdx.x == 0) s_max = 0;
-    tile_minplus<RW, CP>(acc, [&](int k) { return T + (size_t)inc[k].y * P.TP + m0; }, P.TP - m0, R + n0, P.RP,
-                         P.RP - n0, cnt[1 + p], half, nsm);
+    tile_minplus<RW, CP, W, KS>(acc, [&](int k) { return (int)inc[k].y; }, T + m0, P.TP, P.TP - m0, R + n0, P.RP,
+                            P.RP - n0, cnt[1 + p], half, nsm);
     uint16_t* U = P.U + ((size_t)i * g2 + p) * P.TP * P.RP;
     uint32_t mx = 0;
     const int col = n0 + lane * 2 * CP;
 #pragma unroll
-    for (int r = 0; r < RW; ++r) {
-        const int e = m0 + warp * RW + r;
+    for (int r = 0; r < NR; ++r) {
+        const int e = m0 + row0 + r;
 #pragma unroll
         for (int c = 0; c < CP; ++c) {
             if (col + 2 * c >= P.RP) continue;
@@ -538,13 +525,13 @@ __global__ void __launch_bounds__(kThreads, 2) lift_kernel(const NodeBuild P) {
     __syncthreads();
     if (lane == 0 && mx) atomicMax(&s_max, (int)mx);
     __syncthreads();
-    if (threadIdx.x == 0 && s_max) atomicMax(P.vmax + 4 * i + 2, s_max);
+    if (threadIdx.x == 0 && s_max) atomicMax(P.state + kNodeState * i + 2, s_max);
 }
 
 // D tiles: unit = (children p <= q, tile of p's ports x tile of q's ports).
-template <int RW, int CP>
-__global__ void __launch_bounds__(kThreads, 2) node_tile_kernel(const NodeBuild P) {
-    constexpr int TM = 8 * RW, TN = 64 * CP;
+template <int RW, int CP, int W, int KS>
+__global__ void __launch_bounds__(32 * W * KS, 2) node_tile_kernel(const NodeBuild P) {
+    constexpr int TM = W * RW, TN = 64 * CP, NR = RW / KS;
     static_assert(TM == TN, "square tiles");
     extern __shared__ __align__(16) unsigned char nsm[];
     __shared__ int s_chg;
@@ -563,17 +550,16 @@ __global__ void __launch_bounds__(kThreads, 2) node_tile_kernel(const NodeBuild 
         J = u % nt;
     }
     const int node = node_id(P, i), m0 = I * TM, n0 = J * TN;
-    const int* vm = P.vmax + 4 * i;
+    const int* vm = P.state + kNodeState * i;
     const bool half = max(vm[0], vm[2]) <= kHalfMax;
     const uint2* inc = P.inc + ((size_t)i * g2 + q) * P.capI;
     const uint16_t* U = P.U + ((size_t)i * g2 + p) * P.TP * P.RP + m0;
     const uint16_t* R = P.R + ((size_t)i * g2 + q) * P.capI * P.RP + n0;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t acc[RW][CP];
-    fill_inf<RW, CP>(acc);
+    const int row0 = first_row<RW, W, KS>(), lane = threadIdx.x & 31;
+    uint32_t acc[NR][CP];
     if (threadIdx.x == 0) s_chg = 0;
-    tile_minplus<RW, CP>(acc, [&](int k) { return U + (size_t)inc[k].y * P.RP; }, P.RP - m0, R, P.RP, P.RP - n0,
-                         P.cnt[(size_t)i * (1 + g2) + 1 + q], half, nsm);
+    tile_minplus<RW, CP, W, KS>(acc, [&](int k) { return (int)inc[k].y; }, U, P.RP, P.RP - m0, R, P.RP, P.RP - n0,
+                            P.cnt[(size_t)i * (1 + g2) + 1 + q], half, nsm);
     uint16_t* D = node_mat(P, node);
     const int col = n0 + lane * 2 * CP;  // port of q; nP is a multiple of 4
     if (p == q) {
@@ -582,28 +568,37 @@ __global__ void __launch_bounds__(kThreads, 2) node_tile_kernel(const NodeBuild 
 #pragma unroll
         for (int c = 0; c < 2 * CP; ++c) ce[c] = P.cext[min(col + c, nP - 1)];
 #pragma unroll
-        for (int r = 0; r < RW; ++r) {
-            const uint16_t* crow = cm + (size_t)P.cext[min(m0 + warp * RW + r, nP - 1)] * P.C.NP;
+        for (int r = 0; r < NR; ++r) {
+            const uint16_t* crow = cm + (size_t)P.cext[min(m0 + row0 + r, nP - 1)] * P.C.NP;
 #pragma unroll
             for (int c = 0; c < CP; ++c)
                 acc[r][c] = min2(acc[r][c], (uint32_t)crow[ce[2 * c]] | ((uint32_t)crow[ce[2 * c + 1]] << 16));
         }
     }
     bool chg = false;
+    if (P.changed && col < nP) {  // against the old matrix, before any store
+        uint32_t cext[CP];
+#pragma unroll
+        for (int c = 0; c < CP; ++c)
+            cext[c] = (P.isext[q * nP + col + 2 * c] ? 0xffffu : 0u) |
+                      (P.isext[q * nP + col + 2 * c + 1] ? 0xffff0000u : 0u);
+        uint32_t diff = 0;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const int row = p * nP + min(m0 + row0 + r, nP - 1);
+            const bool on = m0 + row0 + r < nP && P.isext[row];
+            const uint32_t* d = reinterpret_cast<const uint32_t*>(D + (size_t)row * NP + q * nP + col);
+#pragma unroll
+            for (int c = 0; c < CP; ++c) diff |= on ? (d[c] ^ acc[r][c]) & cext[c] : 0u;
+        }
+        chg = diff != 0;
+    }
     if (col < nP) {
 #pragma unroll
-        for (int r = 0; r < RW; ++r) {
-            const int row = m0 + warp * RW + r;
+        for (int r = 0; r < NR; ++r) {
+            const int row = m0 + row0 + r;
             if (row >= nP) continue;
             uint32_t* d = reinterpret_cast<uint32_t*>(D + (size_t)(p * nP + row) * NP + q * nP + col);
-            if (P.changed && P.isext[p * nP + row]) {
-#pragma unroll
-                for (int c = 0; c < CP; ++c) {
-                    const uint32_t diff = d[c] ^ acc[r][c];
-                    chg |= (diff & 0xffffu) && P.isext[q * nP + col + 2 * c];
-                    chg |= (diff >> 16) && P.isext[q * nP + col + 2 * c + 1];
-                }
-            }
             if constexpr (CP == 2) *reinterpret_cast<uint2*>(d) = make_uint2(acc[r][0], acc[r][1]);
             else d[0] = acc[r][0];
         }
@@ -615,9 +610,9 @@ __global__ void __launch_bounds__(kThreads, 2) node_tile_kernel(const NodeBuild 
     }
     if (p == q && I == J) return;
     uint16_t* Tt = reinterpret_cast<uint16_t*>(nsm);
-    transpose_store<RW, CP>(Tt, acc);
+    transpose_store<TM, NR, CP>(Tt, acc, row0);
     __syncthreads();
-    for (int idx = threadIdx.x; idx < TN * (TM / 8); idx += kThreads) {
+    for (int idx = threadIdx.x; idx < TN * (TM / 8); idx += 32 * W * KS) {
         const int j = idx / (TM / 8), c8 = idx % (TM / 8);
         if (n0 + j >= nP || m0 + c8 * 8 >= nP) continue;
         const uint4 v = transposed_chunk<TM, CP>(Tt, j, c8);
@@ -828,6 +823,23 @@ void allow_smem(K kernel, size_t bytes) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// U, then D.
+template <int RW, int CP, int W, int KS>
+void launch_products(const NodeBuild& P, int n, cudaStream_t st) {
+    constexpr int TM = W * RW, TN = 64 * CP;
+    const size_t smem = tile_smem_bytes<RW, CP, W>();
+    const int g2 = P.g * P.g, nt = (P.nP + TM - 1) / TM;
+    allow_smem(lift_kernel<RW, CP, W, KS>, smem);
+    allow_smem(node_tile_kernel<RW, CP, W, KS>, smem);
+    lift_kernel<RW, CP, W, KS><<<dim3(blocks_for(P.n_seams, TM) * blocks_for(P.RP, TN), g2, n), 32 * W * KS, smem, st>>>(P);
+    node_tile_kernel<RW, CP, W, KS>
+        <<<dim3(g2 * nt * (nt + 1) / 2 + g2 * (g2 - 1) / 2 * nt * nt, n), 32 * W * KS, smem, st>>>(P);
+}
+
+// Fewer 128 x 128 tiles than this leave SMs idle or with one CTA (8 warps), whose
+// latencies show.
+constexpr size_t kWideTiles = 2 * 148;
+
 }  // namespace
 
 void launch_pad_fill(MatSet M, int count, cudaStream_t st) {
@@ -854,21 +866,16 @@ size_t node_build_layout(NodeBuild& P, int n, unsigned char* base) {
         return p;
     };
     P.cnt = reinterpret_cast<int*>(take(n * (1 + g2) * sizeof(int)));
-    P.vmax = reinterpret_cast<int*>(take((size_t)n * 4 * sizeof(int)));
+    P.state = reinterpret_cast<int*>(take((size_t)n * kNodeState * sizeof(int)));
     P.edge = reinterpret_cast<int4*>(take((size_t)n * P.TP * sizeof(int4)));
     P.inc = reinterpret_cast<uint2*>(take(n * g2 * P.capI * sizeof(uint2)));
     P.R = reinterpret_cast<uint16_t*>(take(n * g2 * P.capI * P.RP * sizeof(uint16_t)));
     P.T = reinterpret_cast<uint16_t*>(take((size_t)n * P.TP * P.TP * sizeof(uint16_t)));
-    P.P = reinterpret_cast<uint16_t*>(take((size_t)2 * n * B * P.TP * sizeof(uint16_t)));
     P.U = reinterpret_cast<uint16_t*>(take(n * g2 * P.TP * P.RP * sizeof(uint16_t)));
     return off;
 }
 
-void launch_seam_count(const NodeBuild& P, int n, int* most, cudaStream_t st) {
-    if (n > 0) seam_count_kernel<<<n, 128, 0, st>>>(P, most);
-}
-
-void launch_node_build(const NodeBuild& P, int n, int most_seams, cudaStream_t st) {
+void launch_node_build(const NodeBuild& P, int n, cudaStream_t st) {
     if (n <= 0) return;
     const int g2 = P.g * P.g;
     if (node_build_small(P)) {
@@ -882,40 +889,22 @@ void launch_node_build(const NodeBuild& P, int n, int most_seams, cudaStream_t s
         }
         return;
     }
-    seam_list_kernel<<<n, 256, 0, st>>>(P);
-    const int cap = std::min(P.capI, most_seams);  // a child's incidences are distinct edges
-    const int rounds = (most_seams + B - 1) / B;
-    if (rounds > 0) {
-        lift_rows_kernel<<<dim3(blocks_for(cap, kWarps), g2, n), kThreads, 0, st>>>(P);
-        const unsigned tiles = P.TP / 64;
-        seam_block_kernel<<<dim3(tiles * tiles, n), kThreads, 0, st>>>(P);
-        const size_t smem = std::max(kStagePanelSmem, tile_smem_bytes<16, 2>());
-        allow_smem(seam_stage_kernel, smem);
-        const int nt = P.TP >= 128 ? (most_seams + 127) / 128 : 1;
-        for (int t = 0; t <= rounds; ++t) {
-            const int units = (t < rounds ? (P.TP >= 128 ? 2 * nt : 1) : 0) + (t > 0 ? nt * (nt + 1) / 2 : 0);
-            seam_stage_kernel<<<dim3(units, n), kThreads, smem, st>>>(P, t);
-        }
-        seam_max_kernel<<<dim3(rounds, n), kThreads, 0, st>>>(P);
-        // 64-wide tiles for children of up to 64 ports
-        if (P.nP <= 64) {
-            const size_t sm = tile_smem_bytes<8, 1>();
-            lift_kernel<8, 1><<<dim3(blocks_for(most_seams, 64) * blocks_for(P.RP, 64), g2, n), kThreads, sm, st>>>(P);
-        } else {
-            const size_t sm = tile_smem_bytes<16, 2>();
-            allow_smem(lift_kernel<16, 2>, sm);
-            lift_kernel<16, 2><<<dim3(blocks_for(most_seams, 128) * blocks_for(P.RP, 128), g2, n), kThreads, sm, st>>>(P);
-        }
-    }
-    const int TM = P.nP <= 64 ? 64 : 128;
-    const int nt = (P.nP + TM - 1) / TM;
-    const dim3 grid(g2 * nt * (nt + 1) / 2 + g2 * (g2 - 1) / 2 * nt * nt, n);
-    if (P.nP <= 64) {
-        node_tile_kernel<8, 1><<<grid, kThreads, tile_smem_bytes<8, 1>(), st>>>(P);
-    } else {
-        allow_smem(node_tile_kernel<16, 2>, tile_smem_bytes<16, 2>());
-        node_tile_kernel<16, 2><<<grid, kThreads, tile_smem_bytes<16, 2>(), st>>>(P);
-    }
+    // Grids cover every seam candidate: the active ones are counted on the device
+    // (CTAs beyond them return at once), so the host waits for nothing.
+    const int m = P.n_seams;
+    seam_list_kernel<<<n, std::min(1024, (m + 31) / 32 * 32), 0, st>>>(P);
+    lift_rows_kernel<<<dim3(blocks_for(P.capI, kWarps), g2, n), kThreads, 0, st>>>(P);
+    const unsigned tiles = P.TP / 64;
+    seam_block_kernel<<<dim3(4 * tiles * tiles, n), kThreads, 0, st>>>(P);
+    const unsigned nq = blocks_for(m, 64);
+    allow_smem(seam_square_kernel, tile_smem_bytes<16, 1, 4>());
+    for (int t = 0; (1 << t) < m; ++t)  // paths of up to m crossings
+        seam_square_kernel<<<dim3(nq * (nq + 1) / 2, n), kSquareThreads, tile_smem_bytes<16, 1, 4>(), st>>>(P, t);
+    // 128 x 128 tiles where they fill the chip, else 64 x 64 ones (four times the CTAs)
+    const int nt = (P.nP + 127) / 128;
+    const bool wide = P.nP > 64 && (size_t)n * (g2 * nt * (nt + 1) / 2 + g2 * (g2 - 1) / 2 * nt * nt) >= kWideTiles;
+    if (wide) launch_products<16, 2, 8, 1>(P, n, st);
+    else launch_products<16, 1, 4, 2>(P, n, st);
 }
 
 }  // namespace hb
