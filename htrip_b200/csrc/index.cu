@@ -1554,6 +1554,7 @@ struct QueryPlan {
     int ldm = 8;   // stride of the sorted-order M
     int cfg = 0;
     int o_vp0 = 0, o_inv = 0, o_l0 = 0, n_l0 = 0;
+    int chain = 0, o_chain = 0;  // QueryParams::chain and its table
     struct Lvl {
         int o_groups = 0, n_groups = 0, max_group = 0, slots = 0;
         int o_items = 0, n_items = 0, split = 1;
@@ -1604,6 +1605,19 @@ int query_split_items(const htrip_index* h) {
     auto it = grid.find(h->device);
     if (it == grid.end()) it = grid.emplace(h->device, hb::query_grid_blocks(h->device)).first;
     return it->second;
+}
+
+// Levels lifted viewpoint by viewpoint (QueryParams::chain): from the leaves
+// up, matrices of padded order <= 1024 (a viewpoint's rows are at most 0.5 MB,
+// read by one CTA in a few microseconds) while a child holds at most about 4
+// viewpoints: with more, the tiled project items read a matrix row once for RW
+// viewpoints.
+int query_chain(const htrip_index* h, int k) {
+    int c = 0;
+    while (c < std::min(h->H, hb::kMaxChain) && h->L[c + 1].NP <= hb::kMaxChainNP &&
+           (int64_t)k <= 4 * (int64_t)h->L[c].nnodes)
+        ++c;
+    return c;
 }
 
 // Plans a query; force_cfg >= 0 imposes the tile configuration (requests
@@ -1675,6 +1689,7 @@ void make_plan(const htrip_index* h, const int32_t* vps, const uint8_t* pass_fla
     P.cfg = force_cfg >= 0 ? force_cfg : choose_query_cfg(h, ns, H >= 1 ? P.lv[H].max_group : ns);
     const hb::QueryTile tile = hb::query_config_tile(P.cfg);
     const int RW = tile.RW, NC = tile.NCOL;
+    P.chain = query_chain(h, k);
     // Slot layout: every child group's run starts on an RW boundary.
     std::vector<std::vector<int>> slot_of(H + 1);
     int max_slots = ns;
@@ -1706,6 +1721,23 @@ void make_plan(const htrip_index* h, const int32_t* vps, const uint8_t* pass_fla
     } else {
         P.n_l0 = 0;
     }
+    P.o_chain = (int)P.buf.size();
+    if (P.chain > 0) {
+        P.buf.resize(P.buf.size() + (size_t)ns * hb::kChainInts, 0);
+        int* tab = P.buf.data() + P.o_chain;
+        int gl = 1;  // leaves per level-l node side
+        for (int l = 1; l <= std::min(P.chain + 1, H); ++l) {
+            gl *= g;
+            auto same = [&](int i, int j) { return v[i].tx / gl == v[j].tx / gl && v[i].ty / gl == v[j].ty / gl; };
+            for (int gi = 0; gi < (int)cgs[l].size(); ++gi)
+                for (int t = 0; t < cgs[l][gi].cnt; ++t) {
+                    const int i = cgs[l][gi].start + t;
+                    const bool shared = (i > 0 && same(i, i - 1)) || (i + 1 < ns && same(i, i + 1));
+                    tab[i * hb::kChainInts + 2 * (l - 1)] = slot_of[l][i];
+                    tab[i * hb::kChainInts + 2 * (l - 1) + 1] = 2 * gi + (shared ? 1 : 0);
+                }
+        }
+    }
     const int target_items = 296;
     for (int l = 1; l <= H; ++l) {
         const Level& Lv = h->L[l];
@@ -1716,7 +1748,7 @@ void make_plan(const htrip_index* h, const int32_t* vps, const uint8_t* pass_fla
         // project items; at the root a viewpoint of child q meets only
         // viewpoints of children >= q (i < j), so earlier blocks are skipped.
         Q.o_items = (int)P.buf.size();
-        for (int gi = 0; gi < (int)G.size(); ++gi) {
+        for (int gi = 0; gi < (int)G.size() && l > P.chain; ++gi) {
             const int n_begin = (l == H) ? (G[gi].quad * Lv.nP) / NC * NC : 0;
             for (int m0 = 0; m0 < G[gi].cnt; m0 += RW)
                 for (int n0 = n_begin; n0 < Lv.NP; n0 += NC) P.buf.insert(P.buf.end(), {gi, m0, n0});
@@ -1878,7 +1910,7 @@ void query_units(const htrip_index* h, const QueryPlan& P, int n_phases, int* un
     const int H = h->H;
     for (int t = 0; t < n_phases; ++t) units[t] = 0;
     const long fill = (long)P.n_l0 * h->L[0].nExt;
-    units[0] = (int)((fill + hb::kQueryL0Chunk - 1) / hb::kQueryL0Chunk) +
+    units[0] = (P.chain ? P.n_sorted : (int)((fill + hb::kQueryL0Chunk - 1) / hb::kQueryL0Chunk)) +
                (P.n_sorted + hb::kQueryThreads - 1) / hb::kQueryThreads;
     for (int t = 1; t <= H + 1; ++t)
         units[t] = (t <= H ? P.lv[t].n_items * P.lv[t].split : 0) + (t - 1 >= 1 ? P.lv[t - 1].n_meet : 0);
@@ -1902,6 +1934,10 @@ hb::QueryParams make_params(const htrip_index* h, const QueryPlan& P, unsigned c
     Q.vp0 = plan + P.o_vp0;
     Q.inv = plan + P.o_inv;
     Q.l0 = plan + P.o_l0;
+    Q.chain = P.chain;
+    Q.g = h->g;
+    Q.leaves_x = h->leaves_x;
+    Q.chain_tab = plan + P.o_chain;
     Q.ext0 = h->L[0].d_ext.p;
     Q.leaves = h->L[0].ms();
     for (int l = 0; l < H; ++l) Q.X[l] = reinterpret_cast<uint16_t*>(base + L.X[i][l]);
@@ -2167,6 +2203,7 @@ DevPlanLayout devplan_layout(const htrip_index* h, int k, int cfg, bool out_in_a
     G.RW = (int)RW;
     G.NC = (int)NC;
     G.nExt0 = h->L[0].nExt;
+    G.chain = query_chain(h, k);
     auto log2_exact = [](int v) {
         int sh = 0;
         while ((1 << sh) < v) ++sh;
@@ -2203,7 +2240,7 @@ DevPlanLayout devplan_layout(const htrip_index* h, int k, int cfg, bool out_in_a
         const long NP = h->L[l].NP;
         O.cap_groups[l] = (int)ngr;
         O.cap_slots[l] = (int)slots;
-        O.cap_items[l] = (int)(rows * ((NP + NC - 1) / NC));
+        O.cap_items[l] = l <= G.chain ? 0 : (int)(rows * ((NP + NC - 1) / NC));
         // meet base items: per group, ceil(span / NC) slot tiles x its row
         // tiles; the port split adds at most kPlanTargetItems
         O.cap_meet[l] = (int)(((span + NC - 1) / NC + 1) * rows + hb::kPlanTargetItems);
@@ -2213,6 +2250,7 @@ DevPlanLayout devplan_layout(const htrip_index* h, int k, int cfg, bool out_in_a
     O.o_vp0 = take(4 * (size_t)k);
     O.o_inv = take(k);
     O.o_rec = take(hb::plan_record_ints());
+    O.o_chain = take(H >= 1 ? (size_t)hb::kChainInts * k : 0);
     O.o_l0 = take(H >= 1 ? 2 * (size_t)O.cap_slots[1] : 0);
     for (int l = 1; l <= H; ++l) {
         O.o_groups[l] = take(5 * (size_t)O.cap_groups[l]);
@@ -3235,6 +3273,8 @@ static htrip_status arena_phases(const QueryArena& A, cudaStream_t st, uint64_t*
     ck(cudaMemcpyAsync(t, A.dev.p + A.last_words + kTraceOffset, sizeof(t), cudaMemcpyDeviceToHost, st), "trace d2h");
     ck(cudaStreamSynchronize(st), "trace sync");
     const int P = A.last_phases;
+    for (int i = 1; i <= P; ++i)  // a phase without units left no stamp: it ends with the one before
+        if (t[i] == 0) t[i] = t[i - 1];
     *n = std::min<int32_t>(max_n, P);
     for (int i = 0; i < *n; ++i) ns[i] = t[i + 1] > t[i] ? t[i + 1] - t[i] : 0;
     if (max_n >= 2 * P) {

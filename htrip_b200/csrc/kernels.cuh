@@ -228,6 +228,11 @@ cudaError_t launch_open(const OpenLaunch& L, int grid, cudaStream_t st);
 
 // --- query (query.cu) -------------------------------------------------------
 constexpr int kMaxQueryLevels = 16;
+// Levels 1 .. QueryParams::chain are lifted viewpoint by viewpoint (one CTA takes
+// a viewpoint through all of them, query.cu); at most this many, with matrices of at most
+// this padded order.
+constexpr int kMaxChain = 4, kMaxChainNP = 1024;
+constexpr int kChainInts = 2 * (kMaxChain + 1);
 constexpr int kNumQueryConfigs = 4;
 
 // Warp tile of a query work item: RW viewpoint rows x NCOL columns.
@@ -260,6 +265,9 @@ struct QueryLevel {
 // One queryAllPairs request of a launch.
 struct QueryParams {
     int H, k, ns, ldv, ldm, n_l0_slots, nExt0, cfg;
+    int chain, g, leaves_x;  // levels lifted by the chain units; group, leaves per row
+    const int* chain_tab;    // per sorted viewpoint, levels l = 1 .. min(chain + 1, H): {level-l slot,
+                             // level-l group * 2 + (its level-l node holds another viewpoint)}
     const int* vp0;         // per sorted viewpoint {leaf, u, leaf-run start, leaf-run end}
     const int* inv;         // original index -> sorted index or -1
     const int* l0;          // per level-1 slot {sorted index or -1, level-1 group}
@@ -291,7 +299,8 @@ inline size_t query_counter_words(int H, int k) { return 4 + (size_t)(H + 1) * (
 
 // CTA work units of a request in phase t of the launch (host and device
 // agree on these numbers):
-//   t = 0          level-0 port gathers in chunks of kQueryL0Chunk, then
+//   t = 0          chain > 0: one unit per viewpoint (levels 0 .. chain); else
+//                  level-0 port gathers in chunks of kQueryL0Chunk; then
 //                  same-leaf pair rows in chunks of kQueryThreads
 //   1 <= t <= H+1  project items of level t (t <= H; `split` units per
 //                  item, its parts in order), then meet items of level t-1
@@ -332,6 +341,7 @@ struct PlanGeom {
     int side[kMaxQueryLevels + 1];     // node side in cells per level
     int nodes_x[kMaxQueryLevels + 1];  // nodes per row per level
     int nP[kMaxQueryLevels + 1], NP[kMaxQueryLevels + 1];
+    int chain;                         // levels without project items (QueryParams::chain)
     int split_items;                   // a level whose template split is > 1 runs split only
                                        // with at most this many project items
 };
@@ -345,7 +355,7 @@ struct PlanLayout {
     int k, kpow;            // kpow = plan_kpow(k): the sort size
     size_t sort_bytes;      // plan_sort_bytes(kpow)
     int* plan;
-    int o_vp0, o_inv, o_l0, o_rec;
+    int o_vp0, o_inv, o_l0, o_rec, o_chain;
     long long flags_off[kMaxQueryLevels + 1];
     unsigned* ticket;
     unsigned ticket_base;

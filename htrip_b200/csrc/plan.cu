@@ -370,7 +370,7 @@ plan_query_kernel(const int32_t* __restrict__ vps, const uint8_t* __restrict__ p
             }
             W.ghead[q] = h;
             const int n_begin = (l == H) ? (W.gquad[q] * nP) / NC * NC : 0;
-            const int items = (cnt + RW - 1) / RW * ((NP - n_begin + NC - 1) / NC);
+            const int items = l <= G.chain ? 0 : (cnt + RW - 1) / RW * ((NP - n_begin + NC - 1) / NC);
             // base items: per RW-row tile jb, the NC-slot tiles from the node's
             // first slot that reach a later row: ceil((rel + jb + nj - 1) / NC)
             int meet = 0;
@@ -407,6 +407,15 @@ plan_query_kernel(const int32_t* __restrict__ vps, const uint8_t* __restrict__ p
                     const int i = W.gstart[q] + idx;
                     s2v[s] = i;
                     W.slot[i] = s;
+                    if (l <= G.chain + 1) {  // (only read when chain > 0)
+                        const int gl = G.side[l] / G.b, gsh = G.g_shift >= 0 ? G.g_shift * l : -1;
+                        const int nx = divp(W.vtx[i], gl, gsh), ny = divp(W.vty[i], gl, gsh);
+                        int* ct = plan + O.o_chain + i * kChainInts + 2 * (l - 1);
+                        ct[0] = s;
+                        ct[1] = 2 * q + ((i > 0 && divp(W.vtx[i - 1], gl, gsh) == nx && divp(W.vty[i - 1], gl, gsh) == ny) ||
+                                         (i + 1 < ns && divp(W.vtx[i + 1], gl, gsh) == nx &&
+                                          divp(W.vty[i + 1], gl, gsh) == ny));
+                    }
                     if (l == 1) {
                         l0[2 * s] = i;
                         l0[2 * s + 1] = q;
@@ -534,7 +543,8 @@ plan_query_kernel(const int32_t* __restrict__ vps, const uint8_t* __restrict__ p
         const int t = lane;
         long u;
         if (t == 0)
-            u = ((long)n_l0 * G.nExt0 + kQueryL0Chunk - 1) / kQueryL0Chunk + (ns + kQueryThreads - 1) / kQueryThreads;
+            u = (G.chain ? (long)ns : ((long)n_l0 * G.nExt0 + kQueryL0Chunk - 1) / kQueryL0Chunk) +
+                (ns + kQueryThreads - 1) / kQueryThreads;
         else if (t <= H + 1)
             u = (t <= H ? items_t : 0) + (t >= 2 ? meet_t : 0);
         else
@@ -549,6 +559,10 @@ plan_query_kernel(const int32_t* __restrict__ vps, const uint8_t* __restrict__ p
         Pq->ldv = ldv;
         Pq->ldm = max(8, (ns + 7) / 8 * 8);
         Pq->n_l0_slots = n_l0;
+        Pq->chain = G.chain;
+        Pq->g = G.g;
+        Pq->leaves_x = G.leaves_x;
+        Pq->chain_tab = plan + O.o_chain;
         Pq->vp0 = plan + O.o_vp0;
         Pq->inv = plan + O.o_inv;
         Pq->l0 = plan + O.o_l0;

@@ -18,7 +18,19 @@
 // (all INF), the unclamped 2-op update (all <= 5535) and the clamped one.
 // Two 256-thread CTAs per SM keep two items in flight.
 //
-//   level 0  X0[p][s] = leaf D[u][port p] for every viewpoint (+ finite-port
+//   chain    levels 0 .. chain of one viewpoint, one CTA: x_0 = its leaf's distances
+//            to the ports, then per level y = x (x) D_U rows of its child over the
+//            node's columns and x = y at the exterior ports, x kept in shared memory.
+//            The lowest levels have few viewpoints per child (mostly one), so
+//            a tile of RW viewpoint rows is mostly padding there, and
+//            handing a level on to the next through L2 (fence, count, poll, flags)
+//            costs 7-10 us.  Measured, query kernel before and after (B200): 256 x 256
+//            street map, b = 16 (three of four levels in the chain), k = 2: 57 -> 41 us,
+//            k = 16: 62 -> 50 us; 512 x 512 maze, k = 256: 168 -> 123 us; 1000 x 1013
+//            street map, k = 509: 797 -> 655 us.  About half of a unit's time goes to
+//            fetching its instructions (each CTA runs most of them once): loops here
+//            stay rolled, and a deeper copy ring measured slower.
+//   level 0  (no chain) X0[p][s] = leaf D[u][port p] for every viewpoint (+ finite-port
 //            flags of its level-1 child group) and same-leaf pairs
 //            (minplus_oracle.cpp:990-1048).
 //   project Yt_l[c][s] = min_p X_{l-1}[p][s] (+) D_U[q*nP + p][c] over the ports
@@ -145,7 +157,7 @@ __device__ __forceinline__ int warp_minplus_list(uint32_t (&acc)[RW][CP], const 
         cp_wait<NS - 1>();
         __syncwarp();
         const int st = it % NS;
-#pragma unroll
+#pragma unroll 1
         for (int u = 0; u < U; ++u) {
             if (first + it * stride + u < n) {
                 const uint32_t* slot = pipe + (st * U + u) * SW;
@@ -216,10 +228,14 @@ __device__ __forceinline__ void count_work(unsigned long long* work, int n, int 
 __device__ __forceinline__ int compact_flags(const uint8_t* __restrict__ flags, int kb, int ke, int* kl, int* wsum) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = ke - kb;
-    const int per = (n + kThreads - 1) / kThreads;
+    const int per = (n + kThreads - 1) / kThreads;  // <= 16: kMaxList flags
     const int p0 = kb + tid * per, p1 = min(ke, p0 + per);
-    int cntl = 0;
-    for (int p = p0; p < p1; ++p) cntl += __ldcg(flags + p) != 0;
+    // the thread's flags are read once, all loads in flight together
+    uint32_t mask = 0;
+#pragma unroll 4
+    for (int j = 0; j < per; ++j)
+        if (p0 + j < p1) mask |= (uint32_t)(__ldcg(flags + p0 + j) != 0) << j;
+    const int cntl = __popc(mask);
     int incl = cntl;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -235,8 +251,7 @@ __device__ __forceinline__ int compact_flags(const uint8_t* __restrict__ flags, 
         total += wsum[w];
     }
     int pos = base + incl - cntl;
-    for (int p = p0; p < p1; ++p)
-        if (__ldcg(flags + p)) kl[pos++] = p;
+    for (; mask; mask &= mask - 1) kl[pos++] = p0 + __ffs(mask) - 1;
     __syncthreads();
     return total;
 }
@@ -322,12 +337,13 @@ __device__ __forceinline__ unsigned long long global_timer() {
 // Shared memory of the persistent kernel: compacted row list (nP <= 4096
 // ports), scan partials and the split-K reduction buffer.
 constexpr int kMaxList = 4096 + 64;
+constexpr size_t kChainSmemBytes = 16 * 1024;  // ChainSmem
 // The staging rings (during an item's k-loop) and the split-K reduction
 // buffer (after it) share one region.
 template <int RW, int CP>
 constexpr size_t query_smem_bytes() {
     return (size_t)kMaxList * sizeof(int) +
-           std::max((size_t)kWarps * RW * CP * 32, (size_t)kWarps * pipe_warp_words<RW, CP>()) * sizeof(uint32_t);
+           std::max<size_t>(kChainSmemBytes, std::max((size_t)kWarps * RW * CP * 32, (size_t)kWarps * pipe_warp_words<RW, CP>()) * sizeof(uint32_t));
 }
 
 // Per-item metadata staged in shared memory at the start of an item (its
@@ -382,6 +398,187 @@ __device__ bool combine_parts(const QueryLevel& L, int item, int part, uint32_t 
 __device__ __forceinline__ bool dirty_at(const uint8_t* dirty, int j, int l) {
     const int d = dirty[j];
     return d != 0 && d - 1 <= l;
+}
+
+// Chain unit of viewpoint v (see the file's head).  Its X and Y columns and the
+// finite-port flags are written where another unit reads them: those of levels whose
+// node holds another viewpoint (their meets), and X of level `chain` (the
+// project items above).  `tab` receives the viewpoint's table row for the signal.
+// A level is a chain of round trips: so everything that does not depend on the
+// level below (tables, pointers, the rows' way through the TLB) is fetched
+// for all levels at the start.
+struct ChainLevel {
+    const uint16_t* D;   // rows of the viewpoint's child
+    uint16_t *X, *Y;     // the level's columns in the viewpoint's slots
+    uint8_t* flags;      // finite-port flags of the viewpoint's group of this level
+    int NP, nP;
+};
+struct ChainSmem {
+    int16_t ext[2 * kMaxChainNP];       // per level, column -> exterior port or -1 (NP entries each)
+    int2 list[256];                     // finite ports of the child: {row offset, value in both halves}
+    uint16_t x[kMaxChainNP];            // port distances of the level below
+    uint16_t red[8 * kThreads];         // partial rows of the row groups
+    uint8_t chunk[kMaxChainNP / 8];     // the 8-column chunks of the level to compute
+    ChainLevel lv[kMaxChain + 1];
+    int wcnt[kWarps], ccnt[kWarps];
+};
+static_assert(sizeof(ChainSmem) <= kChainSmemBytes, "shared memory of a chain unit");
+
+__device__ __forceinline__ void do_chain(const QueryParams& P, int v, ChainSmem& S, int* tab) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ldv = P.ldv, H = P.H, top = P.chain;
+    const int4 vp = *reinterpret_cast<const int4*>(P.vp0 + 4 * v);  // {leaf, cell, ..}
+    if (tid < kChainInts) tab[tid] = P.chain_tab[v * kChainInts + tid];
+    bool skip = false;
+    if (P.dirty) {
+        const int d = P.dirty[v];
+        skip = d == 0 || d - 1 > top;  // nothing changed at levels <= chain
+    }
+    if (skip) {
+        __syncthreads();
+        return;
+    }
+    {   // exterior tables of all levels, 8 columns per thread and step
+        int o = 0;
+#pragma unroll 1
+        for (int l = 1; l <= top; ++l) {
+            const int n = P.lv[l].NP / 8, c = (tid + kThreads - (o / 8) % kThreads) % kThreads;
+            if (c < n) {
+                const int4 a = reinterpret_cast<const int4*>(P.lv[l].ext_inv)[2 * c];
+                const int4 b = reinterpret_cast<const int4*>(P.lv[l].ext_inv)[2 * c + 1];
+                *reinterpret_cast<uint4*>(S.ext + o + 8 * c) =
+                    make_uint4((a.x & 0xffff) | (a.y << 16), (a.z & 0xffff) | (a.w << 16), (b.x & 0xffff) | (b.y << 16),
+                               (b.z & 0xffff) | (b.w << 16));
+            }
+            o += 8 * n;
+        }
+    }
+    {
+        const uint16_t* row = P.leaves.base + ((size_t)vp.x * P.leaves.NP + vp.y) * P.leaves.NP;
+        for (int p = tid; p < P.nExt0; p += kThreads) S.x[p] = row[P.ext0[p]];
+    }
+    __syncthreads();  // tab
+    if (warp == kWarps - 1 && lane <= top) {  // level l's pieces, one lane each (lane top: the level above)
+        const int l = lane + 1;
+        ChainLevel c{};
+        c.X = lane < H ? P.X[lane] + (l <= H ? tab[2 * lane] : 0) : nullptr;  // X_{l-1}, in level-l slots
+        if (l <= H) {
+            const QueryLevel& L = P.lv[l];
+            const int* grp = L.groups + 5 * (tab[2 * lane + 1] >> 1);
+            const int node = grp[0], q = grp[1];
+            c.D = L.D + ((size_t)node * L.NP + (size_t)q * L.nP) * L.NP;
+            c.Y = P.Y[l] + tab[2 * lane];
+            c.flags = L.flags + (size_t)(tab[2 * lane + 1] >> 1) * L.nP;
+            c.NP = L.NP;
+            c.nP = L.nP;
+            if (l <= top) asm volatile("prefetch.global.L2 [%0];" ::"l"(c.D));  // its page's translation
+        }
+        S.lv[lane] = c;
+    }
+    __syncthreads();
+    if (tab[1] & 1) {  // the level-1 meets read X_0
+        const ChainLevel& L = S.lv[0];
+        for (int p = tid; p < P.nExt0; p += kThreads) {
+            const uint16_t d = S.x[p];
+            L.X[(size_t)p * ldv] = d;
+            if (d < INF) L.flags[p] = 1;
+        }
+    }
+    unsigned long long entries = 0, rows = 0;
+    const int16_t* ext = S.ext;
+#pragma unroll 1
+    for (int l = 1; l <= top; ++l) {
+        const ChainLevel L = S.lv[l - 1];
+        const int NP = L.NP;
+        const bool put_y = tab[2 * (l - 1) + 1] & 1;  // the level's meets read Y
+        // The finite ports (nP <= 256: one step) and the columns to compute, in
+        // chunks of 8: all where the level's meets read Y, else those with an exterior
+        // port (about half).
+        const uint32_t a0 = tid < L.nP ? S.x[tid] : INF;
+        bool need = tid < NP / 8;
+        if (need && !put_y) {
+            const uint4 e = *reinterpret_cast<const uint4*>(ext + 8 * tid);
+            need = (e.x & e.y & e.z & e.w) != 0xffffffffu;
+        }
+        const unsigned bal = __ballot_sync(FULL, a0 < INF), cbal = __ballot_sync(FULL, need);
+        if (lane == 0) {
+            S.wcnt[warp] = __popc(bal);
+            S.ccnt[warp] = __popc(cbal);
+        }
+        __syncthreads();
+        int at = __popc(bal & ((1u << lane) - 1u)), n = 0, cat = __popc(cbal & ((1u << lane) - 1u)), G = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            if (w < warp) {
+                at += S.wcnt[w];
+                cat += S.ccnt[w];
+            }
+            n += S.wcnt[w];
+            G += S.ccnt[w];
+        }
+        if (a0 < INF) S.list[at] = make_int2(tid * NP, (int)splat(a0));
+        if (need) S.chunk[cat] = (uint8_t)tid;
+        __syncthreads();
+        // A thread takes one chunk of every nG-th listed row, 8 loads in flight.
+        const int rg = tid / G, nG = kThreads / G, cg = S.chunk[tid - rg * G];
+        rows += n;
+        entries += (unsigned long long)n * (8 * G);
+        uint32_t acc[4] = {INF2, INF2, INF2, INF2};
+        if (rg < nG && rg < n) {
+            const uint16_t* D = L.D + 8 * cg;
+            constexpr int U = 8;
+#pragma unroll 1
+            for (int i = rg; i < n; i += U * nG) {
+                uint4 b[U];
+                uint32_t a[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int2 e = S.list[min(i + u * nG, n - 1)];  // past the end: the last row again
+                    a[u] = (uint32_t)e.y;
+                    b[u] = __ldg(reinterpret_cast<const uint4*>(D + e.x));
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t tt = INF2 - a[u];
+                    acc[0] = acc_clamp(acc[0], b[u].x, a[u], tt);
+                    acc[1] = acc_clamp(acc[1], b[u].y, a[u], tt);
+                    acc[2] = acc_clamp(acc[2], b[u].z, a[u], tt);
+                    acc[3] = acc_clamp(acc[3], b[u].w, a[u], tt);
+                }
+            }
+        }
+        if (rg < nG) *reinterpret_cast<uint4*>(&S.red[8 * tid]) = make_uint4(acc[0], acc[1], acc[2], acc[3]);
+        __syncthreads();
+        const bool put_x = l < H && (l == top || (tab[2 * l + 1] & 1));
+        uint16_t* X = S.lv[l].X;
+        uint8_t* fl = S.lv[l].flags;
+#pragma unroll 1
+        for (int pw = tid; pw < 4 * G; pw += kThreads) {  // red: [row group][chunk place][8 columns]
+            const int c = 8 * S.chunk[pw >> 2] + 2 * (pw & 3);
+            const uint32_t e2 = *reinterpret_cast<const uint32_t*>(ext + c);
+            uint32_t m = INF2;
+#pragma unroll 1
+            for (int r = 0; r < nG; ++r) m = min2(m, *reinterpret_cast<const uint32_t*>(&S.red[8 * r * G + 2 * pw]));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint16_t y = (uint16_t)(m >> (16 * h));
+                const int e = (int16_t)(e2 >> (16 * h));
+                if (put_y) L.Y[(size_t)(c + h) * ldv] = y;
+                if (l < H && e >= 0) {
+                    S.x[e] = y;
+                    if (put_x) {
+                        X[(size_t)e * ldv] = y;
+                        if (y < INF) fl[e] = 1;
+                    }
+                }
+            }
+        }
+        ext += NP;
+        __syncthreads();
+    }
+    if (P.work && tid == 0) {
+        atomicAdd(P.work, entries);
+        atomicAdd(P.work + 1, rows);
+    }
 }
 
 template <int RW, int CP>
@@ -544,13 +741,18 @@ __device__ void unit_prologue(const QueryParams& P, int t, int u, ItemMeta& im) 
 // metadata is staged (unit_prologue).  Returns
 // false for a part of a split project item that did not complete it.
 template <int RW, int CP>
-__device__ bool run_unit(const QueryParams& P, int t, int u, int* kl, int* wsum, uint32_t* red, ItemMeta& im) {
+__device__ bool run_unit(const QueryParams& P, int t, int u, int* kl, int* wsum, uint32_t* red, ItemMeta& im,
+                         int* chain_row) {
     const int tid = threadIdx.x;
+    if (t == 0 && u < P.ns && P.chain > 0) {
+        do_chain(P, u, *reinterpret_cast<ChainSmem*>(red), chain_row);
+        return true;
+    }
     if (t == 0) {
         // level 0: X0 in level-1 slot order (+ level-1 flags), same-leaf pairs
         const int S1 = P.n_l0_slots;
         const int total = S1 * P.nExt0;
-        const int n_fill = (total + kQueryL0Chunk - 1) / kQueryL0Chunk;
+        const int n_fill = P.chain > 0 ? P.ns : (total + kQueryL0Chunk - 1) / kQueryL0Chunk;
         if (u < n_fill) {
             const int e1 = min(total, (u + 1) * kQueryL0Chunk);
             for (int e = u * kQueryL0Chunk + tid; e < e1; e += kThreads) {
@@ -604,6 +806,9 @@ __device__ bool run_unit(const QueryParams& P, int t, int u, int* kl, int* wsum,
 // Dataflow order.  Instead of a grid barrier after every phase, each unit
 // waits for the units it reads and counts itself done on the request's
 // completion counters (QueryParams::ctr):
+//   project, level chain + 1  the chain units of its group's viewpoints: ctr[4 + l*k + g]
+//     (chain > 0, group g)      reaches cnt_g (a chain unit adds 1 for each level
+//                               l = 2 .. chain + 1)
 //   project, level 1          all level-0 gather units (ctr[0])
 //   project, level l >= 2     the level-(l-1) project items of its group's
 //     (group g)               node: ctr[4 + l*k + g] reaches cnt_g x column
@@ -611,7 +816,8 @@ __device__ bool run_unit(const QueryParams& P, int t, int u, int* kl, int* wsum,
 //                             lifts into group g; each item adds its rows)
 //   meet, level l < H         the level-l project items of its node, i.e.
 //                             the counter of the level-(l+1) group it lifts to
-//   meet, level H             every root project item (ctr[2])
+//   (levels <= chain count viewpoints, as above)
+//   meet, level H             every root project item (ctr[2]; chain = H: every viewpoint)
 //   output                    every project, meet and pair unit (ctr[1])
 // A project item cut into parts (QueryLevel::split) counts toward its
 // consumers once, when the part that completes it has run the epilogue.
@@ -629,6 +835,20 @@ constexpr unsigned kWaitPolls = 1u << 24;
 // so that it runs beside thread 0's fence and counts for the previous unit.
 constexpr int kWaiter = 32;
 
+// Hand-over of a unit's results: the CTA barrier before the counts orders every
+// thread's stores before them, and one acquire-release fence (before all of a
+// unit's counts: a release per count costs a fence each, about 1 us) with
+// the waiter's acquire makes them visible to the CTA behind the waiter's barrier.
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;\n" ::: "memory"); }
+__device__ __forceinline__ void add_count(unsigned* p, unsigned v) {
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
+}
+
 // Bounded wait of the whole CTA until *c >= target: thread kWaiter polls,
 // the CTA follows.  False after a timeout (recorded in *status) or when
 // another CTA has recorded one.
@@ -636,10 +856,9 @@ __device__ __forceinline__ bool wait_count(const unsigned* c, unsigned target, i
                                            unsigned limit = kWaitPolls) {
     int ok = 1;
     if (threadIdx.x == kWaiter) {
-        const volatile unsigned* vc = c;
         const volatile int* vs = status;
         unsigned it = 0;
-        while (*vc < target) {
+        while (ld_acquire(c) < target) {
             if (*vs != 0) {
                 ok = 0;
                 break;
@@ -651,7 +870,6 @@ __device__ __forceinline__ bool wait_count(const unsigned* c, unsigned target, i
             }
             __nanosleep(32);
         }
-        __threadfence();
     }
     return __syncthreads_and(ok) != 0;
 }
@@ -685,7 +903,11 @@ __device__ __forceinline__ bool dep_wait(const QueryParams& P, int t, int u, int
         } else {
             const int np = t <= H ? P.lv[t].n_items * P.lv[t].split : 0;
             if (u < np) {  // project item (part) of level t
-                if (t == 1) {
+                if (t == P.chain + 1 && t > 1) {
+                    const int gi = P.lv[t].items[3 * (u / P.lv[t].split)];
+                    target = (unsigned)P.lv[t].groups[5 * gi + 3];
+                    c = P.ctr + 4 + (size_t)t * P.k + gi;
+                } else if (t == 1) {
                     const long total = (long)P.n_l0_slots * P.nExt0;
                     target = (unsigned)((total + kQueryL0Chunk - 1) / kQueryL0Chunk);
                     c = P.ctr;
@@ -697,12 +919,12 @@ __device__ __forceinline__ bool dep_wait(const QueryParams& P, int t, int u, int
             } else {  // meet item of level t - 1
                 const int l = t - 1;
                 if (l == H) {
-                    target = (unsigned)P.lv[H].n_items;
+                    target = (unsigned)(P.chain == H ? P.ns : P.lv[H].n_items);
                     c = P.ctr + 2;
                 } else {
                     const int j0 = P.lv[l].meet[7 * (u - np) + 1];
                     const int pg = P.lv[l].lift[2 * j0 + 1];
-                    target = (unsigned)P.lv[l + 1].groups[5 * pg + 3] * col_tiles(P.lv[l].NP, NC);
+                    target = (unsigned)P.lv[l + 1].groups[5 * pg + 3] * (l <= P.chain ? 1u : col_tiles(P.lv[l].NP, NC));
                     c = P.ctr + 4 + (size_t)(l + 1) * P.k + pg;
                 }
             }
@@ -716,32 +938,38 @@ __device__ __forceinline__ bool dep_wait(const QueryParams& P, int t, int u, int
 // CTA has issued its stores (the fence orders them before the counts); a
 // project item counts toward its consumers once complete (all its parts).
 template <int RW, int CP>
-__device__ __forceinline__ void dep_signal(const QueryParams& P, int t, int u, bool complete) {
+__device__ __forceinline__ void dep_signal(const QueryParams& P, int t, int u, bool complete, const int* tab) {
     __syncthreads();
     if (threadIdx.x != 0) return;
     const int H = P.H;
     if (t == H + 2) return;
-    __threadfence();
+    fence_gpu();
     if (t == 0) {
+        if (P.chain > 0 && u < P.ns) {  // tab: the chain unit's table row
+            for (int l = 2; l <= min(P.chain + 1, H); ++l)
+                add_count(P.ctr + 4 + (size_t)l * P.k + (tab[2 * (l - 1) + 1] >> 1), 1u);
+            if (P.chain == H) add_count(P.ctr + 2, 1u);
+            return;
+        }
         const long total = (long)P.n_l0_slots * P.nExt0;
-        const int n_fill = (int)((total + kQueryL0Chunk - 1) / kQueryL0Chunk);
-        atomicAdd(P.ctr + (u < n_fill ? 0 : 1), 1u);
+        const int n_fill = P.chain > 0 ? P.ns : (int)((total + kQueryL0Chunk - 1) / kQueryL0Chunk);
+        add_count(P.ctr + (u < n_fill ? 0 : 1), 1u);
         return;
     }
     const int S = t <= H ? P.lv[t].split : 1;
     const int np = t <= H ? P.lv[t].n_items * S : 0;
     if (u < np && complete) {
         if (t == H) {
-            atomicAdd(P.ctr + 2, 1u);
+            add_count(P.ctr + 2, 1u);
         } else {
             const int* it = P.lv[t].items + 3 * (u / S);
             const int* G = P.lv[t].groups + 5 * it[0];
             const int rows = min(RW, G[3] - it[1]);
             const int pg = P.lv[t].lift[2 * G[2] + 1];
-            atomicAdd(P.ctr + 4 + (size_t)(t + 1) * P.k + pg, (unsigned)rows);
+            add_count(P.ctr + 4 + (size_t)(t + 1) * P.k + pg, (unsigned)rows);
         }
     }
-    atomicAdd(P.ctr + 1, 1u);
+    add_count(P.ctr + 1, 1u);
 }
 
 // The persistent kernel.  Barrier mode: phases separated by grid barriers;
@@ -754,6 +982,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads) q_persistent_kernel(
     uint32_t* red = reinterpret_cast<uint32_t*>(qsm + kMaxList);
     __shared__ int wsum[kWarps];
     __shared__ ItemMeta im;
+    __shared__ int chain_row[kChainInts];
     const bool stamp = B.trace && blockIdx.x == 0 && threadIdx.x == 0;
     if (stamp) B.trace[0] = global_timer();
     if (B.dataflow) {
@@ -761,16 +990,19 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads) q_persistent_kernel(
         // count word, unused here); a CTA takes its next ticket when it starts
         // a unit, so the fetch overlaps the work.
         __shared__ int next_w;
-        int total = 0;
-        for (int t = 0; t < B.n_phases; ++t) total += B.unit_pre[(size_t)t * (B.n_req + 1) + B.n_req];
+        __shared__ int phase_units[kMaxQueryPhases];
         if (threadIdx.x == 0) next_w = (int)atomicAdd(B.bar, 1u);
+        if (threadIdx.x >= 32 && threadIdx.x - 32 < B.n_phases)
+            phase_units[threadIdx.x - 32] = B.unit_pre[(size_t)(threadIdx.x - 32) * (B.n_req + 1) + B.n_req];
         __syncthreads();
+        int total = 0;
+        for (int t = 0; t < B.n_phases; ++t) total += phase_units[t];
         for (;;) {
             const int w = next_w;
             if (w >= total) break;
             int t = 0, wl = w;
             for (;;) {
-                const int nt = B.unit_pre[(size_t)t * (B.n_req + 1) + B.n_req];
+                const int nt = phase_units[t];
                 if (wl < nt) break;
                 wl -= nt;
                 ++t;
@@ -788,9 +1020,9 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads) q_persistent_kernel(
             if (!dep_wait<RW, CP>(P, t, u, B.status)) return;
             // every thread has read next_w (the wait is a CTA barrier)
             const int nxt = threadIdx.x == 0 ? (int)atomicAdd(B.bar, 1u) : 0;
-            const bool complete = run_unit<RW, CP>(P, t, u, kl, wsum, red, im);
+            const bool complete = run_unit<RW, CP>(P, t, u, kl, wsum, red, im, chain_row);
             if (threadIdx.x == 0) next_w = nxt;
-            dep_signal<RW, CP>(P, t, u, complete);  // begins with a CTA barrier: next_w is visible after it
+            dep_signal<RW, CP>(P, t, u, complete, chain_row);  // begins with a CTA barrier: next_w is visible after it
             if (B.trace && threadIdx.x == 0) {
                 const unsigned long long now = global_timer();
                 atomicMax(B.trace + t + 1, now);
@@ -811,7 +1043,7 @@ __global__ void __launch_bounds__(kThreads, 512 / kThreads) q_persistent_kernel(
             }
             unit_prologue<RW, CP>(B.req[lo], t, w - pre[lo], im);
             __syncthreads();
-            run_unit<RW, CP>(B.req[lo], t, w - pre[lo], kl, wsum, red, im);
+            run_unit<RW, CP>(B.req[lo], t, w - pre[lo], kl, wsum, red, im, chain_row);
         }
         if (B.trace && threadIdx.x == 0)  // the phase's last CTA to finish its units
             atomicMax(B.trace + kMaxQueryPhases + 1 + t, global_timer());
