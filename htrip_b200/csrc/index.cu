@@ -1806,11 +1806,14 @@ void make_plan(const htrip_index* h, const int32_t* vps, const uint8_t* pass_fla
 // Query launches.  One cooperative launch of the persistent kernel serves
 // any number of planned requests of one device (indexes of any shape, any
 // k).  Device scratch of a launch, every piece 256-byte aligned:
-//   [QueryParams x n][unit prefix, n_phases x (n+1) ints][4 words][plans]
+//   [QueryParams x n][unit prefix, n_phases x (n+1) ints][plans][launch words]
 //       <- one host->device copy of the staged head (words start at zero)
-//   [M of every request]      <- one memset to 0xFF (no pair found yet)
-//   [flags + completion counters of every request]  <- one memset to 0
-//   [X_0..X_{H-1} Y_1..Y_H of every request][results k*k u16 of every request]
+//   [results k*k u16 of every request]   -> one device->host copy with the words
+//   [M of every request]      <- preset to 0xFF (no pair found yet)
+//   [flags + completion counters of every request]  <- preset to 0
+//   [X_0..X_{H-1} Y_1..Y_H of every request]
+// Small launches (kPresetCopy) stage the presets behind the head: one copy instead of a
+// copy and two memsets.
 // ---------------------------------------------------------------------------
 
 struct QueryReq {
@@ -1826,9 +1829,13 @@ constexpr size_t kWorkOffset = 16;
 constexpr size_t kTraceOffset = 64;
 constexpr size_t kWordsBytes = kTraceOffset + (2 * hb::kMaxQueryPhases + 1) * sizeof(unsigned long long);
 
+// Up to this many bytes of results, pair matrices and flags are preset by the copy of
+// the staged head; a memset costs about 2 us of a call, as much as copying this.
+constexpr size_t kPresetCopy = 32 * 1024;
+
 struct LaunchLayout {
     int n = 0, n_phases = 0;
-    size_t o_params = 0, o_pre = 0, o_words = 0, head = 0;
+    size_t o_params = 0, o_pre = 0, o_words = 0, head = 0, staged = 0;
     size_t o_M = 0, M_bytes = 0, o_flags = 0, flags_bytes = 0, o_out = 0, out_bytes = 0, total = 0;
     std::vector<size_t> plan, M, flags, ctr, ticket, part, out;
     std::vector<std::array<size_t, hb::kMaxQueryLevels + 1>> X, Y;
@@ -1871,9 +1878,12 @@ LaunchLayout layout_launch(const std::vector<QueryReq>& R) {
     };
     L.o_params = take(R.size() * sizeof(hb::QueryParams));
     L.o_pre = take((size_t)L.n_phases * (R.size() + 1) * sizeof(int));
-    L.o_words = take(kWordsBytes);
     for (const auto& r : R) L.plan.push_back(take(r.P->buf.size() * sizeof(int)));
+    L.o_words = take(kWordsBytes);
     L.head = off;
+    L.o_out = off;
+    for (const auto& r : R) L.out.push_back(r.out_dev ? 0 : take((size_t)r.P->k * r.P->k * sizeof(uint16_t)));
+    L.out_bytes = off - L.o_out;
     L.o_M = off;
     for (const auto& r : R) L.M.push_back(take((size_t)r.P->ldm * r.P->ldm * sizeof(uint32_t)));
     L.M_bytes = off - L.o_M;
@@ -1885,6 +1895,7 @@ LaunchLayout layout_launch(const std::vector<QueryReq>& R) {
         L.ticket.push_back(root.split > 1 ? take((size_t)root.n_items * sizeof(unsigned)) : 0);
     }
     L.flags_bytes = off - L.o_flags;
+    L.staged = off - L.head <= kPresetCopy ? off : L.head;
     for (const auto& r : R) {
         const QueryPlan::Lvl& root = r.P->lv[r.h->H];
         const hb::QueryTile tile = hb::query_config_tile(r.P->cfg);
@@ -1897,9 +1908,6 @@ LaunchLayout layout_launch(const std::vector<QueryReq>& R) {
         L.X.push_back(x);
         L.Y.push_back(y);
     }
-    L.o_out = off;
-    for (const auto& r : R) L.out.push_back(r.out_dev ? 0 : take((size_t)r.P->k * r.P->k * sizeof(uint16_t)));
-    L.out_bytes = off - L.o_out;
     L.total = off;
     return L;
 }
@@ -1975,9 +1983,8 @@ hb::QueryParams make_params(const htrip_index* h, const QueryPlan& P, unsigned c
     return Q;
 }
 
-// Stages the head of the launch into `stage` (>= L.head bytes of host
-// memory), then issues on `st`: the head copy, the two presets and the
-// kernel, bracketed by ev[0] / ev[1] when given.  Returns the device
+// Stages the head of the launch into `stage` (>= L.staged bytes of host
+// memory), then issues on `st`: the head copy, the presets and the kernel, bracketed by ev[0] / ev[1] when given.  Returns the device
 // pointers of the results in `outs`.
 // With `dirty` (one request; an incremental refresh in an arena that holds
 // the previous launch of the same plan) the pair matrix and the finite-port
@@ -1987,7 +1994,10 @@ void issue_query_launch(cudaStream_t st, int device, int& grid, int cfg, const s
                         const LaunchLayout& L, unsigned char* base, unsigned char* stage, const cudaEvent_t* ev,
                         std::vector<uint16_t*>& outs, const uint8_t* dirty = nullptr) {
     for (const auto& r : R) check_query_shape(r.h);
-    std::memset(stage, 0, L.head);
+    const bool preset = L.staged > L.head && !dirty;  // the presets travel with the head
+    const size_t bytes = preset ? L.staged : L.head;
+    std::memset(stage, 0, bytes);
+    if (preset) std::memset(stage + L.o_M, 0xFF, L.M_bytes);
     outs.resize(R.size());
     auto* params = reinterpret_cast<hb::QueryParams*>(stage + L.o_params);
     auto* pre = reinterpret_cast<int*>(stage + L.o_pre);
@@ -2002,11 +2012,11 @@ void issue_query_launch(cudaStream_t st, int device, int& grid, int cfg, const s
         for (int t = 0; t < L.n_phases; ++t)
             pre[(size_t)t * (L.n + 1) + i + 1] = pre[(size_t)t * (L.n + 1) + i] + units[t];
     }
-    ck(cudaMemcpyAsync(base, stage, L.head, cudaMemcpyHostToDevice, st), "query launch head");
-    if (!dirty) {
+    ck(cudaMemcpyAsync(base, stage, bytes, cudaMemcpyHostToDevice, st), "query launch head");
+    if (!preset && !dirty) {
         ck(cudaMemsetAsync(base + L.o_M, 0xFF, L.M_bytes, st), "pair matrix preset");
         ck(cudaMemsetAsync(base + L.o_flags, 0, L.flags_bytes, st), "flag preset");
-    } else {  // only the completion counters and the split items' tickets start at zero
+    } else if (dirty) {  // only the completion counters and the split items' tickets start at zero
         for (size_t i = 0; i < R.size(); ++i) {
             ck(cudaMemsetAsync(base + L.ctr[i], 0,
                                hb::query_counter_words(R[i].h->H, R[i].P->k) * sizeof(unsigned), st), "counters");
@@ -2048,8 +2058,9 @@ int run_queries(QueryArena& A, int device, cudaStream_t st, const std::vector<Qu
     // arena or the pinned staging: wait for it before reusing or growing them.
     if (A.ev_valid) ck(cudaEventSynchronize(A.ev[1]), "previous launch");
     A.dev.reserve(L.total, st);
-    A.stage.reserve(L.head);
-    A.outstage.reserve(L.out_bytes + 256);
+    A.stage.reserve(L.staged);
+    const size_t back = L.o_out - L.o_words + L.out_bytes;  // launch words and results
+    A.outstage.reserve(back);
     if (!A.ev[0]) {
         ck(cudaEventCreate(&A.ev[0]), "event");
         ck(cudaEventCreate(&A.ev[1]), "event");
@@ -2059,25 +2070,23 @@ int run_queries(QueryArena& A, int device, cudaStream_t st, const std::vector<Qu
     A.ev_valid = true;
     A.last_words = L.o_words;
     A.last_phases = L.n_phases;
-    A.last_h2d = L.head;
+    A.last_h2d = dirty ? L.head : L.staged;
     A.last_d2h = 0;
-    int* status_host = reinterpret_cast<int*>(A.outstage.p + L.out_bytes);
     bool any_host = false;
     for (size_t i = 0; i < R.size(); ++i) any_host |= !R[i].out_dev && host_out[i];
-    if (any_host) {
-        ck(cudaMemcpyAsync(A.outstage.p, A.dev.p + L.o_out, L.out_bytes, cudaMemcpyDeviceToHost, st), "results");
-        A.last_d2h += L.out_bytes;
+    if (sync || any_host) {  // the status word leads the launch words
+        const size_t n = any_host ? back : sizeof(int);
+        ck(cudaMemcpyAsync(A.outstage.p, A.dev.p + L.o_words, n, cudaMemcpyDeviceToHost, st), "results");
+        A.last_d2h = n;
     }
     if (!sync) return 0;
-    ck(cudaMemcpyAsync(status_host, A.dev.p + L.o_words, sizeof(int), cudaMemcpyDeviceToHost, st), "status");
-    A.last_d2h += sizeof(int);
     ck(cudaStreamSynchronize(st), "query sync");
     if (any_host)
         for (size_t i = 0; i < R.size(); ++i)
             if (!R[i].out_dev && host_out[i])
-                std::memcpy(host_out[i], A.outstage.p + (L.out[i] - L.o_out),
+                std::memcpy(host_out[i], A.outstage.p + (L.out[i] - L.o_words),
                             (size_t)R[i].P->k * R[i].P->k * sizeof(uint16_t));
-    return *status_host;
+    return *reinterpret_cast<const int*>(A.outstage.p);
 }
 
 // Same-cfg planning for a launch: every request of one launch uses the
@@ -2146,9 +2155,9 @@ int choose_query_cfg(const htrip_index* h, int ns, int root_group) {
 // waits for the GPU before the launch: a query with device-resident inputs
 // is two launches (planner, query kernel) and no copy.  Arena layout, every
 // piece 256-byte aligned:
-//   [QueryParams][unit prefix][launch words][viewpoints 8k + flags k]
-//   [plan ints][M][flags + completion counters][X_0..X_{H-1} Y_1..Y_H]
-//   [result k*k u16, host-bound calls]
+//   [QueryParams][unit prefix][launch words][result k*k u16, host-bound calls]
+//   [viewpoints 8k + flags k][plan ints][M][flags + completion counters]
+//   [X_0..X_{H-1} Y_1..Y_H]
 // The plan capacities are worst cases for k viewpoints, so the planner's
 // overflow status (2) is a guard, not a path: a synchronous call that sees
 // it replans on the host.
@@ -2167,10 +2176,14 @@ struct DevPlanLayout {
 // shared-memory sort, Morton codes below 2^52 (they carry the viewpoint index
 // in the low 12 bits), and the query kernel's depth and port limits.  It
 // does, by default, when the viewpoints are already on the device (the host
-// would otherwise wait for their copy); with host viewpoints the host plans
-// (its plan goes out with the viewpoints' copy anyway, and measured faster).
+// would otherwise wait for their copy), and from kDevPlanHostK viewpoints on when
+// they come from the host: the host's planning grows with k, the device's costs
+// about 20 us whatever k is.  Whole calls, host / device planned: 256 x 256 street map
+// k = 48 104 / 114 us, 64 109 / 110, 128 137 / 129, 512 267 / 220; 512 x 512 maze
+// k = 48 128 / 131, 64 142 / 139, 128 175 / 156, 512 423 / 316.
 // HTRIP_QUERY_PLANNER=host plans every query on the host, =device every
 // query it can on the device.
+constexpr int kDevPlanHostK = 64;
 bool devplan_supported(const htrip_index* h, int k, bool host_inputs) {
     if (k < 1 || k > hb::plan_max_k() || h->H > hb::kMaxQueryLevels) return false;
     static const int mode = [] {
@@ -2179,7 +2192,7 @@ bool devplan_supported(const htrip_index* h, int k, bool host_inputs) {
         if (e && std::strcmp(e, "device") == 0) return 2;
         return 0;
     }();
-    if (mode == 1 || (mode == 0 && host_inputs)) return false;
+    if (mode == 1 || (mode == 0 && host_inputs && k < kDevPlanHostK)) return false;
     double codes = 1;
     for (int l = 0; l < std::max(h->H, 1); ++l) codes *= (double)h->g * h->g;
     if (codes >= 4503599627370496.0) return false;  // 2^52
@@ -2271,6 +2284,7 @@ DevPlanLayout devplan_layout(const htrip_index* h, int k, int cfg, bool out_in_a
     D.o_params = takeb(sizeof(hb::QueryParams));
     D.o_pre = takeb((size_t)D.n_phases * 2 * sizeof(int));
     D.o_words = takeb(kWordsBytes);
+    D.o_out = out_in_arena ? takeb((size_t)k * k * sizeof(uint16_t)) : 0;  // behind the words: one copy back
     D.o_in = takeb(9 * (size_t)k);
     D.o_plan = takeb(n * sizeof(int));
     const size_t ldm = std::max<size_t>(8, ((size_t)k + 7) / 8 * 8);
@@ -2290,7 +2304,6 @@ DevPlanLayout devplan_layout(const htrip_index* h, int k, int cfg, bool out_in_a
     D.o_part = D.root_split > 1 ? takeb(root_items * D.root_split * RW * NC * 2) : 0;
     for (int l = 0; l < H; ++l) D.X[l] = takeb(query_x_rows(h, l) * O.cap_ldv * sizeof(uint16_t));
     for (int l = 1; l <= H; ++l) D.Y[l] = takeb(query_y_rows(h, l) * O.cap_ldv * sizeof(uint16_t));
-    D.o_out = out_in_arena ? takeb((size_t)k * k * sizeof(uint16_t)) : 0;
     D.total = off;
     O.words_bytes = (int)kWordsBytes;
     // preset blocks: about 64 KB each, no more than fit beside the planner
@@ -2446,14 +2459,14 @@ int run_devplan(htrip_index* h, int k, int cfg, const int32_t* vps_host, const u
     A.last_d2h = 0;
     if (!to_host) return 0;
     const size_t ob = (size_t)k * k * sizeof(uint16_t);
-    A.outstage.reserve(align256(ob) + 256);
-    int* status_host = reinterpret_cast<int*>(A.outstage.p + align256(ob));
-    ck(cudaMemcpyAsync(A.outstage.p, out, ob, cudaMemcpyDeviceToHost, st), "result");
-    ck(cudaMemcpyAsync(status_host, O.words, sizeof(int), cudaMemcpyDeviceToHost, st), "status");
-    A.last_d2h = ob + sizeof(int);
+    const size_t lead = D.o_out - D.o_words;  // the status word leads the launch words
+    A.outstage.reserve(lead + ob);
+    ck(cudaMemcpyAsync(A.outstage.p, base + D.o_words, lead + ob, cudaMemcpyDeviceToHost, st), "result");
+    A.last_d2h = lead + ob;
     ck(cudaStreamSynchronize(st), "query sync");
-    if (*status_host == 0) std::memcpy(host_out, A.outstage.p, ob);
-    return *status_host;
+    const int status = *reinterpret_cast<const int*>(A.outstage.p);
+    if (status == 0) std::memcpy(host_out, A.outstage.p + lead, ob);
+    return status;
 }
 
 // ---------------------------------------------------------------------------
@@ -2933,7 +2946,7 @@ htrip_status htrip_query_all_pairs_noalloc(htrip_index* h, const int32_t* vps, i
         return fail(HTRIP_ERR_UNSUPPORTED, "query needs " + std::to_string(L.total) +
                                                " bytes of device scratch; the allocation-free entry point has " +
                                                std::to_string(kNoAllocScratchBytes) + " (fewer viewpoints or a smaller map)");
-    std::vector<unsigned char> stage(L.head);
+    std::vector<unsigned char> stage(L.staged);
     std::lock_guard<std::mutex> lock(g_noalloc_mu);
     unsigned char* base = noalloc_scratch(h->device);
     cudaStream_t st = h->stream;
