@@ -774,7 +774,11 @@ void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int 
         hb::launch_leaf_bfs(h->pass.p, h->S, h->b, h->leaves_x, count(0), h->L[0].ms(), st,
                             bs.all ? nullptr : reinterpret_cast<const int*>(ds + o_leaves));
     ck(cudaGetLastError(), "leaf bfs");
-    if (!wl.empty()) {
+    if (!wl.empty() && h->L[0].NP == 64) {
+        hb::launch_leaf_weight_close(h->pass.p, h->wts.p, h->S, h->b, h->leaves_x, (int)wl.size(), h->L[0].ms(),
+                                     reinterpret_cast<const int*>(ds + o_wl), st);
+        ck(cudaGetLastError(), "weighted leaves");
+    } else if (!wl.empty()) {
         hb::launch_leaf_weight_init(h->pass.p, h->wts.p, h->S, h->b, h->leaves_x, (int)wl.size(), h->L[0].ms(),
                                     h->L[0].kflag.p, reinterpret_cast<const int*>(ds + o_wl), st);
         ck(cudaGetLastError(), "weighted leaf init");

@@ -5,8 +5,8 @@
 // padding; matrix m of a level lives at base + m*NP*NP.  All arithmetic is
 // the exact clamped min-plus of minplus.cuh, so every result is identical to
 // the reference's scalar / AVX2 arithmetic.
+#include "closure.cuh"
 #include "kernels.cuh"
-#include "minplus.cuh"
 
 #include <algorithm>
 
@@ -30,62 +30,81 @@ __global__ void passable_kernel(const uint8_t* __restrict__ observed, int rows, 
 }
 
 // ---------------------------------------------------------------------------
-// Leaf APSP: one warp per source cell, bit-parallel BFS.  Lane r owns row r
-// of the b x b leaf as a bitmask; a BFS level is one shift/shuffle step, so
-// the BFS level number is the reference's BFS distance (leaf_tile.cpp:111-152).
-// Non-passable sources keep the tropical identity row (leaf_tile.cpp:66-68).
+// Leaf APSP (leaf_tile.cpp:111-152): breadth-first search from every cell of a
+// b x b leaf at once.  Thread t = cell t holds the set of sources that reach it
+// as a bit mask over SRC sources; a step ORs the four neighbours' sets, and the
+// bits it adds are the sources at that distance.  Non-passable sources keep
+// the tropical identity row (leaf_tile.cpp:66-68).  A CTA has 256 / TL leaves of TL
+// threads (TL = 1024: one) and SRC sources; their distances are gathered in
+// shared memory and written as SRC-column row pieces.
+// Bound by the write of D (1024 x 1024 map, b = 8: 134 MB, 20 us at the measured copy
+// rate).  One warp per source with a lane per leaf row, which this replaces, had
+// 8 of 32 lanes at work and took 615 us there; this takes 111 us (256 x 256 map,
+// b = 16: 95 -> 45 us).
 // ---------------------------------------------------------------------------
-constexpr int kBfsWarps = 8;
+template <int SRC> struct SourceSet;
+template <> struct SourceSet<64> { typedef unsigned long long T; };
+template <> struct SourceSet<32> { typedef uint32_t T; };
 
-__global__ void __launch_bounds__(kBfsWarps * 32)
+template <int TL, int SRC>
+constexpr size_t bfs_leaf_smem() {
+    return (size_t)TL * (2 * sizeof(typename SourceSet<SRC>::T) + (SRC + 2) * sizeof(uint16_t));
+}
+
+template <int TL, int SRC>
+__global__ void __launch_bounds__(TL < 256 ? 256 : TL)
 leaf_bfs_kernel(const uint8_t* __restrict__ pass, int S, int b, int leaves_x, MatSet L, const int* __restrict__ list,
-                int y0) {
-    extern __shared__ __align__(16) uint16_t sm_rows[];
-    const int leaf = list ? list[y0 + blockIdx.y] : y0 + blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int src = blockIdx.x * kBfsWarps + warp;
-    const int NP = L.NP, n = b * b;
-    if (src >= NP) return;
-    uint16_t* row = sm_rows + (size_t)warp * NP;
-    const int ty = leaf / leaves_x, tx = leaf % leaves_x;
-    const int R0 = ty * b, C0 = tx * b;
-    uint32_t m = 0;
-    if (lane < b) {
-        const uint8_t* p = pass + (size_t)(R0 + lane) * S + C0;
-        for (int c = 0; c < b; ++c) m |= (uint32_t)(p[c] != 0) << c;
+                int n_leaves) {
+    typedef typename SourceSet<SRC>::T Set;
+    constexpr int LD = SRC + 2;  // padded row: the cells' entries for one source hit distinct banks
+    extern __shared__ __align__(16) unsigned char bsm[];
+    const int sub = threadIdx.x / TL, t = threadIdx.x % TL;
+    const int at = blockIdx.x * (blockDim.x / TL) + sub;
+    const bool live = at < n_leaves;
+    const int leaf = live ? (list ? list[at] : at) : 0;
+    const int NP = L.NP, n = b * b, s0 = blockIdx.y * SRC;
+    Set* reach = reinterpret_cast<Set*>(bsm + sub * bfs_leaf_smem<TL, SRC>());  // [2][TL]
+    uint16_t* dist = reinterpret_cast<uint16_t*>(reach + 2 * TL);               // [TL][LD]
+    const int r = t / b, c = t - r * b;
+    const bool open = live && t < n &&
+                      pass[(size_t)(leaf / leaves_x * b + r) * S + (leaf % leaves_x) * b + c] != 0;
+    uint16_t* row = dist + t * LD;
+    for (int j = 0; j < SRC / 2; ++j) reinterpret_cast<uint32_t*>(row)[j] = INF2;
+    Set mine = 0;
+    if (t >= s0 && t < s0 + SRC && t < n) {
+        row[t - s0] = 0;
+        if (open) mine = (Set)1 << (t - s0);
     }
-    for (int j = lane; j < NP; j += 32) row[j] = INF;
-    __syncwarp();
-    if (src < n) {
-        const int sr = src / b, sc = src % b;
-        const uint32_t srow = __shfl_sync(FULL, m, sr);
-        if (lane == 0) row[src] = 0;
-        if ((srow >> sc) & 1u) {
-            const uint32_t rowmask = (b == 32) ? FULL : ((1u << b) - 1u);
-            uint32_t vis = (lane == sr) ? (1u << sc) : 0u;
-            uint32_t front = vis;
-            for (int d = 1;; ++d) {
-                uint32_t up = __shfl_up_sync(FULL, front, 1);
-                uint32_t dn = __shfl_down_sync(FULL, front, 1);
-                if (lane == 0) up = 0;
-                if (lane == 31) dn = 0;
-                const uint32_t nb = ((front << 1) | (front >> 1) | up | dn) & rowmask;
-                uint32_t nw = nb & m & ~vis;
-                vis |= nw;
-                front = nw;
-                if (!__any_sync(FULL, nw)) break;
-                while (nw) {
-                    const int c = __ffs(nw) - 1;
-                    nw &= nw - 1;
-                    row[lane * b + c] = (uint16_t)d;
-                }
-            }
+    reach[t] = mine;
+    __syncthreads();
+    const bool left = c > 0, right = c < b - 1, up = r > 0, down = r < b - 1 && t < n;
+    for (int d = 1, p = 0;; ++d, p ^= 1) {
+        const Set* R = reach + p * TL + t;
+        Set add = 0;
+        if (open) {
+            if (left) add |= R[-1];
+            if (right) add |= R[1];
+            if (up) add |= R[-b];
+            if (down) add |= R[b];
+            add &= ~mine;
+            mine |= add;
+        }
+        reach[(p ^ 1) * TL + t] = mine;
+        if (!__syncthreads_or(add != 0)) break;
+        while (add) {
+            const int s = SRC == 64 ? __ffsll((long long)add) - 1 : __ffs((int)add) - 1;
+            add &= add - 1;
+            row[s] = (uint16_t)d;
         }
     }
-    __syncwarp();
-    uint4* dst = reinterpret_cast<uint4*>(mat_ptr(L, leaf) + (size_t)src * NP);
-    const uint4* s4 = reinterpret_cast<const uint4*>(row);
-    for (int j = lane; j < NP / 8; j += 32) dst[j] = s4[j];
+    __syncthreads();
+    if (!live) return;
+    uint16_t* out = L.base + (size_t)leaf * NP * NP + s0;
+    for (int e = t; e < NP * (SRC / 2); e += TL) {
+        const int i = e / (SRC / 2), w = e % (SRC / 2);
+        reinterpret_cast<uint32_t*>(out + (size_t)i * NP)[w] =
+            i < n ? reinterpret_cast<const uint32_t*>(dist + i * LD)[w] : INF2;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -130,6 +149,44 @@ __global__ void leaf_weight_init_kernel(const uint8_t* __restrict__ pass, const 
         const uint16_t w = edge_weight(wts[cu], wts[cv]);
         if (w < INF) row[vr * b + vc] = w;
     }
+}
+
+// The same for leaves of padded order 64 (b <= 8), closed in place: Floyd-Warshall
+// over the passable cells on the whole matrix in shared memory, one CTA per
+// leaf (init, compaction and one closure round of three kernels took 72 us for one leaf,
+// this 13 us).
+__global__ void __launch_bounds__(kThreads)
+leaf_weight_close_kernel(const uint8_t* __restrict__ pass, const uint16_t* __restrict__ wts, int S, int b, int leaves_x,
+                         MatSet L, const int* __restrict__ list) {
+    __shared__ __align__(16) uint16_t D[B][kTLD];
+    __shared__ uint16_t w[B];  // the cells' weights, INF where not passable
+    const int leaf = list[blockIdx.x], tid = threadIdx.x, n = b * b;
+    const int R0 = (leaf / leaves_x) * b, C0 = (leaf % leaves_x) * b;
+    if (tid < B) {
+        w[tid] = INF;
+        if (tid < n) {
+            const size_t c = (size_t)(R0 + tid / b) * S + C0 + tid % b;
+            if (pass[c]) w[tid] = min(wts[c], INF);
+        }
+    }
+    __syncthreads();
+    for (int idx = tid; idx < B * B; idx += kThreads) {
+        const int u = idx / B, v = idx % B;
+        uint16_t d = INF;
+        if (u == v && u < n) {
+            d = 0;
+        } else if (u < n && v < n) {
+            const int dr = u / b - v / b, dc = u % b - v % b;
+            if (dr * dr + dc * dc == 1) d = edge_weight(w[u], w[v]);  // INF unless both are passable
+        }
+        D[u][v] = d;
+    }
+    __syncthreads();
+    // a pivot that is not passable has an INF row: no change.  D[k][k] = 0 below n.
+    close_pivot_block(D, n);
+    uint16_t* out = mat_ptr(L, leaf);
+    for (int idx = tid; idx < B * B / 8; idx += kThreads)
+        reinterpret_cast<uint4*>(out)[idx] = *reinterpret_cast<const uint4*>(&D[idx / 8][(idx % 8) * 8]);
 }
 
 // ---------------------------------------------------------------------------
@@ -546,13 +603,21 @@ void launch_passable(const uint8_t* observed, int rows, int cols, uint8_t* pass,
     passable_kernel<<<dim3(blocks_for(S, 64), blocks_for(S, 4)), block, 0, st>>>(observed, rows, cols, pass, S);
 }
 
+template <int TL, int SRC>
+static void launch_bfs_t(const uint8_t* pass, int S, int b, int leaves_x, int n_leaves, MatSet leaves,
+                         cudaStream_t st, const int* list) {
+    constexpr int threads = TL < 256 ? 256 : TL, per = threads / TL;
+    const size_t smem = per * bfs_leaf_smem<TL, SRC>();
+    cudaFuncSetAttribute(leaf_bfs_kernel<TL, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const dim3 grid(blocks_for(n_leaves, per), leaves.NP / SRC);
+    leaf_bfs_kernel<TL, SRC><<<grid, threads, smem, st>>>(pass, S, b, leaves_x, leaves, list, n_leaves);
+}
+
 void launch_leaf_bfs(const uint8_t* pass, int S, int b, int leaves_x, int n_leaves, MatSet leaves,
                      cudaStream_t st, const int* list) {
-    const size_t smem = (size_t)kBfsWarps * leaves.NP * sizeof(uint16_t);
-    for (int y0 = 0; y0 < n_leaves; y0 += kMaxGridY) {
-        dim3 grid(blocks_for(leaves.NP, kBfsWarps), std::min(kMaxGridY, n_leaves - y0));
-        leaf_bfs_kernel<<<grid, kBfsWarps * 32, smem, st>>>(pass, S, b, leaves_x, leaves, list, y0);
-    }
+    if (b <= 8) launch_bfs_t<64, 64>(pass, S, b, leaves_x, n_leaves, leaves, st, list);
+    else if (b <= 16) launch_bfs_t<256, 64>(pass, S, b, leaves_x, n_leaves, leaves, st, list);
+    else launch_bfs_t<1024, 32>(pass, S, b, leaves_x, n_leaves, leaves, st, list);
 }
 
 void launch_leaf_weight_init(const uint8_t* pass, const uint16_t* wts, int S, int b, int leaves_x, int n_leaves,
@@ -562,6 +627,11 @@ void launch_leaf_weight_init(const uint8_t* pass, const uint16_t* wts, int S, in
         dim3 grid(blocks_for(leaves.NP, kWarps), std::min(kMaxGridY, n_leaves - y0));
         leaf_weight_init_kernel<<<grid, kWarps * 32, 0, st>>>(pass, wts, S, b, leaves_x, leaves, kflag, list, y0);
     }
+}
+
+void launch_leaf_weight_close(const uint8_t* pass, const uint16_t* wts, int S, int b, int leaves_x, int n_leaves,
+                              MatSet leaves, const int* list, cudaStream_t st) {
+    leaf_weight_close_kernel<<<n_leaves, kThreads, 0, st>>>(pass, wts, S, b, leaves_x, leaves, list);
 }
 
 void launch_compact_pivots(const Slot* S, int n, int NP, int* slot_cnt, cudaStream_t st) {

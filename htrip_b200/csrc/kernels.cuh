@@ -70,6 +70,10 @@ void launch_pad_fill(MatSet M, int count, cudaStream_t st);
 void launch_leaf_weight_init(const uint8_t* pass, const uint16_t* wts, int S, int b, int leaves_x, int n_leaves,
                              MatSet leaves, uint8_t* kflag, const int* list, cudaStream_t st);
 
+// The same and the closure in one kernel, for leaves of padded order 64.
+void launch_leaf_weight_close(const uint8_t* pass, const uint16_t* wts, int S, int b, int leaves_x, int n_leaves,
+                              MatSet leaves, const int* list, cudaStream_t st);
+
 // One matrix of an update launch (any index, any map size: the launch's
 // matrices share b, g and level, hence order, padding and port tables).
 struct Slot {

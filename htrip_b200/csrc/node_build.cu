@@ -20,7 +20,7 @@
 // bit for bit; each matrix is written once instead of once per 64 pivots.
 // Measured against the blocked closure over the seam endpoints that it
 // replaces (device time, B200): building a 1024 x 1024 street map, b = 8, 22.8 ->
-// 5.2 ms; one weight change on a 256 x 256 map, b = 8, 2.45 -> 0.53 ms.
+// 4.6 ms; one weight change on a 256 x 256 map, b = 8, 2.45 -> 0.42 ms.
 #include "closure.cuh"
 #include "kernels.cuh"
 
@@ -625,13 +625,17 @@ __global__ void __launch_bounds__(32 * W * KS, 2) node_tile_kernel(const NodeBui
 // ---------------------------------------------------------------------------
 // Nodes with at most 64 seams and 64 ports per child (the lowest levels, of
 // which there are thousands): one CTA does a whole node in shared memory.
-// LC lanes hold the column pairs of a child (16 for up to 32 ports).
+// LC lanes hold the column pairs of a child (16 for up to 32 ports); NT threads.
+// Latency-bound, so global loads go out in batches (R rows four at a time, a
+// row's child summary before the products) and the product loops are unrolled:
+// one node of 64 seams 91 -> 56 us, 1024 of them 341 -> 285 us, 4096 of 32 seams
+// 252 -> 217 us.
 // ---------------------------------------------------------------------------
 constexpr int kSmallSeams = 64, kSmallPorts = 64;
 
 struct SmallLayout {
     int RP, ldU;  // row strides of R and U (multiples of 8)
-    size_t o_inc, o_R, o_T, o_U, total;
+    size_t o_inc, o_ext, o_R, o_T, o_U, total;
 };
 __host__ __device__ inline SmallLayout small_layout(int g2, int nP, int capI) {
     SmallLayout L;
@@ -640,6 +644,8 @@ __host__ __device__ inline SmallLayout small_layout(int g2, int nP, int capI) {
     size_t o = kSmallSeams * sizeof(int4);
     L.o_inc = o;
     o += (size_t)g2 * capI * sizeof(uint2);
+    L.o_ext = o;
+    o += kSmallPorts * sizeof(int);
     o = (o + 15) / 16 * 16;
     L.o_R = o;
     o += (size_t)g2 * capI * L.RP * sizeof(uint16_t);
@@ -651,8 +657,9 @@ __host__ __device__ inline SmallLayout small_layout(int g2, int nP, int capI) {
     return L;
 }
 
-template <int LC>
-__global__ void __launch_bounds__(kThreads) node_small_kernel(const NodeBuild P) {
+template <int LC, int NT>
+__global__ void __launch_bounds__(NT) node_small_kernel(const NodeBuild P) {
+    constexpr int kW = NT / 32;
     extern __shared__ __align__(16) unsigned char nsm[];
     __shared__ int q_cnt[256];
     __shared__ int s_w0, s_nE, s_chg;
@@ -662,12 +669,14 @@ __global__ void __launch_bounds__(kThreads) node_small_kernel(const NodeBuild P)
     const SmallLayout L = small_layout(g2, nP, P.capI);
     int4* edge = reinterpret_cast<int4*>(nsm);
     uint2* inc = reinterpret_cast<uint2*>(nsm + L.o_inc);
+    int* cext = reinterpret_cast<int*>(nsm + L.o_ext);
     uint16_t* R = reinterpret_cast<uint16_t*>(nsm + L.o_R);
     uint16_t (*T)[kTLD] = reinterpret_cast<uint16_t (*)[kTLD]>(nsm + L.o_T);
     uint16_t* U = reinterpret_cast<uint16_t*>(nsm + L.o_U);
     const int node = node_id(P, i);
     if (tid < g2) q_cnt[tid] = 0;
     if (tid == 0) s_chg = 0;
+    for (int j = tid; j < nP; j += NT) cext[j] = P.cext[j];
     uint16_t w = INF;
     unsigned bal = 0;
     if (tid < kSmallSeams) {
@@ -688,17 +697,31 @@ __global__ void __launch_bounds__(kThreads) node_small_kernel(const NodeBuild P)
     }
     __syncthreads();
     const int nE = s_w0 + s_nE;
-    for (int q = 0; q < g2; ++q) {
-        const uint16_t* cm = child_mat(P, node, q);
-        for (int k = warp; k < q_cnt[q]; k += kWarps) {
-            const uint2 rec = inc[q * P.capI + k];
-            const uint16_t* crow = cm + (size_t)P.cext[rec.x & 0xffffu] * P.C.NP;
-            for (int j = lane; j < L.RP; j += 32)
-                R[(q * P.capI + k) * L.RP + j] = j < nP ? (uint16_t)sat_add(crow[P.cext[j]], rec.x >> 16) : INF;
+    // R: the two incidences of every edge, one warp per row, four rows in flight
+    for (int r0 = warp; r0 < 2 * nE; r0 += 4 * kW) {
+        uint32_t v[4][2], off[4];
+        int at[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int r = min(r0 + x * kW, 2 * nE - 1);
+            const int4 e = edge[r >> 1];
+            const int q = r & 1 ? e.x >> 8 : e.x & 255, k = r & 1 ? (int)((unsigned)e.y >> 16) : e.y & 0xffff;
+            const int port = r & 1 ? (int)((unsigned)e.z >> 16) : e.z & 0xffff;
+            const uint16_t* crow = child_mat(P, node, q) + (size_t)cext[port] * P.C.NP;
+            at[x] = (q * P.capI + k) * L.RP;
+            off[x] = r & 1 ? (uint32_t)e.w : 0u;
+            v[x][0] = lane < nP ? __ldg(crow + cext[lane]) : INF;
+            v[x][1] = lane + 32 < nP ? __ldg(crow + cext[lane + 32]) : INF;
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            if (r0 + x * kW >= 2 * nE) continue;
+            if (lane < L.RP) R[at[x] + lane] = (uint16_t)sat_add(v[x][0], off[x]);
+            if (lane + 32 < L.RP) R[at[x] + lane + 32] = (uint16_t)sat_add(v[x][1], off[x]);
         }
     }
     __syncthreads();
-    for (int idx = tid; idx < B * B; idx += kThreads) {
+    for (int idx = tid; idx < B * B; idx += NT) {
         const int a = idx >> 6, c = idx & 63;
         uint32_t v = INF;
         if (a < nE && c < nE) {
@@ -716,10 +739,12 @@ __global__ void __launch_bounds__(kThreads) node_small_kernel(const NodeBuild P)
         T[a][c] = (uint16_t)v;
     }
     __syncthreads();
-    close_pivot_block(T, nE);
+    if (tid < kThreads) close_pivot_block(T, nE);
+    else
+        for (int k = 0; k < nE; ++k) __syncthreads();  // its barriers
     __syncthreads();
     // sub-warps of LC lanes; a lane holds one column pair of a child
-    constexpr int kSub = 32 / LC, kSubs = kWarps * kSub;
+    constexpr int kSub = 32 / LC, kSubs = kW * kSub;
     const int sub = warp * kSub + lane / LC, cl = lane % LC;
     const bool col_ok = 2 * cl < nP;
     {   // U: items of 4 edges x one child
@@ -727,7 +752,9 @@ __global__ void __launch_bounds__(kThreads) node_small_kernel(const NodeBuild P)
         for (int it = sub; it < ng * g2; it += kSubs) {
             const int p = it / ng, e0 = (it - p * ng) * 4;
             uint32_t acc[4] = {INF2, INF2, INF2, INF2};
-            for (int k = 0; k < q_cnt[p]; ++k) {
+            const int n = q_cnt[p];
+#pragma unroll 4
+            for (int k = 0; k < n; ++k) {
                 const uint2 a = *reinterpret_cast<const uint2*>(&T[inc[p * P.capI + k].y][e0]);
                 const uint32_t bv = reinterpret_cast<const uint32_t*>(R + (p * P.capI + k) * L.RP)[col_ok ? cl : 0];
                 const uint32_t av[4] = {splat(a.x), splat(a.x >> 16), splat(a.y), splat(a.y >> 16)};
@@ -754,10 +781,23 @@ __global__ void __launch_bounds__(kThreads) node_small_kernel(const NodeBuild P)
         }
         if (q >= g2) break;
         const int i0 = (it - first) * 8;
-        uint32_t acc[8];
+        const int lo = q * nP, hi = lo + nP, col = lo + 2 * cl;
+        uint32_t acc[8], own[8];  // own: the rows' child summary (rows of child q)
 #pragma unroll
-        for (int r = 0; r < 8; ++r) acc[r] = INF2;
-        for (int k = 0; k < q_cnt[q]; ++k) {
+        for (int r = 0; r < 8; ++r) acc[r] = own[r] = INF2;
+        if (col_ok && i0 + 8 > lo) {
+            const uint16_t* cm = child_mat(P, node, q);
+            const int c0 = cext[2 * cl], c1 = cext[2 * cl + 1];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const int row = min(max(i0 + r - lo, 0), nP - 1);
+                const uint16_t* crow = cm + (size_t)cext[row] * P.C.NP;
+                if (i0 + r >= lo) own[r] = (uint32_t)__ldg(crow + c0) | ((uint32_t)__ldg(crow + c1) << 16);
+            }
+        }
+        const int n = q_cnt[q];
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) {
             const uint4 a = *reinterpret_cast<const uint4*>(U + inc[q * P.capI + k].y * L.ldU + i0);
             const uint32_t bv = reinterpret_cast<const uint32_t*>(R + (q * P.capI + k) * L.RP)[col_ok ? cl : 0];
             const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
@@ -769,16 +809,11 @@ __global__ void __launch_bounds__(kThreads) node_small_kernel(const NodeBuild P)
             }
         }
         if (!col_ok) continue;
-        const int lo = q * nP, hi = lo + nP, col = lo + 2 * cl;
-        const uint16_t* cm = child_mat(P, node, q);
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
             const int row = i0 + r;
             if (row >= hi) continue;
-            if (row >= lo) {
-                const uint16_t* crow = cm + (size_t)P.cext[row - lo] * P.C.NP;
-                acc[r] = min2(acc[r], (uint32_t)crow[P.cext[2 * cl]] | ((uint32_t)crow[P.cext[2 * cl + 1]] << 16));
-            }
+            acc[r] = min2(acc[r], own[r]);
             uint32_t* d = reinterpret_cast<uint32_t*>(D + (size_t)row * NP + col);
             if (P.changed && P.isext[row]) {
                 const uint32_t diff = *d ^ acc[r];
@@ -881,11 +916,11 @@ void launch_node_build(const NodeBuild& P, int n, cudaStream_t st) {
     if (node_build_small(P)) {
         const size_t smem = small_layout(g2, P.nP, P.capI).total;
         if (P.nP <= 32) {
-            allow_smem(node_small_kernel<16>, smem);
-            node_small_kernel<16><<<n, kThreads, smem, st>>>(P);
+            allow_smem(node_small_kernel<16, 256>, smem);
+            node_small_kernel<16, 256><<<n, 256, smem, st>>>(P);
         } else {
-            allow_smem(node_small_kernel<32>, smem);
-            node_small_kernel<32><<<n, kThreads, smem, st>>>(P);
+            allow_smem(node_small_kernel<32, 512>, smem);
+            node_small_kernel<32, 512><<<n, 512, smem, st>>>(P);
         }
         return;
     }

@@ -49,6 +49,9 @@ CASES = [
     ("street", 120, 100, 8, 2),
     ("maze", 128, 97, 8, 2),
     ("snake", 64, 64, 8, 2),      # distances up to 2 k
+    ("noise", 21, 20, 7, 2),      # leaves of 49 cells (fewer than their padded order)
+    ("noise", 40, 36, 9, 2),      # leaves of 81 cells: 256 threads, padded order 128
+    ("maze", 31, 31, 31, 2),      # one leaf of 961 cells, 32 sources a time
     ("snake", 200, 200, 16, 2),   # up to 20 k: sums above half of the range
 ]
 
