@@ -33,12 +33,9 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-// Distances of at most kHalfMax add up below kHalfInf, so with INF replaced
-// by kHalfInf a sum needs no clamp: it never wraps (65534 at most) and a sum
-// of kHalfInf or more means INF.
-constexpr int kHalfMax = 16383;
-constexpr uint32_t kHalfInf = 32767u;
-constexpr uint32_t kHalfInf2 = 0x7FFF7FFFu;
+// Half range (closure.cuh): distances of at most kHalfMax add up below kHalfInf, so
+// with INF replaced by kHalfInf a sum needs no clamp: it never wraps (65534 at most)
+// and a sum of kHalfInf or more means INF.
 
 __device__ __forceinline__ int node_id(const NodeBuild& P, int i) { return P.list ? P.list[i] : P.first + i; }
 
@@ -373,10 +370,7 @@ __device__ __forceinline__ void tile_minplus(uint32_t (&out)[RW / KS][CP], ARow 
 #pragma unroll
         for (int r = 0; r < RW / KS; ++r)
 #pragma unroll
-            for (int c = 0; c < CP; ++c) {
-                const uint32_t lo = out[r][c] & 0xffffu, hi = out[r][c] >> 16;
-                out[r][c] = (lo >= kHalfInf ? (uint32_t)INF : lo) | ((hi >= kHalfInf ? (uint32_t)INF : hi) << 16);
-            }
+            for (int c = 0; c < CP; ++c) out[r][c] = half_to_full(out[r][c]);
     }
 }
 

@@ -423,82 +423,6 @@ __device__ void compact_unit(const OpenLaunch& L, int l, int s) {
 // stored in the slot's panel, with the 64-column blocks holding a finite
 // value flagged for the update.
 // ---------------------------------------------------------------------------
-// Class of pivot k for warp w's 8 rows of T* (entries T*[k][8w .. 8w+7]):
-// 0 all INF (skip), 1 all <= INF_HEADROOM (2-op form), 2 otherwise.
-__device__ __forceinline__ void panel_classes(uint16_t (*Ts)[kTLD], int mk, uint8_t* cls) {
-    for (int idx = threadIdx.x; idx < mk * kWarps; idx += kThreads) {
-        const int k = idx / kWarps, w = idx % kWarps;
-        uint32_t mn = 0xffffu, mx = 0;
-#pragma unroll
-        for (int rr = 0; rr < 8; ++rr) {
-            const uint32_t v = Ts[k][w * 8 + rr];
-            mn = min(mn, v);
-            mx = max(mx, v);
-        }
-        cls[idx] = mn >= INF ? 0 : (mx <= INF_HEADROOM ? 1 : 2);
-    }
-}
-
-// acc[r][c] = min_k T*[k][8w + r] (+) Bs[k][lane's pair c]  (T* symmetric:
-// T*[k][a] = T*[a][k]); warp w owns pivot rows 8w..8w+7.
-template <int CP>
-__device__ __forceinline__ void panel_gemm(uint16_t (*Ts)[kTLD], const uint16_t* Bs, int ldb, int mk,
-                                           const uint8_t* cls, uint32_t (&acc)[8][CP]) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-    for (int rr = 0; rr < 8; ++rr)
-#pragma unroll
-        for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = INF2;
-    if constexpr (CP == 1) {
-        // one column pair per lane: little work per pivot, so the loop is
-        // latency-bound; it runs branch-free (the clamped form is exact for
-        // every value, INF included) and unrolled, so the shared-memory loads
-        // of later pivots overlap the arithmetic of earlier ones
-        (void)cls;
-#pragma unroll 4
-        for (int k = 0; k < mk; ++k) {
-            const uint32_t bv = reinterpret_cast<const uint32_t*>(Bs + k * ldb + lane * 2)[0];
-            const uint4 av = *reinterpret_cast<const uint4*>(&Ts[k][warp * 8]);
-            const uint32_t aw[4] = {av.x, av.y, av.z, av.w};
-#pragma unroll
-            for (int r2 = 0; r2 < 4; ++r2) {
-                const uint32_t a0 = splat(aw[r2]), a1 = splat(aw[r2] >> 16);
-                acc[2 * r2][0] = acc_clamp(acc[2 * r2][0], bv, a0, INF2 - a0);
-                acc[2 * r2 + 1][0] = acc_clamp(acc[2 * r2 + 1][0], bv, a1, INF2 - a1);
-            }
-        }
-    } else {
-        for (int k = 0; k < mk; ++k) {
-            const int c = cls[k * kWarps + warp];
-            if (c == 0) continue;  // uniform over the warp
-            uint32_t bv[CP];
-#pragma unroll
-            for (int cc = 0; cc < CP; ++cc) bv[cc] = reinterpret_cast<const uint32_t*>(Bs + k * ldb + lane * 2 * CP)[cc];
-            const uint4 av = *reinterpret_cast<const uint4*>(&Ts[k][warp * 8]);
-            const uint32_t aw[4] = {av.x, av.y, av.z, av.w};
-            uint32_t aa[8];
-#pragma unroll
-            for (int r2 = 0; r2 < 4; ++r2) {
-                aa[2 * r2] = splat(aw[r2]);
-                aa[2 * r2 + 1] = splat(aw[r2] >> 16);
-            }
-            if (c == 1) {
-#pragma unroll
-                for (int rr = 0; rr < 8; ++rr)
-#pragma unroll
-                    for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = acc_fast(acc[rr][cc], bv[cc], aa[rr]);
-            } else {
-#pragma unroll
-                for (int rr = 0; rr < 8; ++rr) {
-                    const uint32_t tt = INF2 - aa[rr];
-#pragma unroll
-                    for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = acc_clamp(acc[rr][cc], bv[cc], aa[rr], tt);
-                }
-            }
-        }
-    }
-}
-
 __device__ __forceinline__ uint16_t* panel_of(const OpenLaunch& L, int r, int s, int NP) {
     return L.panel + (size_t)(r & 1) * L.panel_stride + (size_t)s * B * NP;
 }
@@ -514,6 +438,12 @@ __device__ __forceinline__ uint8_t* pflags_of(const OpenLaunch& L, int r, int s,
 // to the pivot block and to the tile's columns.  A value it reads either
 // still misses the update or already holds it; the minimum is the updated
 // value both ways, so the panel equals the one made after the update.
+struct PanelSmem {
+    FwSmem<4> fw;              // [T | the tile's pivot rows]
+    alignas(16) uint16_t Q[B][FwSmem<4>::LD];  // round r - 1's panel at {the pivots, the tile's columns}
+    int kc[B];
+};
+
 __device__ void panel_unit(const OpenLaunch& L, int l, int s, int j0, int r, unsigned char* smem) {
     constexpr int NT = 64;
     const int NP = L.geo[l].NP;
@@ -521,79 +451,62 @@ __device__ void panel_unit(const OpenLaunch& L, int l, int s, int j0, int r, uns
     const int mk = min(B, rec.kcnt - r * B);
     if (mk <= 0) return;  // uniform
     const bool ahead = r > 0;
-    uint16_t (*Ts)[kTLD] = reinterpret_cast<uint16_t (*)[kTLD]>(smem);
-    uint16_t (*Ag)[kTLD] = reinterpret_cast<uint16_t (*)[kTLD]>(smem + B * kTLD * sizeof(uint16_t));  // Pp[c][Kc[a]]
-    uint16_t (*Bt)[kTLD] = reinterpret_cast<uint16_t (*)[kTLD]>(smem + 2 * B * kTLD * sizeof(uint16_t));  // tile rows
-    uint16_t* Bs = &Bt[0][0];
-    uint16_t* Pj = Bs + B * kTLD;  // [B][NT]: Pp[c][j0 + j]
-    int* kc = reinterpret_cast<int*>(Pj + B * NT);
-    uint8_t* clsA = reinterpret_cast<uint8_t*>(kc + B);  // [B][kWarps] of Ag
-    __shared__ int tile_any;
+    PanelSmem& W = *reinterpret_cast<PanelSmem*>(smem);
     const uint16_t* D = rec.mat;
     const uint16_t* Pp = ahead ? panel_of(L, r - 1, s, NP) : nullptr;
     const int tid = threadIdx.x;
-    if (tid < mk) kc[tid] = __ldcg(rec.klist + r * B + tid);
-    if (tid == 0) tile_any = 0;
+    if (tid < mk) W.kc[tid] = __ldcg(rec.klist + r * B + tid);
     __syncthreads();
-    {   // the tile's pivot rows (and round r - 1's panel tile) by asynchronous
-        // copies, waited for only where they are used; meanwhile the
-        // scattered pivot block (and its round r - 1 panel columns) with
-        // all of a thread's loads issued first
-        for (int idx = tid; idx < mk * (NT / 8); idx += kThreads) {
-            const int a = idx / (NT / 8), c8 = idx % (NT / 8);
-            cp_async16(Bs + a * kTLD + c8 * 8, D + (size_t)kc[a] * NP + j0 + c8 * 8);
+    uint32_t m[4][4];
+    for (bool half = true;; half = false) {
+        // the tile's pivot rows (and round r - 1's panel tile) by asynchronous
+        // copies; meanwhile the scattered pivot block (and its round r - 1 panel
+        // columns) with all of a thread's loads issued first
+        for (int idx = tid; idx < B * (NT / 8); idx += kThreads) {
+            const int a = idx / (NT / 8), c8 = idx % (NT / 8) * 8;
+            if (a < mk) cp_async16(&W.fw.M[a][B + c8], D + (size_t)W.kc[a] * NP + j0 + c8);
+            else *reinterpret_cast<uint4*>(&W.fw.M[a][B + c8]) = make_uint4(INF2, INF2, INF2, INF2);
+            if (ahead) cp_async16(&W.Q[a][B + c8], Pp + (size_t)a * NP + j0 + c8);
         }
-        if (ahead)
-            for (int idx = tid; idx < B * (NT / 8); idx += kThreads) {
-                const int c = idx / (NT / 8), c8 = idx % (NT / 8);
-                cp_async16(Pj + c * NT + c8 * 8, Pp + (size_t)c * NP + j0 + c8 * 8);
-            }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
         constexpr int NTB = B * B / kThreads;
         uint16_t tv[NTB], pv[NTB];
 #pragma unroll
         for (int x = 0; x < NTB; ++x) {
             const int idx = tid + x * kThreads, a = idx / B, c = idx % B;
-            tv[x] = (a < mk && c < mk) ? __ldcg(D + (size_t)kc[a] * NP + kc[c]) : (a == c ? 0 : INF);
+            tv[x] = (a < mk && c < mk) ? __ldcg(D + (size_t)W.kc[a] * NP + W.kc[c]) : INF;
             // pv: Pp[a][Kc[c]] (row a of the old panel at pivot c)
-            pv[x] = (ahead && c < mk) ? __ldcg(Pp + (size_t)a * NP + kc[c]) : INF;
+            pv[x] = (ahead && c < mk) ? __ldcg(Pp + (size_t)a * NP + W.kc[c]) : INF;
         }
 #pragma unroll
         for (int x = 0; x < NTB; ++x) {
             const int idx = tid + x * kThreads;
-            Ts[idx / B][idx % B] = tv[x];
-            Ag[idx / B][idx % B] = pv[x];
+            W.fw.M[idx / B][idx % B] = tv[x];
+            W.Q[idx / B][idx % B] = pv[x];
         }
-    }
-    __syncthreads();
-    uint32_t acc[2][4];
-    if (ahead) {  // round r - 1's update of the pivot rows: the pivot block, then the tile's columns
-        block_classes(Ag, B, clsA);
-        __syncthreads();
-        gemm64(Ag, &Ag[0][0], kTLD, B, clsA, acc);
-        min_into(&Ts[0][0], kTLD, B, acc);  // rows / columns >= mk: INF from Ag, the identity stays
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();
-        gemm64(Ag, Pj, NT, B, clsA, acc);
-        min_into(Bs, kTLD, mk, acc);
+        // the old panel's update of these rows, then the closure (Q null: round 0)
+        if (fw_panel<4>(W.fw, ahead ? &W.Q[0][0] : nullptr, mk, half, m)) break;
+        __syncthreads();  // every thread has read the verdict
     }
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();
-    uint32_t vb[8];
-    close_pivot_panel(Ts, Bt, mk, vb);
     uint16_t* P = panel_of(L, r, s, NP);
-    const int lane = tid & 31, a = tid >> 2, c0 = (tid & 3) * 16;
-    bool any = false;
-    if (a < mk) {
-        uint4* dst = reinterpret_cast<uint4*>(P + (size_t)a * NP + j0 + c0);
-        dst[0] = make_uint4(vb[0], vb[1], vb[2], vb[3]);
-        dst[1] = make_uint4(vb[4], vb[5], vb[6], vb[7]);
+    const int rg = tid >> 4, cg = tid & 15;
+    bool any = false, wide = false;
+    if (cg >= 8) {  // the tile's columns
 #pragma unroll
-        for (int i = 0; i < 8; ++i) any |= vb[i] != INF2;
+        for (int x = 0; x < 4; ++x) {
+            const int a = 4 * rg + x;
+            if (a >= mk) continue;
+            *reinterpret_cast<uint4*>(P + (size_t)a * NP + j0 + 8 * (cg - 8)) =
+                make_uint4(m[x][0], m[x][1], m[x][2], m[x][3]);
+            any |= m[x][0] != INF2 || m[x][1] != INF2 || m[x][2] != INF2 || m[x][3] != INF2;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) wide |= !half_ok(m[x][w]);
+        }
     }
-    if (__any_sync(FULL, any) && lane == 0) tile_any = 1;
-    __syncthreads();
-    if (tid == 0) pflags_of(L, r, s, NP)[j0 / 64] = tile_any ? 1 : 0;
+    const int flag = (__syncthreads_or(any) ? 1 : 0) | (__syncthreads_or(wide) ? 2 : 0);
+    if (tid == 0) pflags_of(L, r, s, NP)[j0 / 64] = (uint8_t)flag;
 }
 
 // ---------------------------------------------------------------------------
@@ -606,7 +519,8 @@ __device__ void panel_unit(const OpenLaunch& L, int l, int s, int j0, int r, uns
 // Warp w owns rows RW*w .. RW*w + RW - 1 of the tile, each lane CP column
 // pairs.  Per pivot k the warp's RW panel values share one class, staged
 // with the panel: 0 all INF (skip), 1 all <= INF_HEADROOM (2-op form, no
-// wrap), 2 otherwise (3-op clamped form).
+// wrap), 2 otherwise (3-op clamped form).  Panel blocks without a value beyond the half
+// range (their flag's second bit) take the 2-op form throughout, INF as kHalfInf.
 // ---------------------------------------------------------------------------
 template <int RW, int CP>
 __device__ void update_unit(const OpenLaunch& L, int l, int s, int I, int J, int r, unsigned char* smem) {
@@ -618,13 +532,14 @@ __device__ void update_unit(const OpenLaunch& L, int l, int s, int I, int J, int
     const OpenSlotRec rec = ld_rec(L.rec[l] + s);
     const int mk = min(B, rec.kcnt - r * B);
     if (mk <= 0) return;  // uniform; no panel was made for this slot either
-    bool live_i = false, live_j = false;
+    int live_i = 0, live_j = 0;  // 1: a finite value, 2: one beyond the half range
 #pragma unroll
     for (int t = 0; t < TT / 64; ++t) {
-        live_i |= __ldcg(pf + I * (TT / 64) + t) != 0;
-        live_j |= __ldcg(pf + J * (TT / 64) + t) != 0;
+        live_i |= __ldcg(pf + I * (TT / 64) + t);
+        live_j |= __ldcg(pf + J * (TT / 64) + t);
     }
     if (!live_i || !live_j) return;  // uniform
+    const bool half = ((live_i | live_j) & 2) == 0;
     uint32_t* As = reinterpret_cast<uint32_t*>(smem);                                  // [B][TT] splatted
     uint16_t* Bs = reinterpret_cast<uint16_t*>(smem + (size_t)B * TT * sizeof(uint32_t));  // [B][TT]
     uint8_t* cls = smem + (size_t)B * TT * (sizeof(uint32_t) + sizeof(uint16_t));          // [B][kWarps]
@@ -657,7 +572,11 @@ __device__ void update_unit(const OpenLaunch& L, int l, int s, int I, int J, int
         for (int x = 0; x < NS; ++x) {
             const int idx = tid + x * kThreads, a = idx / (TT / 8), c8 = idx % (TT / 8);
             if (a < mk) {
-                const uint32_t w[4] = {va[x].x, va[x].y, va[x].z, va[x].w};
+                uint32_t w[4] = {va[x].x, va[x].y, va[x].z, va[x].w};
+                if (half) {
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) w[t] = min2(w[t], kHalfInf2);
+                }
                 uint4* dst = reinterpret_cast<uint4*>(As + a * TT + c8 * 8);
                 dst[0] = make_uint4(splat(w[0]), splat(w[0] >> 16), splat(w[1]), splat(w[1] >> 16));
                 dst[1] = make_uint4(splat(w[2]), splat(w[2] >> 16), splat(w[3]), splat(w[3] >> 16));
@@ -666,30 +585,36 @@ __device__ void update_unit(const OpenLaunch& L, int l, int s, int I, int J, int
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
     __syncthreads();
-    for (int idx = tid; idx < mk * kWarps; idx += kThreads) {
-        const int a = idx / kWarps, w = idx % kWarps;
-        const uint32_t* ar = As + a * TT + w * RW;
-        uint32_t mn = 0xffffu, mx = 0;
+    if (!half) {
+        for (int idx = tid; idx < mk * kWarps; idx += kThreads) {
+            const int a = idx / kWarps, w = idx % kWarps;
+            const uint32_t* ar = As + a * TT + w * RW;
+            uint32_t mn = 0xffffu, mx = 0;
 #pragma unroll
-        for (int rr = 0; rr < RW; ++rr) {
-            const uint32_t v = ar[rr] & 0xffffu;
-            mn = min(mn, v);
-            mx = max(mx, v);
+            for (int rr = 0; rr < RW; ++rr) {
+                const uint32_t v = ar[rr] & 0xffffu;
+                mn = min(mn, v);
+                mx = max(mx, v);
+            }
+            cls[idx] = mn >= INF ? 0 : (mx <= INF_HEADROOM ? 1 : 2);
         }
-        cls[idx] = mn >= INF ? 0 : (mx <= INF_HEADROOM ? 1 : 2);
+        __syncthreads();
     }
-    __syncthreads();
     uint32_t acc[RW][CP];
 #pragma unroll
     for (int rr = 0; rr < RW; ++rr)
 #pragma unroll
         for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = INF2;
+#pragma unroll 2
     for (int k = 0; k < mk; ++k) {
-        const int c = cls[k * kWarps + warp];
+        const int c = half ? 1 : cls[k * kWarps + warp];
         if (c == 0) continue;  // uniform over the warp
         uint32_t bv[CP];
 #pragma unroll
-        for (int cc = 0; cc < CP; ++cc) bv[cc] = reinterpret_cast<const uint32_t*>(Bs + k * TT + lane * 2 * CP)[cc];
+        for (int cc = 0; cc < CP; ++cc) {
+            bv[cc] = reinterpret_cast<const uint32_t*>(Bs + k * TT + lane * 2 * CP)[cc];
+            if (half) bv[cc] = min2(bv[cc], kHalfInf2);
+        }
         const uint32_t* ar = As + k * TT + warp * RW;
         uint32_t av[RW];
 #pragma unroll
@@ -710,6 +635,12 @@ __device__ void update_unit(const OpenLaunch& L, int l, int s, int I, int J, int
                 for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = acc_clamp(acc[rr][cc], bv[cc], av[rr], tt);
             }
         }
+    }
+    if (half) {  // sums of kHalfInf or more: INF
+#pragma unroll
+        for (int rr = 0; rr < RW; ++rr)
+#pragma unroll
+            for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = half_to_full(acc[rr][cc]);
     }
     // epilogue: new = min(acc, old); changed entries are written
     const int col = jb + lane * 2 * CP;
@@ -854,58 +785,155 @@ __device__ void stage_phase(const OpenLaunch& L, int l, int N, int t, int rounds
 // Levels whose matrices fit in shared memory (NP <= 128: leaves of b <= 11,
 // the lowest node levels): one unit per slot does the whole update of its
 // matrix in shared memory - the child-summary decreases, the edge / seam
-// list, the pivot compaction and every closure round (pivot block,
-// panel, full update) - and writes the matrix back once.  One phase per
-// level instead of 2 + 2 x rounds.
+// list, the pivot compaction and the closure - and writes the matrix back once.
+// One phase per level instead of 2 + 2 x rounds.
 // ---------------------------------------------------------------------------
-template <int RW, int CP>
+// Closure of the matrix Dm (NP x NP in shared memory) over the pivots kl[0 .. k):
+// Floyd-Warshall with the matrix in registers.  Thread (rg, cg) = (t / 16, t % 16) holds
+// rows TR rg .. and columns TR cg .. (TR = NP / 16); a step needs the pivot row
+// only (the matrix is symmetric, so it is the pivot column too), which its
+// owners put into one of two buffers at the step before: one barrier per pivot, two
+// shared loads per thread.  Against 64-pivot rounds of panel and update it does n^2
+// instead of n (n + 128) operations per pivot and is far less code to fetch
+// (a phase of 38 matrices of order 128, up to 59 pivots: 48 -> 30 us; 70 leaves of
+// order 64: 15 -> 12 us).
+// HALF as in fw_panel, which the result false refers to.
+template <int NP, bool HALF>
+__device__ __forceinline__ bool close_small(const uint16_t* Dm, const int* kl, int k, uint16_t (*Pr)[NP], int* mx,
+                                            uint32_t (&d)[NP / 16][NP / 32]) {
+    constexpr int TR = NP / 16, TW = TR / 2;
+    static_assert(TW == 4 || TW == 2, "NP is 128 or 64");
+    const int tid = threadIdx.x, rg = tid >> 4, cg = tid & 15;
+    uint32_t m0 = 0;
+    auto top = [&] {
+        uint32_t m = 0;
+#pragma unroll
+        for (int r = 0; r < TR; ++r)
+#pragma unroll
+            for (int w = 0; w < TW; ++w) {
+                const uint32_t lo = d[r][w] & 0xffffu, hi = d[r][w] >> 16;
+                if (lo < kHalfInf) m = max(m, lo);
+                if (hi < kHalfInf) m = max(m, hi);
+            }
+        return __reduce_max_sync(FULL, m);
+    };
+    auto publish = [&](int s) {  // pivot s's row
+        const int row = kl[s];
+        if (row / TR != rg) return;
+        // predicated stores, one per row the thread holds (selecting the row in C++
+        // becomes an indexed access, which puts d in local memory)
+        const uint32_t at = (uint32_t)__cvta_generic_to_shared(&Pr[s & 1][TR * cg]);
+#pragma unroll
+        for (int r = 0; r < TR; ++r) {
+            if constexpr (TW == 4)
+                asm volatile("{\n.reg .pred p;\nsetp.eq.s32 p, %0, %1;\n@p st.shared.v4.b32 [%2], {%3, %4, %5, %6};\n}\n" ::"r"(row),
+                             "r"(TR * rg + r), "r"(at), "r"(d[r][0]), "r"(d[r][1]), "r"(d[r][2]), "r"(d[r][3])
+                             : "memory");
+            else
+                asm volatile("{\n.reg .pred p;\nsetp.eq.s32 p, %0, %1;\n@p st.shared.v2.b32 [%2], {%3, %4};\n}\n" ::"r"(row),
+                             "r"(TR * rg + r), "r"(at), "r"(d[r][0]), "r"(d[r][1])
+                             : "memory");
+        }
+    };
+#pragma unroll
+    for (int r = 0; r < TR; ++r) {
+        ld_words<TW>(Dm + (TR * rg + r) * NP + TR * cg, d[r]);
+        if constexpr (HALF)
+#pragma unroll
+            for (int w = 0; w < TW; ++w) d[r][w] = min2(d[r][w], kHalfInf2);
+    }
+    if constexpr (HALF) m0 = top();
+    if (k > 0) publish(0);
+    __syncthreads();
+#pragma unroll 1
+    for (int s = 0; s < k; ++s) {
+        uint32_t a[TW], b[TW];
+        ld_words<TW>(&Pr[s & 1][TR * rg], a);
+        ld_words<TW>(&Pr[s & 1][TR * cg], b);
+#pragma unroll
+        for (int r = 0; r < TR; ++r) {
+            const uint32_t aa = splat(r & 1 ? a[r / 2] >> 16 : a[r / 2]);
+#pragma unroll
+            for (int w = 0; w < TW; ++w) d[r][w] = acc_mode<HALF>(d[r][w], b[w], aa);
+        }
+        if (s + 1 < k) publish(s + 1);
+        __syncthreads();
+    }
+    if constexpr (HALF) {
+        const uint32_t z = top();
+        if ((tid & 31) == 0) {
+            atomicMax(mx, (int)m0);
+            atomicMax(mx + 1, (int)z);
+        }
+        __syncthreads();
+        if (mx[0] + mx[1] >= (int)kHalfInf) return false;
+#pragma unroll
+        for (int r = 0; r < TR; ++r)
+#pragma unroll
+            for (int w = 0; w < TW; ++w) d[r][w] = half_to_full(d[r][w]);
+    }
+    return true;
+}
+
+template <int NP>
 __device__ void small_unit(const OpenLaunch& L, int l, int s, unsigned char* smem) {
-    constexpr int NP = 8 * RW;
-    static_assert(NP == 64 * CP, "square matrix of 8 warps x RW rows and 32 lanes x CP pairs");
+    constexpr int TR = NP / 16, TW = TR / 2;
     const OpenLevelGeom& G = L.geo[l];
     const int4 e = ld_slot(L.slots[l] + s);
     const OpenTask& T = L.tasks[e.x];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint16_t* Dg = node_mat(T.lv[l], e.y, NP);
     uint16_t* Dm = reinterpret_cast<uint16_t*>(smem);                               // [NP][NP]
-    uint16_t* Pm = Dm + NP * NP;                                                     // [B][NP]
-    uint16_t (*Ts)[kTLD] = reinterpret_cast<uint16_t (*)[kTLD]>(Pm + B * NP);       // [B][kTLD]
-    int* kl = reinterpret_cast<int*>(&Ts[B][0]);                                     // [NP]
+    uint16_t (*Pr)[NP] = reinterpret_cast<uint16_t (*)[NP]>(Dm + NP * NP);          // [2][NP] pivot rows
+    int* kl = reinterpret_cast<int*>(Pr + 2);                                        // [NP]
     uint8_t* fl = reinterpret_cast<uint8_t*>(kl + NP);                               // [NP]
-    uint8_t* cls = fl + NP;                                                          // [B][kWarps]
-    __shared__ int s_dec, s_chg, s_np, s_k;
+    __shared__ int s_dec, s_chg, s_np, s_k, s_mx[2];
     __shared__ int wtot[kWarps];
     for (int idx = tid; idx < NP * NP / 8; idx += kThreads) cp_async16(Dm + idx * 8, Dg + idx * 8);
     for (int j = tid; j < NP / 4; j += kThreads) reinterpret_cast<unsigned*>(fl)[j] = 0u;
-    if (tid == 0) { s_dec = 0; s_chg = 0; s_np = 0; }
+    if (tid == 0) { s_dec = 0; s_chg = 0; s_np = 0; s_mx[0] = s_mx[1] = 0; }
     cp_async_wait_all();
     __syncthreads();
     bool dec = false, chg = false;
     if (l >= 1) {  // child-summary decreases (internal_node.cpp:343-353), as in insert_phase
-        const int nx = T.lv[l].nodes_x, g = L.g, nP = G.nP, cNP = G.childNP;
-        for (int q = 0; q < g * g; ++q) {
-            const int child = ((e.y / nx) * g + q / g) * T.lv[l - 1].nodes_x + ((e.y % nx) * g + q % g);
-            if (__ldcg(T.lv[l - 1].dstamp + child) != T.stamp) continue;  // uniform
-            const uint16_t* cm = node_mat(T.lv[l - 1], child, cNP);
-            constexpr int U = 4;  // a thread's loads of U entries first, then their updates
-            for (int b0 = tid; b0 < nP * nP; b0 += U * kThreads) {
-                uint16_t w[U];
-                int ab[U];
+        // rows of the decreased children's summaries, one warp per row, the loads
+        // of four rows in flight
+        const int nx = T.lv[l].nodes_x, g = L.g, g2 = g * g, nP = G.nP, cNP = G.childNP;
+        __shared__ int s_child[256], s_quad[256], s_nd;
+        if (tid == 0) s_nd = 0;
+        __syncthreads();
+        if (tid < g2) {
+            const int child = ((e.y / nx) * g + tid / g) * T.lv[l - 1].nodes_x + ((e.y % nx) * g + tid % g);
+            if (__ldcg(T.lv[l - 1].dstamp + child) == T.stamp) {
+                const int x = atomicAdd(&s_nd, 1);
+                s_child[x] = child;
+                s_quad[x] = tid;
+            }
+        }
+        __syncthreads();
+        const int rows = s_nd * nP;
+        constexpr int U = 4, kCols = (NP + 31) / 32;  // nP <= NP
+        for (int r0 = warp; r0 < rows; r0 += U * kWarps) {
+            uint16_t w[U][kCols];
+            int at[U];
 #pragma unroll
-                for (int x = 0; x < U; ++x) {
-                    const int idx = b0 + x * kThreads;
-                    ab[x] = -1;
-                    if (idx < nP * nP) {
-                        const int p = idx / nP, pp = idx - p * nP;
-                        w[x] = __ldcg(cm + (size_t)G.child_ext[p] * cNP + G.child_ext[pp]);
-                        ab[x] = (q * nP + p) * NP + q * nP + pp;
-                    }
-                }
+            for (int x = 0; x < U; ++x) {
+                const int r = min(r0 + x * kWarps, rows - 1), ci = r / nP, p = r - ci * nP;
+                const uint16_t* crow = node_mat(T.lv[l - 1], s_child[ci], cNP) + (size_t)G.child_ext[p] * cNP;
+                at[x] = (s_quad[ci] * nP + p) * NP + s_quad[ci] * nP;
 #pragma unroll
-                for (int x = 0; x < U; ++x) {
-                    if (ab[x] >= 0 && w[x] < Dm[ab[x]]) {
-                        const int a = ab[x] / NP, b = ab[x] % NP;
-                        Dm[ab[x]] = w[x];  // (b, a) is written by its own thread
+                for (int y = 0; y < kCols; ++y)
+                    if (lane + 32 * y < nP) w[x][y] = __ldcg(crow + G.child_ext[lane + 32 * y]);
+            }
+#pragma unroll
+            for (int x = 0; x < U; ++x) {
+                if (r0 + x * kWarps >= rows) continue;
+#pragma unroll
+                for (int y = 0; y < kCols; ++y) {
+                    const int pp = lane + 32 * y;
+                    if (pp < nP && w[x][y] < Dm[at[x] + pp]) {
+                        const int a = at[x] / NP, b = at[x] % NP + pp;
+                        Dm[at[x] + pp] = w[x][y];  // (b, a) is written by its own row
                         fl[a] = 1;
                         fl[b] = 1;
                         dec |= G.isext[a] && G.isext[b];
@@ -967,109 +995,46 @@ __device__ void small_unit(const OpenLaunch& L, int l, int s, unsigned char* sme
             atomicAdd(&T.out->bytes, 4ull * n * n + 4ull * (unsigned long long)k * n);
         }
     }
-    for (int r = 0; r * B < k; ++r) {
-        const int mk = min(B, k - r * B);
-        const int* kc = kl + r * B;
-        for (int idx = tid; idx < B * B; idx += kThreads) {
-            const int a = idx / B, c = idx % B;
-            Ts[a][c] = (a < mk && c < mk) ? Dm[kc[a] * NP + kc[c]] : (a == c ? 0 : INF);
-        }
-        for (int idx = tid; idx < mk * (NP / 8); idx += kThreads) {  // the pivot rows
-            const int a = idx / (NP / 8), c8 = idx % (NP / 8);
-            reinterpret_cast<uint4*>(Pm + a * NP)[c8] = reinterpret_cast<const uint4*>(Dm + kc[a] * NP)[c8];
-        }
-        __syncthreads();
-        close_pivot_block(Ts, mk);
-        panel_classes(Ts, mk, cls);
-        __syncthreads();
-        {   // the panel P = T* (x) D[Kc, :], into Pm
-            uint32_t pacc[8][CP];
-            panel_gemm<CP>(Ts, Pm, NP, mk, cls, pacc);
-            __syncthreads();
+    uint32_t d[TR][TW];
+    const int rg = tid >> 4, cg = tid & 15;
+    bool ok = true;
 #pragma unroll
-            for (int rr = 0; rr < 8; ++rr) {
-                const int a = warp * 8 + rr;
-                if (a < mk)
+    for (int r = 0; r < TR; ++r) {
+        uint32_t w[TW];
+        ld_words<TW>(Dm + (TR * rg + r) * NP + TR * cg, w);
 #pragma unroll
-                    for (int cc = 0; cc < CP; ++cc)
-                        reinterpret_cast<uint32_t*>(Pm + a * NP + lane * 2 * CP)[cc] = pacc[rr][cc];
+        for (int x = 0; x < TW; ++x) ok &= half_ok(w[x]);
+    }
+    bool done = false;
+    if (__syncthreads_and(ok)) {
+        done = close_small<NP, true>(Dm, kl, k, Pr, s_mx, d);
+        __syncthreads();  // the pivot row buffers are free
+    }
+    if (!done) close_small<NP, false>(Dm, kl, k, Pr, s_mx, d);
+    {
+        uint32_t cext[TW];
+#pragma unroll
+        for (int w = 0; w < TW; ++w)
+            cext[w] = (G.isext[TR * cg + 2 * w] ? 0xffffu : 0u) | (G.isext[TR * cg + 2 * w + 1] ? 0xffff0000u : 0u);
+#pragma unroll
+        for (int r = 0; r < TR; ++r) {
+            const int row = TR * rg + r;
+            uint32_t old[TW], ch = 0;
+            ld_words<TW>(Dm + row * NP + TR * cg, old);
+#pragma unroll
+            for (int w = 0; w < TW; ++w) {
+                ch |= d[r][w] ^ old[w];
+                if (G.isext[row]) dec |= ((d[r][w] ^ old[w]) & cext[w]) != 0;
             }
+            chg |= ch != 0;
         }
-        __syncthreads();
-        for (int idx = tid; idx < mk * kWarps; idx += kThreads) {  // update classes per warp row group
-            const int a = idx / kWarps, w = idx % kWarps;
-            uint32_t mn = 0xffffu, mx = 0;
-#pragma unroll
-            for (int rr = 0; rr < RW; ++rr) {
-                const uint32_t v = Pm[a * NP + w * RW + rr];
-                mn = min(mn, v);
-                mx = max(mx, v);
-            }
-            cls[idx] = mn >= INF ? 0 : (mx <= INF_HEADROOM ? 1 : 2);
-        }
-        __syncthreads();
-        // D = min(D, P^T (x) P): warp w rows RW*w.., lane CP pairs
-        uint32_t acc[RW][CP];
-#pragma unroll
-        for (int rr = 0; rr < RW; ++rr)
-#pragma unroll
-            for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = INF2;
-        for (int kk = 0; kk < mk; ++kk) {
-            const int c = cls[kk * kWarps + warp];
-            if (c == 0) continue;  // uniform over the warp
-            uint32_t bv[CP];
-#pragma unroll
-            for (int cc = 0; cc < CP; ++cc) bv[cc] = reinterpret_cast<const uint32_t*>(Pm + kk * NP + lane * 2 * CP)[cc];
-            uint32_t av[RW];
-#pragma unroll
-            for (int q2 = 0; q2 < RW / 2; ++q2) {
-                const uint32_t w2 = reinterpret_cast<const uint32_t*>(Pm + kk * NP + warp * RW)[q2];
-                av[2 * q2] = splat(w2);
-                av[2 * q2 + 1] = splat(w2 >> 16);
-            }
-            if (c == 1) {
-#pragma unroll
-                for (int rr = 0; rr < RW; ++rr)
-#pragma unroll
-                    for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = acc_fast(acc[rr][cc], bv[cc], av[rr]);
-            } else {
-#pragma unroll
-                for (int rr = 0; rr < RW; ++rr) {
-                    const uint32_t tt = INF2 - av[rr];
-#pragma unroll
-                    for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = acc_clamp(acc[rr][cc], bv[cc], av[rr], tt);
-                }
-            }
-        }
-        const int col = lane * 2 * CP;
-        uint32_t cext[CP];
-#pragma unroll
-        for (int cc = 0; cc < CP; ++cc)
-            cext[cc] = (G.isext[col + 2 * cc] ? 0xffffu : 0u) | (G.isext[col + 2 * cc + 1] ? 0xffff0000u : 0u);
-#pragma unroll
-        for (int rr = 0; rr < RW; ++rr) {
-            const int row = warp * RW + rr;
-            uint32_t* dp = reinterpret_cast<uint32_t*>(Dm + row * NP + col);
-            const bool rext = G.isext[row] != 0;
-#pragma unroll
-            for (int cc = 0; cc < CP; ++cc) {
-                const uint32_t o = dp[cc], nv = min2(acc[rr][cc], o);
-                const uint32_t diff = nv ^ o;
-                if (diff) {
-                    dp[cc] = nv;
-                    chg = true;
-                    if (rext) dec |= (diff & cext[cc]) != 0;
-                }
-            }
-        }
-        __syncthreads();
     }
     if (__any_sync(FULL, chg) && lane == 0) s_chg = 1;
     if (__any_sync(FULL, dec) && lane == 0) s_dec = 1;
     __syncthreads();
     if (s_chg)
-        for (int idx = tid; idx < NP * NP / 8; idx += kThreads)
-            reinterpret_cast<uint4*>(Dg)[idx] = reinterpret_cast<const uint4*>(Dm)[idx];
+#pragma unroll
+        for (int r = 0; r < TR; ++r) st_words<TW>(Dg + (TR * rg + r) * NP + TR * cg, d[r]);
     if (tid == 0) {
         T.lv[l].kcnt[e.y] = k;
         if (s_dec) mark_dec(L, l, e.x, e.y);
@@ -1079,17 +1044,18 @@ __device__ void small_unit(const OpenLaunch& L, int l, int s, unsigned char* sme
 __device__ void small_phase(const OpenLaunch& L, int l, int N, int* s_unit, unsigned char* smem) {
     const int NP = L.geo[l].NP;
     for (int s = next_unit(L, s_unit); s < N; s = next_unit(L, s_unit)) {
-        if (NP == 128) small_unit<16, 2>(L, l, s, smem);
-        else small_unit<8, 1>(L, l, s, smem);
+        if (NP == 128) small_unit<128>(L, l, s, smem);
+        else small_unit<64>(L, l, s, smem);
     }
 }
 
-constexpr size_t kPanelSmem = (size_t)3 * B * kTLD * sizeof(uint16_t) + (size_t)B * 64 * sizeof(uint16_t) +
-                              B * sizeof(int) + (size_t)B * kWarps;
+constexpr size_t kPanelSmem = sizeof(PanelSmem);
 constexpr size_t kUpdateSmem = (size_t)B * 128 * (sizeof(uint32_t) + sizeof(uint16_t)) + (size_t)B * kWarps +
                                (size_t)128 * 128 * sizeof(uint16_t);
 constexpr size_t kTransposeSmem = (size_t)128 * (128 + 8) * sizeof(uint16_t);
-constexpr size_t kOpenSmem = std::max(std::max(kPanelSmem, (size_t)kInsertSmem), std::max(kUpdateSmem, kTransposeSmem));
+constexpr size_t kSmallSmem = (size_t)128 * 128 * 2 + 2 * 128 * 2 + 128 * 5;
+constexpr size_t kOpenSmem =
+    std::max({kPanelSmem, (size_t)kInsertSmem, kUpdateSmem, kTransposeSmem, kSmallSmem});
 
 // SM-aware order of the CTAs, for the units a CTA takes without a ticket:
 // the first CTA to start on each SM gets places 0 .. S - 1 (S SMs), the
