@@ -198,6 +198,26 @@ struct CoopChain {
 };
 CoopChain g_coop[kCoopMaxDevices];
 
+// A second stream for a launch that runs beside another one, and the events
+// that put it between that stream's neighbours.
+struct SideStream {
+    cudaStream_t st = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    void reserve(bool want) {
+        if (!want || join) return;
+        if (!st) ck(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream");
+        if (!fork) ck(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "event");
+        ck(cudaEventCreateWithFlags(&join, cudaEventDisableTiming), "event");
+    }
+    void release() {
+        if (st) cudaStreamDestroy(st);
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+        st = nullptr;
+        fork = join = nullptr;
+    }
+};
+
 template <class F>
 void coop_launch(int device, cudaStream_t st, F&& launch, const char* what) {
     CoopChain& c = g_coop[std::clamp(device, 0, kCoopMaxDevices - 1)];
@@ -286,6 +306,7 @@ struct UpdateArena {
     HostBuf nstage;
     PoolBuf<unsigned char> nlist, nscratch;
     int open_grid = 0;             // CTAs of the persistent opening kernel
+    SideStream side;               // openings of indexes of several (b, g), side by side
     // phase time stamps of the last device-driven opening launch (device,
     // and where they are in the arena)
     size_t trace_off = 0;
@@ -300,6 +321,7 @@ struct UpdateArena {
         nstage.release();
         nlist.release();
         nscratch.release();
+        side.release();
         if (ev_cnt) cudaEventDestroy(ev_cnt);
         ev_cnt = nullptr;
         trace_valid = 0;
@@ -1310,7 +1332,7 @@ bool open_on_device() {
 
 // Device-driven openings of any number of tasks (distinct indexes of one
 // device): tasks of equal (b, g) share one launch of the persistent opening
-// kernel (open.cu).  Per launch the host uploads, in one copy, the task
+// kernel (open.cu).  The host uploads, in one copy, every launch's task
 // descriptors, every level's work list (level 0: the touched leaves with
 // their opened edges; levels >= 1: the nodes with new seams, with room for
 // the parents the device appends) and the edge / seam triples; the kernel
@@ -1326,10 +1348,14 @@ void run_open_device(std::vector<OpenTask*>& tasks, UpdateArena& A, cudaStream_t
         size_t o_tasks = 0, o_out = 0, o_words = 0, o_trace = 0, o_slots[hb::kOpenMaxLevels] = {}, o_trip = 0;
         size_t o_dchild[hb::kOpenMaxLevels] = {}, o_rec[hb::kOpenMaxLevels] = {}, o_sm = 0;
         size_t begin = 0, end = 0;
+        size_t panel_elems = 1, pflag_bytes = 1;
         int n_trip = 0;
+        int64_t tiles = 0, most = 0;  // 128 x 128 tiles of the listed matrices: of all levels, of one at most
+        int grid = 0;                 // CTAs (0: all)
+        bool side = false;            // runs beside the launch before it
     };
     std::vector<GL> gl;
-    size_t off = 0, panel_elems = 1, pflag_bytes = 1;
+    size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t o = off;
         off += align256(std::max<size_t>(bytes, 1));
@@ -1374,8 +1400,11 @@ void run_open_device(std::vector<OpenTask*>& tasks, UpdateArena& A, cudaStream_t
             int np = 64;
             for (OpenTask* T : g.ts)
                 if (T->h->H >= l) np = T->h->L[l].NP;
-            panel_elems = std::max(panel_elems, (size_t)g.cap[l] * hb::kOpenB * np);
-            pflag_bytes = std::max(pflag_bytes, (size_t)g.cap[l] * (np / 64));
+            const int64_t tiles = (int64_t)g.cap[l] * ((np + 127) / 128) * ((np + 127) / 128);
+            g.tiles += tiles;
+            g.most = std::max(g.most, tiles);
+            g.panel_elems = std::max(g.panel_elems, (size_t)g.cap[l] * hb::kOpenB * np);
+            g.pflag_bytes = std::max(g.pflag_bytes, (size_t)g.cap[l] * (np / 64));
         }
         g.begin = off;
         g.o_tasks = take(g.ts.size() * sizeof(hb::OpenTask));
@@ -1393,14 +1422,42 @@ void run_open_device(std::vector<OpenTask*>& tasks, UpdateArena& A, cudaStream_t
     A.dev.reserve(off, st);
     A.stage.reserve(off);
     A.rb.reserve(off);
+    if (!A.open_grid) A.open_grid = hb::open_grid_blocks(device);
+    // An opening's phases are mostly latencies (a CTA has a few tiles in a phase),
+    // so two launches run side by side, each on CTAs in the ratio of its tiles but
+    // on an eighth of them at least; all CTAs are resident together, and no launch
+    // waits for another.  One after the other -> side by side, an opening of the
+    // batch: 6 maps of 256 with b = 8 and 6 with b = 16, 16 cells each, 540 -> 378 us,
+    // 384 cells 2041 -> 1664; 16 of 256 and one of 64, 384 cells 2280 -> 2218.
+    // Not where one launch has above 64 tiles for a CTA and keeps the GPU busy by
+    // itself (8 maps of 1024 and one of 64 on half of it each: 2253 -> 2703).
+    bool two = false;
+    for (size_t i = 1; i < gl.size(); ++i) {
+        GL &x = gl[i - 1], &y = gl[i];
+        if (x.side || A.open_grid < 8 || std::max(x.most, y.most) > 64 * (int64_t)A.open_grid)
+            continue;
+        const int low = A.open_grid / 8;
+        y.grid = std::clamp((int)(A.open_grid * (double)y.tiles / (double)std::max<int64_t>(1, x.tiles + y.tiles)), low,
+                            A.open_grid - low);
+        x.grid = A.open_grid - y.grid;
+        y.side = two = true;
+    }
+    A.side.reserve(two);
     // two panel and flag buffers: a round's panel is made while the update
     // of the round before reads the other one
-    panel_elems = (panel_elems + 127) / 128 * 128;
-    pflag_bytes = (pflag_bytes + 255) / 256 * 256;
-    A.panel.reserve(2 * panel_elems, st);
-    A.pflags.reserve(2 * pflag_bytes, st);
-    if (!A.open_grid) A.open_grid = hb::open_grid_blocks(device);
+    // (a second pair of buffers for the launch that runs beside the first one)
+    size_t panel_elems[2] = {0, 0}, pflag_bytes[2] = {0, 0};
+    for (size_t i = 0; i < gl.size(); ++i) {
+        GL& g = gl[i];
+        g.panel_elems = (g.panel_elems + 127) / 128 * 128;
+        g.pflag_bytes = (g.pflag_bytes + 255) / 256 * 256;
+        panel_elems[g.side] = std::max(panel_elems[g.side], 2 * g.panel_elems);
+        pflag_bytes[g.side] = std::max(pflag_bytes[g.side], 2 * g.pflag_bytes);
+    }
+    A.panel.reserve(panel_elems[0] + panel_elems[1], st);
+    A.pflags.reserve(pflag_bytes[0] + pflag_bytes[1], st);
     unsigned char* base = A.dev.p;
+    std::vector<hb::OpenLaunch> launches;
     for (GL& g : gl) {
         unsigned char* hs = A.stage.p;
         std::memset(hs + g.begin, 0, g.end - g.begin);
@@ -1489,19 +1546,34 @@ void run_open_device(std::vector<OpenTask*>& tasks, UpdateArena& A, cudaStream_t
         OL.bar = reinterpret_cast<unsigned*>(OL.status + 1);
         OL.sm = reinterpret_cast<unsigned*>(base + g.o_sm);
         OL.triples = reinterpret_cast<const int*>(base + g.o_trip);
-        OL.panel = A.panel.p;
-        OL.pflags = A.pflags.p;
+        OL.panel = A.panel.p + (g.side ? panel_elems[0] : 0);
+        OL.pflags = A.pflags.p + (g.side ? pflag_bytes[0] : 0);
         OL.trace = reinterpret_cast<unsigned long long*>(base + g.o_trace);
-        OL.panel_stride = panel_elems;
-        OL.pflag_stride = pflag_bytes;
-        ck(cudaMemcpyAsync(base + g.begin, hs + g.begin, g.end - g.begin, cudaMemcpyHostToDevice, st), "open upload");
-        coop_launch(device, st, [&] { return hb::launch_open(OL, A.open_grid, st); }, "opening kernel");
-        // statistics and the status word back (the trace stays on the device)
-        ck(cudaMemcpyAsync(A.rb.p + g.o_out, base + g.o_out, g.o_trace - g.o_out, cudaMemcpyDeviceToHost, st),
-           "open results");
+        OL.panel_stride = g.panel_elems;
+        OL.pflag_stride = g.pflag_bytes;
+        launches.push_back(OL);
         A.trace_off = g.o_trace;
         A.trace_valid = 1;
     }
+    ck(cudaMemcpyAsync(base, A.stage.p, off, cudaMemcpyHostToDevice, st), "open upload");
+    for (size_t i = 0; i < gl.size(); ++i) {
+        const bool beside = i + 1 < gl.size() && gl[i + 1].side;
+        coop_launch(device, st, [&] {
+            if (!beside) return hb::launch_open(launches[i], A.open_grid, st);
+            cudaError_t e = cudaEventRecord(A.side.fork, st);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(A.side.st, A.side.fork, 0);
+            if (e == cudaSuccess) e = hb::launch_open(launches[i + 1], gl[i + 1].grid, A.side.st);
+            if (e != cudaSuccess) return e;
+            e = hb::launch_open(launches[i], gl[i].grid, st);
+            const cudaError_t r = cudaEventRecord(A.side.join, A.side.st);
+            const cudaError_t w = cudaStreamWaitEvent(st, A.side.join, 0);
+            return e != cudaSuccess ? e : r != cudaSuccess ? r : w;
+        }, "opening kernel");
+        i += beside;
+    }
+    for (const GL& g : gl)  // statistics and the status word back (the trace stays on the device)
+        ck(cudaMemcpyAsync(A.rb.p + g.o_out, base + g.o_out, g.o_trace - g.o_out, cudaMemcpyDeviceToHost, st),
+           "open results");
     ck(cudaStreamSynchronize(st), "opening");
     for (GL& g : gl) {
         const int* words = reinterpret_cast<const int*>(A.rb.p + g.o_words);

@@ -61,3 +61,33 @@ def test_openings_match_the_oracle(gpu, kind, rows, cols, b, g, steps):
         for lvl in range(1, dev.H + 1):
             for n in range(dev.level_dims(lvl)[3]):
                 assert np.array_equal(dev.node_DU(lvl, n), cpu.node_DU(lvl, n)), f"level {lvl} node {n}"
+
+
+@pytest.mark.parametrize("maps", [
+    ((64, 8, 2), (64, 16, 2)),
+    ((32, 4, 2), (200, 8, 2), (60, 5, 3)),                # the third launch runs by itself
+    ((32, 8, 2), (256, 16, 2), (48, 16, 2), (48, 4, 2), (32, 8, 2)),
+])
+def test_launches_side_by_side(gpu, maps):
+    """One opening over indexes of several (b, g): their launches share the GPU."""
+    from htrip_b200.minplus_oracle import Batch, HierarchyConfig, MinPlusOracle
+    batch, runs = Batch(), []
+    for i, (side, b, g) in enumerate(maps):
+        observed, cells = W.withheld_open(make_grid("noise", side, side, i), 60, i)
+        dev, cpu = MinPlusOracle(HierarchyConfig(b, g, g)), PortOracle(b, g)
+        assert dev.build(observed) and cpu.build(observed)
+        runs.append((dev, cpu, observed, cells))
+    for at, m in ((0, 3), (3, 57)):
+        parts = [cells[at:at + m] for _, _, _, cells in runs]
+        for (dev, cpu, observed, _), part in zip(runs, parts):
+            observed[part[:, 0], part[:, 1]] = FREE
+        batch.open([(dev, part, observed) for (dev, _, observed, _), part in zip(runs, parts)])
+        for (dev, cpu, observed, _), part in zip(runs, parts):
+            cpu.open_batch(part, observed)
+            st = dev.last_batch_stats
+            assert (st.n_touched_leaves, st.n_dirty_ancestors, st.n_pivots) == cpu.stats()
+            for i in range(dev.num_leaf_tiles_x ** 2):
+                assert np.array_equal(dev.leaf_D(i), cpu.leaf_D(i)), f"leaf {i}"
+            for lvl in range(1, dev.H + 1):
+                for n in range(dev.level_dims(lvl)[3]):
+                    assert np.array_equal(dev.node_DU(lvl, n), cpu.node_DU(lvl, n)), f"level {lvl} node {n}"
