@@ -168,7 +168,7 @@ struct Level {
     int nseams = 0;
     int cap_inc = 0;  // most seam candidates that touch one child
     // device-side tables and state (pieces of htrip_index::arena)
-    Span<int> d_ext, d_seams, d_ext_inv;
+    Span<int> d_ext, d_seams, d_cols;
     Span<uint16_t> mat;
     Span<uint8_t> kflag;
     Span<int> klist, kcnt;
@@ -562,7 +562,7 @@ void alloc_levels(htrip_index* h) {
     for (auto& Lv : h->L) {
         take(Lv.d_ext, std::max(1, Lv.nExt));
         take(Lv.d_seams, Lv.seams.size());
-        take(Lv.d_ext_inv, Lv.NP);
+        take(Lv.d_cols, Lv.NP);
         take(Lv.d_isext, Lv.NP);
     }
     const size_t tables = off;
@@ -589,18 +589,22 @@ void alloc_levels(htrip_index* h) {
     for (auto& Lv : h->L) {
         auto* ext = reinterpret_cast<int*>(host.data() + reinterpret_cast<size_t>(Lv.d_ext.p));
         auto* seams = reinterpret_cast<int*>(host.data() + reinterpret_cast<size_t>(Lv.d_seams.p));
-        auto* inv = reinterpret_cast<int*>(host.data() + reinterpret_cast<size_t>(Lv.d_ext_inv.p));
+        auto* cols = reinterpret_cast<int*>(host.data() + reinterpret_cast<size_t>(Lv.d_cols.p));
         auto* isext = host.data() + reinterpret_cast<size_t>(Lv.d_isext.p);
         std::copy(Lv.ext.begin(), Lv.ext.end(), ext);
         std::copy(Lv.seams.begin(), Lv.seams.end(), seams);
-        std::fill(inv, inv + Lv.NP, -1);
+        std::fill(cols, cols + Lv.NP, -2);  // QueryLevel::cols
         for (int e = 0; e < Lv.nExt; ++e) {
-            inv[Lv.ext[e]] = e;
+            cols[Lv.ext[e]] = 2 * e;
             isext[Lv.ext[e]] = 1;
+        }
+        for (int i = 0; i < Lv.nseams; ++i) {
+            cols[Lv.seams[6 * i]] |= 1;
+            cols[Lv.seams[6 * i + 1]] |= 1;
         }
         place(Lv.d_ext);
         place(Lv.d_seams);
-        place(Lv.d_ext_inv);
+        place(Lv.d_cols);
         place(Lv.d_isext);
         place(Lv.kflag);
         place(Lv.dec);
@@ -2040,7 +2044,7 @@ hb::QueryParams make_params(const htrip_index* h, const QueryPlan& P, unsigned c
         q.D = Lv.mat.p;
         q.NP = Lv.NP;
         q.nP = Lv.nP;
-        q.ext_inv = Lv.d_ext_inv.p;
+        q.cols = Lv.d_cols.p;
         q.groups = plan + PL.o_groups;
         q.flags = flags + PL.flags_off;
         q.items = plan + PL.o_items;
@@ -2491,7 +2495,7 @@ int run_devplan(htrip_index* h, int k, int cfg, const int32_t* vps_host, const u
         T.lv[l].D = Lv.mat.p;
         T.lv[l].NP = Lv.NP;
         T.lv[l].nP = Lv.nP;
-        T.lv[l].ext_inv = Lv.d_ext_inv.p;
+        T.lv[l].cols = Lv.d_cols.p;
         T.lv[l].store_y = 1;
         T.lv[l].split = l == h->H ? D.root_split : 1;
         if (T.lv[l].split > 1) {

@@ -250,7 +250,7 @@ int query_default_config(int NP, int max_group);
 struct QueryLevel {
     const uint16_t* D;      // level matrices (NP x NP each)
     int NP, nP;
-    const int* ext_inv;     // column -> exterior port index or -1 (NP)
+    const int* cols;        // per column (NP) 2 x (its exterior port index or -1) + (it lies on a seam)
     const int* groups;      // 5 ints per child group {node, quad, slot0, cnt, sorted0}
     uint8_t* flags;         // [group][nP] finite-port flags of X_{l-1}
     const int* items;       // project items {group, m0, n0}

@@ -248,7 +248,7 @@ plan_query_kernel(const int32_t* __restrict__ vps, const uint8_t* __restrict__ p
             lv.D = tmpl.lv[l].D;
             lv.NP = tmpl.lv[l].NP;
             lv.nP = tmpl.lv[l].nP;
-            lv.ext_inv = tmpl.lv[l].ext_inv;
+            lv.cols = tmpl.lv[l].cols;
             lv.store_y = tmpl.lv[l].store_y;
             lv.part = tmpl.lv[l].part;
             lv.ticket = tmpl.lv[l].ticket;

@@ -39,6 +39,14 @@
 //            X_l = X_{l-1} (x) child_to_ext (:1113-1154); the epilogue writes
 //            them straight into X_l (level-(l+1) slot order) with the next
 //            level's flags.
+//            Only ports on a seam (about half of a child's) are rows: a path that
+//            leaves the child crosses a seam, and one that stays inside it is
+//            X_{l-1} itself, which the epilogue takes for the child's own
+//            columns and the level below for its pairs.  At the root only
+//            seam columns are read, so tiles without one are left out.  The same
+//            holds in the chain and in meet.  Whole calls, all ports / seam ports:
+//            512 x 512 maze k = 256 199 -> 154 us, the same with corridors of 16 and
+//            k = 64 139 -> 103, 1000 x 1013 street map k = 509 666 -> 523.
 //   meet     M[i][j] = min(M[i][j], min_p Yt_l[q_j*nP + p][i] (+) X_{l-1}[p][j])
 //            for i < j in one node: the inter-child meets (:1157-1326) and the
 //            intra-child shortcut (:1328-1411) are one formula.  Split-K items
@@ -223,9 +231,11 @@ __device__ __forceinline__ void count_work(unsigned long long* work, int n, int 
     atomicAdd(work + 2, (unsigned long long)skipped);
 }
 
-// Compacts the set flags of rows [kb, ke) into kl (ascending); returns the
+// Compacts the rows [kb, ke) of a child whose flag is set and that lie on a seam
+// (`cols`: the child's part of QueryLevel::cols) into kl (ascending); returns the
 // count (block-wide scan; every thread gets the total).
-__device__ __forceinline__ int compact_flags(const uint8_t* __restrict__ flags, int kb, int ke, int* kl, int* wsum) {
+__device__ __forceinline__ int compact_flags(const uint8_t* __restrict__ flags, const int* __restrict__ cols, int kb,
+                                             int ke, int* kl, int* wsum) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = ke - kb;
     const int per = (n + kThreads - 1) / kThreads;  // <= 16: kMaxList flags
@@ -234,7 +244,7 @@ __device__ __forceinline__ int compact_flags(const uint8_t* __restrict__ flags, 
     uint32_t mask = 0;
 #pragma unroll 4
     for (int j = 0; j < per; ++j)
-        if (p0 + j < p1) mask |= (uint32_t)(__ldcg(flags + p0 + j) != 0) << j;
+        if (p0 + j < p1) mask |= (uint32_t)((__ldcg(flags + p0 + j) != 0) & __ldg(cols + p0 + j)) << j;
     const int cntl = __popc(mask);
     int incl = cntl;
 #pragma unroll
@@ -412,11 +422,13 @@ struct ChainLevel {
     uint16_t *X, *Y;     // the level's columns in the viewpoint's slots
     uint8_t* flags;      // finite-port flags of the viewpoint's group of this level
     int NP, nP;
+    int q0;              // the child's first column
 };
 struct ChainSmem {
-    int16_t ext[2 * kMaxChainNP];       // per level, column -> exterior port or -1 (NP entries each)
-    int2 list[256];                     // finite ports of the child: {row offset, value in both halves}
+    int16_t ext[2 * kMaxChainNP];       // per level, the column words (NP entries each, QueryLevel::cols)
+    int2 list[256];                     // finite seam ports of the child: {row offset, value in both halves}
     uint16_t x[kMaxChainNP];            // port distances of the level below
+    uint16_t own[256];                  // the same, kept while x is overwritten
     uint16_t red[8 * kThreads];         // partial rows of the row groups
     uint8_t chunk[kMaxChainNP / 8];     // the 8-column chunks of the level to compute
     ChainLevel lv[kMaxChain + 1];
@@ -443,8 +455,8 @@ __device__ __forceinline__ void do_chain(const QueryParams& P, int v, ChainSmem&
         for (int l = 1; l <= top; ++l) {
             const int n = P.lv[l].NP / 8, c = (tid + kThreads - (o / 8) % kThreads) % kThreads;
             if (c < n) {
-                const int4 a = reinterpret_cast<const int4*>(P.lv[l].ext_inv)[2 * c];
-                const int4 b = reinterpret_cast<const int4*>(P.lv[l].ext_inv)[2 * c + 1];
+                const int4 a = reinterpret_cast<const int4*>(P.lv[l].cols)[2 * c];
+                const int4 b = reinterpret_cast<const int4*>(P.lv[l].cols)[2 * c + 1];
                 *reinterpret_cast<uint4*>(S.ext + o + 8 * c) =
                     make_uint4((a.x & 0xffff) | (a.y << 16), (a.z & 0xffff) | (a.w << 16), (b.x & 0xffff) | (b.y << 16),
                                (b.z & 0xffff) | (b.w << 16));
@@ -470,6 +482,7 @@ __device__ __forceinline__ void do_chain(const QueryParams& P, int v, ChainSmem&
             c.flags = L.flags + (size_t)(tab[2 * lane + 1] >> 1) * L.nP;
             c.NP = L.NP;
             c.nP = L.nP;
+            c.q0 = q * L.nP;
             if (l <= top) asm volatile("prefetch.global.L2 [%0];" ::"l"(c.D));  // its page's translation
         }
         S.lv[lane] = c;
@@ -490,16 +503,18 @@ __device__ __forceinline__ void do_chain(const QueryParams& P, int v, ChainSmem&
         const ChainLevel L = S.lv[l - 1];
         const int NP = L.NP;
         const bool put_y = tab[2 * (l - 1) + 1] & 1;  // the level's meets read Y
-        // The finite ports (nP <= 256: one step) and the columns to compute, in
+        // The finite seam ports (nP <= 256: one step) and the columns to compute, in
         // chunks of 8: all where the level's meets read Y, else those with an exterior
         // port (about half).
         const uint32_t a0 = tid < L.nP ? S.x[tid] : INF;
         bool need = tid < NP / 8;
         if (need && !put_y) {
             const uint4 e = *reinterpret_cast<const uint4*>(ext + 8 * tid);
-            need = (e.x & e.y & e.z & e.w) != 0xffffffffu;
+            need = (~(e.x & e.y & e.z & e.w) & 0x80008000u) != 0;
         }
-        const unsigned bal = __ballot_sync(FULL, a0 < INF), cbal = __ballot_sync(FULL, need);
+        const bool row = a0 < INF && (ext[L.q0 + tid] & 1);
+        if (tid < L.nP) S.own[tid] = (uint16_t)a0;
+        const unsigned bal = __ballot_sync(FULL, row), cbal = __ballot_sync(FULL, need);
         if (lane == 0) {
             S.wcnt[warp] = __popc(bal);
             S.ccnt[warp] = __popc(cbal);
@@ -515,7 +530,7 @@ __device__ __forceinline__ void do_chain(const QueryParams& P, int v, ChainSmem&
             n += S.wcnt[w];
             G += S.ccnt[w];
         }
-        if (a0 < INF) S.list[at] = make_int2(tid * NP, (int)splat(a0));
+        if (row) S.list[at] = make_int2(tid * NP, (int)splat(a0));
         if (need) S.chunk[cat] = (uint8_t)tid;
         __syncthreads();
         // A thread takes one chunk of every nG-th listed row, 8 loads in flight.
@@ -560,8 +575,9 @@ __device__ __forceinline__ void do_chain(const QueryParams& P, int v, ChainSmem&
             for (int r = 0; r < nG; ++r) m = min2(m, *reinterpret_cast<const uint32_t*>(&S.red[8 * r * G + 2 * pw]));
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const uint16_t y = (uint16_t)(m >> (16 * h));
-                const int e = (int16_t)(e2 >> (16 * h));
+                const int p = c + h - L.q0, e = (int16_t)(e2 >> (16 * h)) >> 1;
+                uint16_t y = (uint16_t)(m >> (16 * h));
+                if ((unsigned)p < (unsigned)L.nP) y = min(y, S.own[p]);
                 if (put_y) L.Y[(size_t)(c + h) * ldv] = y;
                 if (l < H && e >= 0) {
                     S.x[e] = y;
@@ -594,7 +610,12 @@ __device__ bool do_project(const QueryParams& P, const QueryLevel& L, const Quer
         for (int r = 0; r < min(RW, G[3] - m0); ++r) any |= dirty_at(P.dirty, G[4] + m0 + r, l);
         if (!any) return L.split <= 1 || part == 0;  // a skipped item counts once
     }
-    const int nA = compact_flags(L.flags + (size_t)gi * L.nP, 0, L.nP, kl, wsum);
+    if (!Ln) {  // the root lifts nothing: only seam columns are read
+        int any = 0;
+        for (int c = n0 + threadIdx.x; c < min(n0 + 64 * CP, L.NP); c += kThreads) any |= __ldg(L.cols + c) & 1;
+        if (!__syncthreads_or(any)) return L.split <= 1 || part == 0;
+    }
+    const int nA = compact_flags(L.flags + (size_t)gi * L.nP, L.cols + q * L.nP, 0, L.nP, kl, wsum);
     const int kb = (int)((long)nA * part / L.split), ke = (int)((long)nA * (part + 1) / L.split);
     const uint16_t* D = L.D + (size_t)node * L.NP * L.NP + (size_t)q * L.nP * L.NP;
     const int col = n0 + lane * 2 * CP;
@@ -623,6 +644,18 @@ __device__ bool do_project(const QueryParams& P, const QueryLevel& L, const Quer
 #pragma unroll
         for (int r = 0; r < RW; ++r)
             v[r] = (uint16_t)((cc & 1) ? (acc[r][cc >> 1] >> 16) : (acc[r][cc >> 1] & 0xffffu));
+        const int own = col + cc - q * L.nP;  // a column of the child itself: reached without leaving it
+        if (do_lift && (unsigned)own < (unsigned)L.nP) {
+            const uint4* x = reinterpret_cast<const uint4*>(Xp + (size_t)own * P.ldv);
+#pragma unroll
+            for (int r8 = 0; r8 < RW / 8; ++r8) {
+                const uint4 o = __ldcg(x + r8);
+                const uint32_t w[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    v[8 * r8 + i] = min(v[8 * r8 + i], (uint16_t)(w[i >> 1] >> (16 * (i & 1))));
+            }
+        }
         if (do_y) {
             uint16_t* y = Y + (size_t)(col + cc) * P.ldv + slot0 + m0;
 #pragma unroll
@@ -671,7 +704,7 @@ __device__ void do_meet(const QueryParams& P, const QueryLevel& L, int item, int
         }
         if (!__syncthreads_or(any)) return;
     }
-    const int nA = compact_flags(L.flags + (size_t)g2 * L.nP, kb, ke, kl, wsum);
+    const int nA = compact_flags(L.flags + (size_t)g2 * L.nP, L.cols + coloff, kb, ke, kl, wsum);
     const uint16_t* Xp = P.X[l - 1] + j0;
     const uint16_t* Y = P.Y[l] + (size_t)coloff * P.ldv + i0;
     uint32_t acc[RW][CP];
@@ -718,7 +751,7 @@ __device__ void unit_prologue(const QueryParams& P, int t, int u, ItemMeta& im) 
         const int slot0 = G[2], cnt = G[3];
         for (int e = tid; e < 64 * CP + RW; e += kThreads) {
             if (e < 64 * CP) {
-                im.col[e] = n0 + e < L.NP ? L.ext_inv[n0 + e] : -1;
+                im.col[e] = n0 + e < L.NP ? L.cols[n0 + e] >> 1 : -1;
             } else {
                 const int r = e - 64 * CP;
                 const bool ok = m0 + r < cnt;

@@ -53,3 +53,29 @@ def test_queries_match_the_oracle(gpu, kind, rows, cols, b, g, ks):
         observed[cells[:, 0], cells[:, 1]] = W.FREE
         dev.onBatchCellsOpened(cells, observed)
         cpu.open_batch(cells, observed)
+
+
+@pytest.mark.parametrize("rows,cols,b,g,k", [(64, 64, 8, 2, 300), (60, 57, 5, 3, 200), (64, 64, 4, 4, 500),
+                                             (200, 200, 16, 2, 700)])
+def test_seam_rows(gpu, rows, cols, b, g, k):
+    """Winding corridors: the shortest way between two ports of a child runs inside it
+    for some and outside for others.  Full and incremental queries, after openings."""
+    from htrip_b200.minplus_oracle import HierarchyConfig, IncrementalState, MinPlusOracle
+    truth = np.full((rows, cols), W.FREE, np.uint8)
+    truth[1::2] = W.OBSTACLE
+    for i in range(1, rows, 2):
+        truth[i, cols - 1 if (i // 2) % 2 == 0 else 0] = W.FREE
+        truth[i, (7 * i) % cols] = W.FREE
+    observed, cells = W.withheld_open(truth, 30, 5)
+    dev, cpu = MinPlusOracle(HierarchyConfig(b, g, g)), PortOracle(b, g)
+    assert dev.build(observed) and cpu.build(observed)
+    vps, state = W.sample_free(observed, k, 3), IncrementalState()
+    for part in (cells[:0], cells[:1], cells[1:]):
+        if len(part):
+            observed[part[:, 0], part[:, 1]] = W.FREE
+            dev.onBatchCellsOpened(part, observed)
+            cpu.open_batch(part, observed)
+        want = port_bfs(observed, vps)
+        assert np.array_equal(cpu.query(vps, observed), want)
+        assert np.array_equal(dev.queryAllPairs(vps, observed), want)
+        assert np.array_equal(dev.queryAllPairsIncremental(vps, observed, state), want)
