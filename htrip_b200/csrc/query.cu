@@ -231,15 +231,14 @@ __device__ __forceinline__ void count_work(unsigned long long* work, int n, int 
     atomicAdd(work + 2, (unsigned long long)skipped);
 }
 
-// Compacts the rows [kb, ke) of a child whose flag is set and that lie on a seam
+// Compacts the rows of a child (n ports) whose flag is set and that lie on a seam
 // (`cols`: the child's part of QueryLevel::cols) into kl (ascending); returns the
 // count (block-wide scan; every thread gets the total).
-__device__ __forceinline__ int compact_flags(const uint8_t* __restrict__ flags, const int* __restrict__ cols, int kb,
-                                             int ke, int* kl, int* wsum) {
+__device__ __forceinline__ int compact_flags(const uint8_t* __restrict__ flags, const int* __restrict__ cols, int n,
+                                             int* kl, int* wsum) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n = ke - kb;
     const int per = (n + kThreads - 1) / kThreads;  // <= 16: kMaxList flags
-    const int p0 = kb + tid * per, p1 = min(ke, p0 + per);
+    const int p0 = tid * per, p1 = min(n, p0 + per);
     // the thread's flags are read once, all loads in flight together
     uint32_t mask = 0;
 #pragma unroll 4
@@ -615,7 +614,7 @@ __device__ bool do_project(const QueryParams& P, const QueryLevel& L, const Quer
         for (int c = n0 + threadIdx.x; c < min(n0 + 64 * CP, L.NP); c += kThreads) any |= __ldg(L.cols + c) & 1;
         if (!__syncthreads_or(any)) return L.split <= 1 || part == 0;
     }
-    const int nA = compact_flags(L.flags + (size_t)gi * L.nP, L.cols + q * L.nP, 0, L.nP, kl, wsum);
+    const int nA = compact_flags(L.flags + (size_t)gi * L.nP, L.cols + q * L.nP, L.nP, kl, wsum);
     const int kb = (int)((long)nA * part / L.split), ke = (int)((long)nA * (part + 1) / L.split);
     const uint16_t* D = L.D + (size_t)node * L.NP * L.NP + (size_t)q * L.nP * L.NP;
     const int col = n0 + lane * 2 * CP;
@@ -704,7 +703,10 @@ __device__ void do_meet(const QueryParams& P, const QueryLevel& L, int item, int
         }
         if (!__syncthreads_or(any)) return;
     }
-    const int nA = compact_flags(L.flags + (size_t)g2 * L.nP, L.cols + coloff, kb, ke, kl, wsum);
+    // the item's share of the rows that count: seam ports lie side by side, so equal
+    // ranges of ports would be unequal work
+    const int nL = compact_flags(L.flags + (size_t)g2 * L.nP, L.cols + coloff, L.nP, kl, wsum);
+    const int k0 = (int)((long)nL * kb / L.nP), nA = (int)((long)nL * ke / L.nP) - k0;
     const uint16_t* Xp = P.X[l - 1] + j0;
     const uint16_t* Y = P.Y[l] + (size_t)coloff * P.ldv + i0;
     uint32_t acc[RW][CP];
@@ -712,7 +714,7 @@ __device__ void do_meet(const QueryParams& P, const QueryLevel& L, int item, int
     for (int r = 0; r < RW; ++r)
 #pragma unroll
         for (int c = 0; c < CP; ++c) acc[r][c] = INF2;
-    const int skipped = warp_minplus_list<RW, CP>(acc, kl, nA, warp, Xp, P.ldv, Y, P.ldv, P.ldv - i0,
+    const int skipped = warp_minplus_list<RW, CP>(acc, kl + k0, nA, warp, Xp, P.ldv, Y, P.ldv, P.ldv - i0,
                                                   red + warp * pipe_warp_words<RW, CP>());
     count_work<RW, CP>(P.work, nA, warp, skipped);
     cta_reduce<RW, CP>(acc, red);
