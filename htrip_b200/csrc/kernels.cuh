@@ -199,8 +199,8 @@ struct OpenLaunch {
     const int* triples;            // (u, v, w)
     uint16_t* panel;               // two buffers (rounds alternate) of, per slot, kOpenB x NP: the
                                    // round's closed pivot rows
-    uint8_t* pflags;               // two buffers of, per slot, NP / 64 flags: 64-column blocks of
-                                   // the panel holding a finite value
+    uint8_t* pflags;               // two buffers of, per slot, NP / 64 bytes, one for 64 columns of
+                                   // the panel: bit 0 a finite value, bit 1 one beyond the half range
     size_t panel_stride;           // elements between the two panel buffers
     size_t pflag_stride;           // bytes between the two flag buffers
     int* status;                   // 0 ok, 1 a bounded barrier wait timed out, 2 a list overflowed

@@ -19,7 +19,7 @@
 //   compact(l) pivot flags -> sorted pivot list per matrix.
 //   rounds     blocked pivot-set Kleene closure, kOpenB pivots per round:
 //              panel: every CTA of a column tile closes the round's pivot
-//                block T = D[K, K] itself (Floyd-Warshall in shared memory)
+//                block T = D[K, K] itself (16 pivots a step in shared memory)
 //                and computes P[:, tile] = T* (x) D[K, tile];
 //              update: D = min(D, P^T (x) P) over upper-triangle tiles, each
 //                also written transposed (D is symmetric), and only where an
