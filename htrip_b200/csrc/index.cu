@@ -2256,14 +2256,14 @@ struct DevPlanLayout {
 // shared-memory sort, Morton codes below 2^52 (they carry the viewpoint index
 // in the low 12 bits), and the query kernel's depth and port limits.  It
 // does, by default, when the viewpoints are already on the device (the host
-// would otherwise wait for their copy), and from kDevPlanHostK viewpoints on when
-// they come from the host: the host's planning grows with k, the device's costs
-// about 20 us whatever k is.  Whole calls, host / device planned: 256 x 256 street map
-// k = 48 104 / 114 us, 64 109 / 110, 128 137 / 129, 512 267 / 220; 512 x 512 maze
-// k = 48 128 / 131, 64 142 / 139, 128 175 / 156, 512 423 / 316.
+// would otherwise wait for their copy).  Viewpoints from the host are planned
+// there although the device is faster from about k = 64 on (whole calls, host /
+// device planned: 512 x 512 maze k = 128 175 / 156 us): the device's arena is sized for
+// the worst case of k (all levels at the slots of the fullest one: 0.1 GB at
+// 512 x 512, b = 16, k = 256), which for hundreds of served indexes took the memory
+// of the indexes themselves and had them evicted.
 // HTRIP_QUERY_PLANNER=host plans every query on the host, =device every
 // query it can on the device.
-constexpr int kDevPlanHostK = 64;
 bool devplan_supported(const htrip_index* h, int k, bool host_inputs) {
     if (k < 1 || k > hb::plan_max_k() || h->H > hb::kMaxQueryLevels) return false;
     static const int mode = [] {
@@ -2272,7 +2272,7 @@ bool devplan_supported(const htrip_index* h, int k, bool host_inputs) {
         if (e && std::strcmp(e, "device") == 0) return 2;
         return 0;
     }();
-    if (mode == 1 || (mode == 0 && host_inputs && k < kDevPlanHostK)) return false;
+    if (mode == 1 || (mode == 0 && host_inputs)) return false;
     double codes = 1;
     for (int l = 0; l < std::max(h->H, 1); ++l) codes *= (double)h->g * h->g;
     if (codes >= 4503599627370496.0) return false;  // 2^52
