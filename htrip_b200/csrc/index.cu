@@ -362,6 +362,7 @@ struct htrip_index {
     int S = 0, H = 0, rows = 0, cols = 0, leaves_x = 0;
     std::vector<Level> L;
     DevBuf<unsigned char> arena;  // every level's tables, state and matrices
+    size_t state_off = 0, state_bytes = 0;  // the arena's per-node state, zero outside an opening call
     DevBuf<uint8_t> pass;
     // scratch of the index's own build / opening launches
     UpdateArena u;
@@ -548,6 +549,12 @@ std::vector<int> weighted_leaves(const htrip_index* h, const std::vector<int>& l
     return out;
 }
 
+// Pivot flags, decrease flags and stamps of every node start at zero.
+void clear_state(htrip_index* h) {
+    ck(cudaMemsetAsync(h->arena.p + h->state_off, 0, h->state_bytes, h->stream), "level state");
+    h->stamp_epoch++;
+}
+
 // One device allocation for all levels: the static tables (one upload), the
 // per-node state that starts at zero (one memset), the pivot lists, then the
 // matrices.  Separate allocations, nine per level, cost a small map's
@@ -615,11 +622,12 @@ void alloc_levels(htrip_index* h) {
         place(Lv.mat);
     }
     ck(cudaMemcpyAsync(base, host.data(), tables, cudaMemcpyHostToDevice, h->stream), "level tables");
-    ck(cudaMemsetAsync(base + tables, 0, zeros - tables, h->stream), "level state");
+    h->state_off = tables;
+    h->state_bytes = zeros - tables;
+    clear_state(h);
     for (auto& Lv : h->L)  // node builds write the logical part of a matrix only
         if (Lv.lvl >= 1) hb::launch_pad_fill(Lv.ms(), Lv.nnodes, h->stream);
     ck(cudaGetLastError(), "padding");
-    h->stamp_epoch++;
 }
 
 // Descriptor of matrix m of level Lv (an index's own level arrays).
@@ -861,6 +869,8 @@ void do_build(htrip_index* h, const uint8_t* observed, int rows, int cols) {
         make_levels(h);
         h->ref_bytes = reference_bytes(h);
         alloc_levels(h);
+    } else {
+        clear_state(h);  // an opening that failed may have left flags set
     }
     cudaStream_t st = h->stream;
     upload_passable(h, observed, rows, cols);
@@ -887,6 +897,7 @@ void do_lift_root(htrip_index* h, const uint8_t* observed, int rows, int cols) {
     ck(cudaStreamSynchronize(st), "sync");
     std::vector<Level> old = std::move(h->L);
     DevBuf<unsigned char> old_arena = h->arena;
+    const size_t old_state_off = h->state_off, old_state_bytes = h->state_bytes;
     h->L.clear();
     h->arena = DevBuf<unsigned char>();
     const int old_rows = h->rows, old_cols = h->cols;
@@ -911,6 +922,8 @@ void do_lift_root(htrip_index* h, const uint8_t* observed, int rows, int cols) {
     } catch (...) {
         h->arena.release();
         h->arena = old_arena;
+        h->state_off = old_state_off;
+        h->state_bytes = old_state_bytes;
         h->L = std::move(old);  // the old matrices are intact
         h->S = old_S;
         h->H = old_H;
@@ -3328,6 +3341,20 @@ htrip_status htrip_selftest_barrier_timeout(int device, int32_t* status, int32_t
 
 htrip_status htrip_selftest_wait_timeout(int device, int32_t* status, int32_t* ctas_returned, float* ms) {
     return timeout_selftest(1, device, status, ctas_returned, ms);
+}
+
+htrip_status htrip_selftest_stale_flags(htrip_index* h) {
+    if (!h) return fail(HTRIP_ERR_INVALID, "null handle");
+    if (const htrip_status rs = ready(h)) return rs;
+    HTRIP_GUARD_BEGIN
+    ck(cudaSetDevice(h->device), "cudaSetDevice");
+    for (const Level& Lv : h->L) {
+        ck(cudaMemsetAsync(Lv.kflag.p, 1, Lv.kflag.n, h->stream), "pivot flags");
+        ck(cudaMemsetAsync(Lv.dec.p, 1, Lv.dec.n, h->stream), "decrease flags");
+    }
+    ck(cudaStreamSynchronize(h->stream), "sync");
+    return HTRIP_OK;
+    HTRIP_GUARD_END
 }
 
 htrip_status htrip_measure_minplus_rate(int device, int variant, double* entries_per_s) {

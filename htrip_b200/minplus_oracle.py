@@ -91,7 +91,7 @@ EXPORTS = (
     "htrip_leaves_changed", "htrip_selftest_barrier_timeout", "htrip_selftest_wait_timeout", "htrip_set_cell_weights",
     "htrip_cell_weight_changed", "htrip_tile_weights_changed", "htrip_server_wait_version",
     "htrip_last_open_levels", "htrip_set_query_work_counting", "htrip_last_query_executed",
-    "htrip_last_open_trace",
+    "htrip_last_open_trace", "htrip_selftest_stale_flags",
 )
 
 
@@ -153,6 +153,7 @@ def load_library(path: str | None = None):
     lib.htrip_cell_blocked.argtypes = [P, I, I, _U8P, I, I]
     lib.htrip_selftest_barrier_timeout.argtypes = [C.c_int, _I32P, _I32P, C.POINTER(C.c_float)]
     lib.htrip_selftest_wait_timeout.argtypes = [C.c_int, _I32P, _I32P, C.POINTER(C.c_float)]
+    lib.htrip_selftest_stale_flags.argtypes = [P]
     lib.htrip_leaves_changed.argtypes = [P, _I32P, I, _U8P, I, I]
     lib.htrip_set_cell_weights.argtypes = [P, _U16P, I, I]
     lib.htrip_cell_weight_changed.argtypes = [P, I, I, C.c_uint16, _U8P, I, I]
@@ -726,6 +727,11 @@ def selftest_wait_timeout(device: int = 0):
     st, ret, ms = C.c_int32(), C.c_int32(), C.c_float()
     _check(lib.htrip_selftest_wait_timeout(device, C.byref(st), C.byref(ret), C.byref(ms)))
     return st.value, ret.value, ms.value
+
+
+def selftest_stale_flags(oracle: "MinPlusOracle"):
+    """Sets the index's pivot and decrease flags, as a failed opening may leave them."""
+    _check(oracle.lib.htrip_selftest_stale_flags(oracle.h))
 
 
 def minplus_rate(device: int = 0, variant: int = 0) -> float:

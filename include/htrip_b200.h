@@ -435,6 +435,10 @@ htrip_status htrip_selftest_barrier_timeout(int device, int32_t* status, int32_t
  * 4, *ms = the launch's duration.                                          */
 htrip_status htrip_selftest_wait_timeout(int device, int32_t* status, int32_t* ctas_returned, float* ms);
 
+/* Leaves the pivot and decrease flags of every matrix set, as an opening that
+ * ended with an error may: htrip_build on the same handle starts clean.    */
+htrip_status htrip_selftest_stale_flags(htrip_index* h);
+
 /* Wait for all work queued on the index's stream.                         */
 htrip_status htrip_sync(htrip_index* h);
 

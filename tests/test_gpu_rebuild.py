@@ -1,0 +1,34 @@
+"""A handle that is built again, and rebuilds in place: what earlier calls left
+behind (flags of a failed opening, a trace, scratch memory, weights, an
+incremental state) reaches no later result.  Matrices, statistics and distances
+against the CPU restatement of the reference, tolerance 0."""
+import pytest
+
+from helpers import FREE, make_grid
+from htrip_b200 import workloads as W
+from oracle.ref import PortOracle, port_available
+
+pytestmark = [pytest.mark.gpu,
+              pytest.mark.skipif(not port_available(), reason="oracle port not built (make -C oracle port)")]
+
+
+def _stats(dev):
+    st = dev.last_batch_stats
+    return st.n_touched_leaves, st.n_dirty_ancestors, st.n_pivots
+
+
+@pytest.mark.parametrize("kind,side,b,g", [("noise", 64, 16, 2), ("street", 100, 8, 2), ("noise", 54, 9, 3)])
+def test_build_on_a_handle_clears_flags_of_a_failed_opening(gpu, kind, side, b, g):
+    from htrip_b200.minplus_oracle import HierarchyConfig, MinPlusOracle, selftest_stale_flags
+    observed, cells = W.withheld_open(make_grid(kind, side, side, b), 30, 5)
+    dev, new, cpu = MinPlusOracle(HierarchyConfig(b, g, g)), MinPlusOracle(HierarchyConfig(b, g, g)), PortOracle(b, g)
+    assert dev.build(observed) and new.build(observed) and cpu.build(observed)
+    selftest_stale_flags(dev)
+    assert dev.build(observed)
+    observed[cells[:, 0], cells[:, 1]] = FREE
+    for o in (dev, new):
+        o.onBatchCellsOpened(cells, observed)
+    cpu.open_batch(cells, observed)
+    assert _stats(dev) == cpu.stats()
+    assert dev.lastOpenLevels() == new.lastOpenLevels()
+    assert dev.stateDigest() == new.stateDigest()
