@@ -1714,9 +1714,10 @@ int query_chain(const htrip_index* h, int k) {
 }
 
 // Plans a query; force_cfg >= 0 imposes the tile configuration (requests
-// that share a launch share one).
+// that share a launch share one); without `chain` no level is lifted viewpoint
+// by viewpoint.
 void make_plan(const htrip_index* h, const int32_t* vps, const uint8_t* pass_flags, int k, QueryPlan& P,
-               int force_cfg = -1) {
+               int force_cfg = -1, bool chain = true) {
     const int b = h->b, g = h->g, H = h->H;
     struct V { uint64_t key; int orig; int tx, ty; };
     std::vector<V> v;
@@ -1782,7 +1783,7 @@ void make_plan(const htrip_index* h, const int32_t* vps, const uint8_t* pass_fla
     P.cfg = force_cfg >= 0 ? force_cfg : choose_query_cfg(h, ns, H >= 1 ? P.lv[H].max_group : ns);
     const hb::QueryTile tile = hb::query_config_tile(P.cfg);
     const int RW = tile.RW, NC = tile.NCOL;
-    P.chain = query_chain(h, k);
+    P.chain = chain ? query_chain(h, k) : 0;
     // Slot layout: every child group's run starts on an RW boundary.
     std::vector<std::vector<int>> slot_of(H + 1);
     int max_slots = ns;
@@ -3034,7 +3035,13 @@ htrip_status htrip_query_all_pairs_noalloc(htrip_index* h, const int32_t* vps, i
     QueryPlan P;
     make_plan(h, vps, pf.data(), k, P);
     const std::vector<QueryReq> R{{h, &P, nullptr}};
-    const LaunchLayout L = layout_launch(R);
+    LaunchLayout L = layout_launch(R);
+    if (L.total > kNoAllocScratchBytes && P.chain > 0) {
+        // many viewpoints in few leaves: the chain's table (40 bytes a viewpoint) takes
+        // more than the project items of its levels would
+        make_plan(h, vps, pf.data(), k, P, -1, false);
+        L = layout_launch(R);
+    }
     if (L.total > kNoAllocScratchBytes)
         return fail(HTRIP_ERR_UNSUPPORTED, "query needs " + std::to_string(L.total) +
                                                " bytes of device scratch; the allocation-free entry point has " +
