@@ -1646,8 +1646,8 @@ struct QueryPlan {
     int ldv = 8;   // slot stride of X / Yt
     int ldm = 8;   // stride of the sorted-order M
     int cfg = 0;
-    int o_vp0 = 0, o_inv = 0, o_l0 = 0, n_l0 = 0;
-    int chain = 0, o_chain = 0;  // QueryParams::chain and its table
+    int o_vp0 = 0, o_inv = 0, o_low = 0, n_l0 = 0;
+    int chain = 0;  // QueryParams::chain
     struct Lvl {
         int o_groups = 0, n_groups = 0, max_group = 0, slots = 0;
         int o_items = 0, n_items = 0, split = 1;
@@ -1802,23 +1802,19 @@ void make_plan(const htrip_index* h, const int32_t* vps, const uint8_t* pass_fla
         P.flags_total += (size_t)Q.n_groups * h->L[l].nP;
     }
     P.ldv = (max_slots + 256 + 7) / 8 * 8;
-    // Level-0 table: per level-1 slot {sorted index or -1, level-1 group}.
-    P.o_l0 = (int)P.buf.size();
-    if (H >= 1) {
-        P.n_l0 = P.lv[1].slots;
+    // Table of the lowest levels (QueryParams::low).
+    P.o_low = (int)P.buf.size();
+    P.n_l0 = H >= 1 ? P.lv[1].slots : 0;
+    if (H >= 1 && P.chain == 0) {
         P.buf.resize(P.buf.size() + 2 * (size_t)P.n_l0, -1);
         for (int gi = 0; gi < (int)cgs[1].size(); ++gi)
             for (int t = 0; t < cgs[1][gi].cnt; ++t) {
-                P.buf[P.o_l0 + 2 * (cgs[1][gi].slot0 + t)] = cgs[1][gi].start + t;
-                P.buf[P.o_l0 + 2 * (cgs[1][gi].slot0 + t) + 1] = gi;
+                P.buf[P.o_low + 2 * (cgs[1][gi].slot0 + t)] = cgs[1][gi].start + t;
+                P.buf[P.o_low + 2 * (cgs[1][gi].slot0 + t) + 1] = gi;
             }
-    } else {
-        P.n_l0 = 0;
-    }
-    P.o_chain = (int)P.buf.size();
-    if (P.chain > 0) {
+    } else if (P.chain > 0) {
         P.buf.resize(P.buf.size() + (size_t)ns * hb::kChainInts, 0);
-        int* tab = P.buf.data() + P.o_chain;
+        int* tab = P.buf.data() + P.o_low;
         int gl = 1;  // leaves per level-l node side
         for (int l = 1; l <= std::min(P.chain + 1, H); ++l) {
             gl *= g;
@@ -2035,11 +2031,8 @@ hb::QueryParams make_params(const htrip_index* h, const QueryPlan& P, unsigned c
     Q.cfg = P.cfg;
     Q.vp0 = plan + P.o_vp0;
     Q.inv = plan + P.o_inv;
-    Q.l0 = plan + P.o_l0;
+    Q.low = plan + P.o_low;
     Q.chain = P.chain;
-    Q.g = h->g;
-    Q.leaves_x = h->leaves_x;
-    Q.chain_tab = plan + P.o_chain;
     Q.ext0 = h->L[0].d_ext.p;
     Q.leaves = h->L[0].ms();
     for (int l = 0; l < H; ++l) Q.X[l] = reinterpret_cast<uint16_t*>(base + L.X[i][l]);
@@ -2357,8 +2350,7 @@ DevPlanLayout devplan_layout(const htrip_index* h, int k, int cfg, bool out_in_a
     O.o_vp0 = take(4 * (size_t)k);
     O.o_inv = take(k);
     O.o_rec = take(hb::plan_record_ints());
-    O.o_chain = take(H >= 1 ? (size_t)hb::kChainInts * k : 0);
-    O.o_l0 = take(H >= 1 ? 2 * (size_t)O.cap_slots[1] : 0);
+    O.o_low = take(H < 1 ? 0 : G.chain > 0 ? (size_t)hb::kChainInts * k : 2 * (size_t)O.cap_slots[1]);
     for (int l = 1; l <= H; ++l) {
         O.o_groups[l] = take(5 * (size_t)O.cap_groups[l]);
         O.o_items[l] = take(3 * (size_t)O.cap_items[l]);

@@ -269,12 +269,12 @@ struct QueryLevel {
 // One queryAllPairs request of a launch.
 struct QueryParams {
     int H, k, ns, ldv, ldm, n_l0_slots, nExt0, cfg;
-    int chain, g, leaves_x;  // levels lifted by the chain units; group, leaves per row
-    const int* chain_tab;    // per sorted viewpoint, levels l = 1 .. min(chain + 1, H): {level-l slot,
-                             // level-l group * 2 + (its level-l node holds another viewpoint)}
+    int chain;              // levels lifted by the chain units
     const int* vp0;         // per sorted viewpoint {leaf, u, leaf-run start, leaf-run end}
     const int* inv;         // original index -> sorted index or -1
-    const int* l0;          // per level-1 slot {sorted index or -1, level-1 group}
+    const int* low;         // chain > 0: per sorted viewpoint, levels l = 1 .. min(chain + 1, H):
+                            // {level-l slot, level-l group * 2 + (its level-l node holds another
+                            // viewpoint)}; else per level-1 slot {sorted index or -1, level-1 group}
     const int* ext0;        // leaf port -> cell
     MatSet leaves;
     uint16_t* X[kMaxQueryLevels + 1];  // port vectors X_l, l < H ([exterior port of level l][ldv])
@@ -359,7 +359,7 @@ struct PlanLayout {
     int k, kpow;            // kpow = plan_kpow(k): the sort size
     size_t sort_bytes;      // plan_sort_bytes(kpow)
     int* plan;
-    int o_vp0, o_inv, o_l0, o_rec, o_chain;
+    int o_vp0, o_inv, o_low, o_rec;
     long long flags_off[kMaxQueryLevels + 1];
     unsigned* ticket;
     unsigned ticket_base;

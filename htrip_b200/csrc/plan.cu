@@ -390,7 +390,7 @@ plan_query_kernel(const int32_t* __restrict__ vps, const uint8_t* __restrict__ p
         if (!fail) {
             int* grp = plan + O.o_groups[l];
             int* s2v = plan + O.o_s2v[l];
-            int* l0 = plan + O.o_l0;
+            int* low = plan + O.o_low;
             int* lift = l < H ? plan + O.o_lift[l] : nullptr;
             int* items = plan + O.o_items[l];
             int* meet = plan + O.o_meet[l];
@@ -407,24 +407,24 @@ plan_query_kernel(const int32_t* __restrict__ vps, const uint8_t* __restrict__ p
                     const int i = W.gstart[q] + idx;
                     s2v[s] = i;
                     W.slot[i] = s;
-                    if (l <= G.chain + 1) {  // (only read when chain > 0)
+                    if (G.chain > 0 && l <= G.chain + 1) {
                         const int gl = G.side[l] / G.b, gsh = G.g_shift >= 0 ? G.g_shift * l : -1;
                         const int nx = divp(W.vtx[i], gl, gsh), ny = divp(W.vty[i], gl, gsh);
-                        int* ct = plan + O.o_chain + i * kChainInts + 2 * (l - 1);
+                        int* ct = low + i * kChainInts + 2 * (l - 1);
                         ct[0] = s;
                         ct[1] = 2 * q + ((i > 0 && divp(W.vtx[i - 1], gl, gsh) == nx && divp(W.vty[i - 1], gl, gsh) == ny) ||
                                          (i + 1 < ns && divp(W.vtx[i + 1], gl, gsh) == nx &&
                                           divp(W.vty[i + 1], gl, gsh) == ny));
                     }
-                    if (l == 1) {
-                        l0[2 * s] = i;
-                        l0[2 * s + 1] = q;
+                    if (l == 1 && G.chain == 0) {
+                        low[2 * s] = i;
+                        low[2 * s + 1] = q;
                     }
                 } else {
                     s2v[s] = -1;
-                    if (l == 1) {
-                        l0[2 * s] = -1;
-                        l0[2 * s + 1] = -1;
+                    if (l == 1 && G.chain == 0) {
+                        low[2 * s] = -1;
+                        low[2 * s + 1] = -1;
                     }
                     if (lift) {
                         lift[2 * s] = 0;
@@ -560,12 +560,9 @@ plan_query_kernel(const int32_t* __restrict__ vps, const uint8_t* __restrict__ p
         Pq->ldm = max(8, (ns + 7) / 8 * 8);
         Pq->n_l0_slots = n_l0;
         Pq->chain = G.chain;
-        Pq->g = G.g;
-        Pq->leaves_x = G.leaves_x;
-        Pq->chain_tab = plan + O.o_chain;
         Pq->vp0 = plan + O.o_vp0;
         Pq->inv = plan + O.o_inv;
-        Pq->l0 = plan + O.o_l0;
+        Pq->low = plan + O.o_low;
         if (bad) O.words[0] = 2;
         // host record in one 8-byte store: seq | root (13 bits) | ns (13 bits) | status (2 bits)
         if (O.info)

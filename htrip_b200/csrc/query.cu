@@ -438,7 +438,7 @@ static_assert(sizeof(ChainSmem) <= kChainSmemBytes, "shared memory of a chain un
 __device__ __forceinline__ void do_chain(const QueryParams& P, int v, ChainSmem& S, int* tab) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ldv = P.ldv, H = P.H, top = P.chain;
     const int4 vp = *reinterpret_cast<const int4*>(P.vp0 + 4 * v);  // {leaf, cell, ..}
-    if (tid < kChainInts) tab[tid] = P.chain_tab[v * kChainInts + tid];
+    if (tid < kChainInts) tab[tid] = P.low[v * kChainInts + tid];
     bool skip = false;
     if (P.dirty) {
         const int d = P.dirty[v];
@@ -792,12 +792,12 @@ __device__ bool run_unit(const QueryParams& P, int t, int u, int* kl, int* wsum,
             const int e1 = min(total, (u + 1) * kQueryL0Chunk);
             for (int e = u * kQueryL0Chunk + tid; e < e1; e += kThreads) {
                 const int p = e / S1, s = e - p * S1;
-                const int j = P.l0[2 * s];
+                const int j = P.low[2 * s];
                 if (j < 0 || (P.dirty && !dirty_at(P.dirty, j, 0))) continue;
                 const int* v = P.vp0 + 4 * j;
                 const uint16_t d = P.leaves.base[((size_t)v[0] * P.leaves.NP + v[1]) * P.leaves.NP + P.ext0[p]];
                 P.X[0][(size_t)p * P.ldv + s] = d;
-                if (d < INF && P.H >= 1) P.lv[1].flags[(size_t)P.l0[2 * s + 1] * P.nExt0 + p] = 1;
+                if (d < INF && P.H >= 1) P.lv[1].flags[(size_t)P.low[2 * s + 1] * P.nExt0 + p] = 1;
             }
         } else {
             const int j = (u - n_fill) * kThreads + tid;
