@@ -310,10 +310,7 @@ inline size_t query_counter_words(int H, int k) { return 4 + (size_t)(H + 1) * (
 //                  item, its parts in order), then meet items of level t-1
 //                  (t >= 2)
 //   t = H+2        output chunks of kQueryFinChunk entries
-#ifndef HB_QUERY_THREADS
-#define HB_QUERY_THREADS 256
-#endif
-constexpr int kQueryThreads = HB_QUERY_THREADS;
+constexpr int kQueryThreads = 256;
 constexpr int kQueryL0Chunk = 512;
 constexpr int kQueryFinChunk = 1024;
 

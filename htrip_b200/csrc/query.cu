@@ -434,6 +434,7 @@ struct ChainSmem {
     int wcnt[kWarps], ccnt[kWarps];
 };
 static_assert(sizeof(ChainSmem) <= kChainSmemBytes, "shared memory of a chain unit");
+static_assert(4 * kThreads >= kMaxChainNP, "a thread per port of a child (a quarter of the node's at most)");
 
 __device__ __forceinline__ void do_chain(const QueryParams& P, int v, ChainSmem& S, int* tab) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ldv = P.ldv, H = P.H, top = P.chain;
