@@ -311,6 +311,11 @@ struct UpdateArena {
     // and where they are in the arena)
     size_t trace_off = 0;
     int trace_valid = 0;
+    // At least n bytes of `dev` for a call; the last opening's trace, which lies in it, is gone.
+    void reserve_dev(size_t n, cudaStream_t st) {
+        trace_valid = 0;
+        dev.reserve(n, st);
+    }
     void release() {
         dev.release();
         snap.release();
@@ -508,7 +513,7 @@ void upload_passable(htrip_index* h, const uint8_t* observed, int rows, int cols
     cudaStream_t st = h->stream;
     const size_t n = (size_t)rows * cols;
     h->pass.reserve((size_t)h->S * h->S);
-    h->u.dev.reserve(std::max<size_t>(1, n), st);
+    h->u.reserve_dev(std::max<size_t>(1, n), st);
     if (n) ck(cudaMemcpyAsync(h->u.dev.p, observed, n, cudaMemcpyHostToDevice, st), "grid");
     hb::launch_passable(h->u.dev.p, rows, cols, h->pass.p, h->S, st);
     ck(cudaGetLastError(), "passability");
@@ -692,7 +697,7 @@ void close_matrices(htrip_index* h, Level& Lv, const std::vector<int>& act) {
     const size_t slots_b = align256(n * sizeof(hb::Slot));
     A.stage.reserve(slots_b);
     A.rb.reserve(n * sizeof(int));
-    A.dev.reserve(slots_b + n * sizeof(int), st);
+    A.reserve_dev(slots_b + n * sizeof(int), st);
     auto* hs = reinterpret_cast<hb::Slot*>(A.stage.p);
     for (int i = 0; i < n; ++i) hs[i] = level_slot(Lv, nullptr, act[i], 0, 0);
     ck(cudaMemcpyAsync(A.dev.p, A.stage.p, n * sizeof(hb::Slot), cudaMemcpyHostToDevice, st), "slots");
@@ -1224,7 +1229,7 @@ void run_open_tasks(std::vector<OpenTask*>& tasks, UpdateArena& A, cudaStream_t 
         const size_t o_piv = o_dec + align256(n_slots);
         const size_t total = o_piv + align256(n_tasks * sizeof(int));
         A.stage.reserve(total);
-        A.dev.reserve(total, st);
+        A.reserve_dev(total, st);
         A.rb.reserve(total - o_cnt);
         std::memset(A.stage.p + o_cnt, 0, total - o_cnt);
         auto* hs = reinterpret_cast<hb::Slot*>(A.stage.p);
@@ -1436,7 +1441,7 @@ void run_open_device(std::vector<OpenTask*>& tasks, UpdateArena& A, cudaStream_t
         g.end = off;
         gl.push_back(std::move(g));
     }
-    A.dev.reserve(off, st);
+    A.reserve_dev(off, st);
     A.stage.reserve(off);
     A.rb.reserve(off);
     if (!A.open_grid) A.open_grid = hb::open_grid_blocks(device);

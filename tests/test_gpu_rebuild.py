@@ -4,7 +4,7 @@ incremental state) reaches no later result.  Matrices, statistics and distances
 against the CPU restatement of the reference, tolerance 0."""
 import pytest
 
-from helpers import FREE, make_grid
+from helpers import FREE, OBST, make_grid
 from htrip_b200 import workloads as W
 from oracle.ref import PortOracle, port_available
 
@@ -32,3 +32,27 @@ def test_build_on_a_handle_clears_flags_of_a_failed_opening(gpu, kind, side, b, 
     assert _stats(dev) == cpu.stats()
     assert dev.lastOpenLevels() == new.lastOpenLevels()
     assert dev.stateDigest() == new.stateDigest()
+
+
+@pytest.mark.parametrize("change", ["build", "blocked", "leaves", "weight"])
+def test_no_opening_trace_after_a_rebuild(gpu, change):
+    """The trace's device memory is the rebuild's staging: it is not read afterwards."""
+    from htrip_b200.minplus_oracle import HierarchyConfig, HtripError, MinPlusOracle
+    observed, cells = W.withheld_open(make_grid("noise", 64, 64, 3), 20, 5)
+    dev = MinPlusOracle(HierarchyConfig(16, 2, 2))
+    assert dev.build(observed)
+    observed[cells[:, 0], cells[:, 1]] = FREE
+    dev.onBatchCellsOpened(cells, observed)
+    assert len(dev.lastOpenTrace()) > 0
+    p = tuple(int(x) for x in cells[0])
+    if change == "build":
+        assert dev.build(observed)
+    elif change == "blocked":
+        observed[p] = OBST
+        dev.onCellBlocked(p, observed)
+    elif change == "leaves":
+        dev.onBatchLeavesChanged([0], observed)
+    else:
+        dev.onCellWeightChanged(p, 5, observed)
+    with pytest.raises(HtripError, match="no device-driven opening"):
+        dev.lastOpenTrace()
