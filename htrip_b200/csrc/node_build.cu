@@ -626,6 +626,7 @@ __global__ void __launch_bounds__(32 * W * KS, 2) node_tile_kernel(const NodeBui
 // 252 -> 217 us.
 // ---------------------------------------------------------------------------
 constexpr int kSmallSeams = 64, kSmallPorts = 64;
+constexpr size_t kSmallSmem = 100 * 1024;  // two CTAs an SM
 
 struct SmallLayout {
     int RP, ldU;  // row strides of R and U (multiples of 8)
@@ -847,6 +848,8 @@ __global__ void pad_fill_kernel(MatSet M, int y0) {
 constexpr int kMaxGridY = 65535;
 inline unsigned blocks_for(size_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
+// `bytes` is one value per kernel, whatever the index: the limit belongs to the kernel and the
+// device, and another thread may be between its own limit and its launch.
 template <class K>
 void allow_smem(K kernel, size_t bytes) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -880,7 +883,7 @@ void launch_pad_fill(MatSet M, int count, cudaStream_t st) {
 
 bool node_build_small(const NodeBuild& P) {
     return P.n_seams <= kSmallSeams && P.nP <= kSmallPorts &&
-           small_layout(P.g * P.g, P.nP, P.capI).total <= 100 * 1024;
+           small_layout(P.g * P.g, P.nP, P.capI).total <= kSmallSmem;
 }
 
 size_t node_build_layout(NodeBuild& P, int n, unsigned char* base) {
@@ -910,10 +913,10 @@ void launch_node_build(const NodeBuild& P, int n, cudaStream_t st) {
     if (node_build_small(P)) {
         const size_t smem = small_layout(g2, P.nP, P.capI).total;
         if (P.nP <= 32) {
-            allow_smem(node_small_kernel<16, 256>, smem);
+            allow_smem(node_small_kernel<16, 256>, kSmallSmem);
             node_small_kernel<16, 256><<<n, 256, smem, st>>>(P);
         } else {
-            allow_smem(node_small_kernel<32, 512>, smem);
+            allow_smem(node_small_kernel<32, 512>, kSmallSmem);
             node_small_kernel<32, 512><<<n, 512, smem, st>>>(P);
         }
         return;

@@ -2,6 +2,8 @@
 behind (flags of a failed opening, a trace, scratch memory, weights, an
 incremental state) reaches no later result.  Matrices, statistics and distances
 against the CPU restatement of the reference, tolerance 0."""
+import threading
+
 import pytest
 
 from helpers import FREE, OBST, make_grid
@@ -56,3 +58,28 @@ def test_no_opening_trace_after_a_rebuild(gpu, change):
         dev.onCellWeightChanged(p, 5, observed)
     with pytest.raises(HtripError, match="no device-driven opening"):
         dev.lastOpenTrace()
+
+
+def test_indexes_of_several_tile_sides_build_at_once(gpu):
+    """Threads with an index each: one's launches do not set limits for the other's."""
+    from htrip_b200.minplus_oracle import HierarchyConfig, MinPlusOracle
+    errors, digests = [], {}
+
+    def work(b):
+        try:
+            grid = make_grid("noise", 2 * b, 2 * b, b)
+            dev = MinPlusOracle(HierarchyConfig(b, 2, 2))
+            assert dev.build(grid)
+            digests[b] = dev.stateDigest()
+            for _ in range(2000):
+                assert dev.build(grid)
+            assert dev.stateDigest() == digests[b]
+        except Exception as e:  # noqa: BLE001 (reported below)
+            errors.append((b, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(b,)) for b in (10, 16, 11, 15)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert errors == []
