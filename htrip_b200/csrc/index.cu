@@ -146,6 +146,25 @@ struct PoolBuf {
     }
 };
 
+// Device scratch that a call needs and its index does not keep: from the
+// device's scratch pool and back to it, in the order of the call's stream.
+struct CallScratch {
+    unsigned char* p = nullptr;
+    cudaStream_t st;
+    CallScratch(size_t bytes, cudaStream_t stream) : st(stream) {
+        if (!bytes) return;
+        int device = 0;
+        ck(cudaGetDevice(&device), "cudaGetDevice");
+        ck(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), bytes, scratch_pool(device), st),
+           "cudaMallocFromPoolAsync");
+    }
+    CallScratch(const CallScratch&) = delete;
+    CallScratch& operator=(const CallScratch&) = delete;
+    ~CallScratch() {
+        if (p) cudaFreeAsync(p, st);
+    }
+};
+
 // A piece of an index's device arena.
 template <class T>
 struct Span {
@@ -302,9 +321,9 @@ struct UpdateArena {
     PoolBuf<uint8_t> pflags;
     HostBuf stage, rb;
     cudaEvent_t ev_cnt = nullptr;  // an opening level's pivot counts reached the host
-    // node builds: the staged node lists and the scratch of the launches (hb::node_build_layout)
+    // node builds: the staged node lists
     HostBuf nstage;
-    PoolBuf<unsigned char> nlist, nscratch;
+    PoolBuf<unsigned char> nlist;
     int open_grid = 0;             // CTAs of the persistent opening kernel
     SideStream side;               // openings of indexes of several (b, g), side by side
     // phase time stamps of the last device-driven opening launch (device,
@@ -325,7 +344,6 @@ struct UpdateArena {
         rb.release();
         nstage.release();
         nlist.release();
-        nscratch.release();
         side.release();
         if (ev_cnt) cudaEventDestroy(ev_cnt);
         ev_cnt = nullptr;
@@ -834,7 +852,8 @@ void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int 
         chunk[l] = (int)std::min<size_t>({(size_t)count(l), std::max<size_t>(1, kNodeScratch / per), (size_t)65535});
         scratch = std::max(scratch, hb::node_build_layout(P, chunk[l], nullptr));
     }
-    if (scratch) A.nscratch.reserve(scratch, st);
+    // for the call alone: 0.2 GB for the root of a 2048 x 2048 map, which an index at rest has no use for
+    CallScratch work(scratch, st);
     for (int l = 1; l <= H; ++l)
         for (int c0 = 0; c0 < count(l); c0 += chunk[l]) {
             hb::NodeBuild P = nb[l];
@@ -843,7 +862,7 @@ void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int 
             if (P.list) P.list += c0;
             if (P.active) P.active += c0;
             if (P.parent) P.parent += c0;
-            if (!hb::node_build_small(P)) hb::node_build_layout(P, n, A.nscratch.p);
+            if (!hb::node_build_small(P)) hb::node_build_layout(P, n, work.p);
             hb::launch_node_build(P, n, st);
             ck(cudaGetLastError(), "node build");
         }
@@ -3680,7 +3699,7 @@ htrip_status htrip_memory_bytes(const htrip_index* h, uint64_t* reference_bytes,
     uint64_t ref = 0, dev = 0;
     if (h->built) {
         ref = h->ref_bytes;
-        dev += h->arena.n + h->u.nlist.n + h->u.nscratch.n;
+        dev += h->arena.n + h->u.nlist.n;
         dev += h->pass.n + h->u.dev.n + h->u.snap.n * 2 + h->u.panel.n * 2 + h->u.pflags.n + h->q.dev.n +
                h->wts.n * sizeof(uint16_t);
     }

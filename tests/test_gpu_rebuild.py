@@ -4,6 +4,7 @@ incremental state) reaches no later result.  Matrices, statistics and distances
 against the CPU restatement of the reference, tolerance 0."""
 import threading
 
+import numpy as np
 import pytest
 
 from helpers import FREE, OBST, make_grid
@@ -83,3 +84,21 @@ def test_indexes_of_several_tile_sides_build_at_once(gpu):
     for t in threads:
         t.join()
     assert errors == []
+
+
+@pytest.mark.parametrize("side,b,g", [(512, 8, 2), (500, 32, 2), (486, 6, 3)])
+def test_build_scratch_is_given_back(gpu, side, b, g):
+    """An index holds its estimate, the staged grid and small tables: per node at most
+    64 bytes of state, per level a few blocks of 256 bytes, lists of a call's leaves and nodes."""
+    from htrip_b200.minplus_oracle import HierarchyConfig, MinPlusOracle, estimate_bytes
+    cfg = HierarchyConfig(b, g, g)
+    grid = make_grid("noise", side, side, 1)
+    dev = MinPlusOracle(cfg)
+    assert dev.build(grid)
+    nodes = dev.num_leaf_tiles_x ** 2 * g * g // (g * g - 1) + 1
+    bound = estimate_bytes(cfg, side, side) + dev.S ** 2 + 64 * nodes + (dev.H + 1) * 16 * 256 + 65536
+    assert dev.deviceMemoryBytes() <= bound
+    p = tuple(int(x) for x in np.argwhere(grid == FREE)[100])
+    grid[p] = OBST
+    dev.onCellBlocked(p, grid)
+    assert dev.deviceMemoryBytes() <= bound
