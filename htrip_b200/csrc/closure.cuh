@@ -1,6 +1,6 @@
-// Block primitives of the pivot-set closures (open.cu, node_build.cu): the
-// Floyd-Warshall of a 64-pivot block with the pivot rows of a column tile, and
-// the 64 x 64 min-plus product.  All run on a 256-thread CTA.
+// Block primitives of the pivot-set closures (open.cu, node_build.cu, kernels.cu): the
+// Floyd-Warshall of a 64-pivot block, alone or with the pivot rows of a column tile.
+// All run on a 256-thread CTA.
 #pragma once
 #include "minplus.cuh"
 
@@ -54,17 +54,16 @@ __device__ __forceinline__ void close_pivot_block(uint16_t (*Ts)[kTLD], int mk) 
 // matrix M = [T | Bt], 64 rows x 32 CW columns (T the pivot block in the first 64,
 // Bt the pivot rows of a column tile), becomes [T* | T* (x) Bt]: a shortest path
 // from pivot a to column j through pivots ends with one entry of a pivot row.
-// Blocked Floyd-Warshall in steps of 16 pivots K: the 16 x 16 block is closed by
-// four squarings (T is symmetric, so a squared entry is a product of two
-// rows), then the rows K follow as block* (x) M[K, :], then M = min(M, P^T (x) P).
-// Thread (rg, cg) = (t / 16, t % 16) owns rows 4 rg .. and columns 2 CW cg .. in
-// registers; 6 CTA barriers per 16 pivots.  A step per pivot with a barrier each, as
-// before, is a chain of 64 shared-memory round trips; the opening kernel's mixed
-// stages (panel with the old panel's update, beside the update) went from 35-38 to
-// 26-30 us, its first panels from 18-20 to 15-17 us.
+// Floyd-Warshall with M in registers: thread (rg, cg) = (t / 16, t % 16) owns rows
+// 4 rg .. and columns 2 CW cg ..; a step needs the pivot row only (T is symmetric, so its
+// T part is the pivot column too), which its owners put into one of two shared rows
+// at the step before: one barrier and two shared loads a step.  Blocks of 16
+// pivots with 6 barriers each, which this replaces, cost 4 us however few the
+// pivots are and no less than this at 64 (device time of an opening with 1 cell, 256 x 256
+// open map, b = 16: 128 -> 115 us; 256 cells, 1024 x 1024 street map, b = 8: 4351 -> 4147 us).
 // HALF: every finite value is <= kHalfMax and INF stands as kHalfInf: sums need
 // no clamp, one fused add-and-min per pair.  Values then saturate at kHalfInf, which
-// is exact while no finite distance reaches it; fw_exact checks that.
+// is exact while no finite distance reaches it; fw_panel checks that.
 // ---------------------------------------------------------------------------
 constexpr int kHalfMax = 16383;
 constexpr uint32_t kHalfInf = 32767u;
@@ -80,8 +79,7 @@ template <int CW>
 struct alignas(16) FwSmem {
     static constexpr int LD = 32 * CW + 8;  // padded row: the 8 rows of a 16-byte access phase hit distinct banks
     uint16_t M[64][LD];
-    uint16_t P[16][LD];
-    uint16_t S[2][16][24];
+    uint16_t P[2][LD];  // pivot rows of this step and the next
     int mx[2];
 };
 
@@ -115,15 +113,15 @@ __device__ __forceinline__ void st_words(uint16_t* p, const uint32_t (&w)[CW]) {
     }
 }
 
-// m[r][.] = min(m[r][.], min_{k < K} A[k][4 rg + r] (+) A[k][columns]) for the
+// m[r][.] = min(m[r][.], min_{k < B} A[k][4 rg + r] (+) A[k][columns]) for the
 // thread's tile; A has rows of stride LD with the pivot columns first.
-template <int CW, bool HALF, int K>
+template <int CW, bool HALF>
 __device__ __forceinline__ void fw_product(const uint16_t* A, uint32_t (&m)[4][CW]) {
     constexpr int LD = FwSmem<CW>::LD;
     const int rg = threadIdx.x >> 4, cg = threadIdx.x & 15;
     const uint16_t *ap = A + 4 * rg, *bp = A + 2 * CW * cg;
 #pragma unroll 2
-    for (int k = 0; k < K; ++k) {
+    for (int k = 0; k < B; ++k) {
         const uint2 a2 = *reinterpret_cast<const uint2*>(ap + k * LD);
         uint32_t b[CW];
         ld_words<CW>(bp + k * LD, b);
@@ -135,139 +133,102 @@ __device__ __forceinline__ void fw_product(const uint16_t* A, uint32_t (&m)[4][C
     }
 }
 
-// M (synchronised) and the thread's tile m of it -> the closed tile in m.
+// The thread's tile m of M -> the closed tile.
 template <int CW, bool HALF>
 __device__ __forceinline__ void fw_close(FwSmem<CW>& F, int mk, uint32_t (&m)[4][CW]) {
-    constexpr int LD = FwSmem<CW>::LD;
-    const int tid = threadIdx.x, rg = tid >> 4, cg = tid & 15;
+    const int rg = threadIdx.x >> 4, cg = threadIdx.x & 15;
+    if (rg == 0) st_words<CW>(&F.P[0][2 * CW * cg], m[0]);
+    __syncthreads();
 #pragma unroll 1
-    for (int k0 = 0; k0 < mk; k0 += 16) {
-        {
-            const uint16_t *ri = &F.M[k0 + rg][k0], *rj = &F.M[k0 + cg][k0];
-#pragma unroll 1
-            for (int q = 0; q < 4; ++q) {
-                uint32_t a[8], b[8], v = HALF ? kHalfInf2 : INF2;
-                ld_words<8>(ri, a);
-                ld_words<8>(rj, b);
+    for (int s0 = 0; s0 < mk; s0 += 4) {
 #pragma unroll
-                for (int x = 0; x < 8; ++x) v = acc_mode<HALF>(v, b[x], a[x]);
-                F.S[q & 1][rg][cg] = (uint16_t)min(v & 0xffffu, v >> 16);
-                __syncthreads();
-                ri = F.S[q & 1][rg];
-                rj = F.S[q & 1][cg];
-            }
+        for (int x = 0; x < 4; ++x) {
+            if (s0 + x >= mk) break;  // uniform
+            const uint2 a2 = *reinterpret_cast<const uint2*>(&F.P[x & 1][4 * rg]);
+            uint32_t b[CW];
+            ld_words<CW>(&F.P[x & 1][2 * CW * cg], b);
+            const uint32_t a[4] = {splat(a2.x), splat(a2.x >> 16), splat(a2.y), splat(a2.y >> 16)};
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int w = 0; w < CW; ++w) m[r][w] = acc_mode<HALF>(m[r][w], b[w], a[r]);
+            if (rg == (s0 + x + 1) >> 2) st_words<CW>(&F.P[(x + 1) & 1][2 * CW * cg], m[(x + 1) & 3]);
+            __syncthreads();
         }
-        {
-            uint32_t acc[CW];
-#pragma unroll
-            for (int w = 0; w < CW; ++w) acc[w] = HALF ? kHalfInf2 : INF2;
-            const uint16_t* bp = &F.M[k0][2 * CW * cg];
-#pragma unroll 4
-            for (int e = 0; e < 16; ++e) {
-                uint32_t b[CW];
-                ld_words<CW>(bp + e * LD, b);
-                const uint32_t a = splat(F.S[1][rg][e]);
-#pragma unroll
-                for (int w = 0; w < CW; ++w) acc[w] = acc_mode<HALF>(acc[w], b[w], a);
-            }
-            st_words<CW>(&F.P[rg][2 * CW * cg], acc);
-        }
-        __syncthreads();
-        fw_product<CW, HALF, 16>(&F.P[0][0], m);
-        if ((rg >> 2) == (k0 >> 4) + 1) {  // the next step's pivot rows
-#pragma unroll
-            for (int r = 0; r < 4; ++r) st_words<CW>(&F.M[4 * rg + r][2 * CW * cg], m[r]);
-        }
-        __syncthreads();
     }
 }
 
-// Whether every value of w fits the half range (INF aside).
-__device__ __forceinline__ bool half_ok(uint32_t w) {
-    const uint32_t lo = w & 0xffffu, hi = w >> 16;
-    return (lo <= (uint32_t)kHalfMax || lo >= INF) && (hi <= (uint32_t)kHalfMax || hi >= INF);
+// Largest finite value of packed words, INF (full range) or kHalfInf (half range, no value
+// above it) aside: the words are shifted so that INF becomes 0.
+template <bool HALF>
+__device__ __forceinline__ uint32_t top_of(uint32_t top, uint32_t w) {
+    constexpr uint32_t shift = 0x10000u - (HALF ? kHalfInf : (uint32_t)INF);
+    return max2(top, add2(w, shift * 0x00010001u));
 }
-// Half-range sums (kHalfInf or more: INF) as full-range values.
+template <bool HALF>
+__device__ __forceinline__ int top_value(uint32_t top) {
+    constexpr int shift = 0x10000 - (HALF ? (int)kHalfInf : (int)INF);
+    return max((int)max(top & 0xffffu, top >> 16) - shift, 0);
+}
+template <bool HALF, int R, int W>
+__device__ __forceinline__ int tile_top(const uint32_t (&m)[R][W]) {
+    uint32_t top = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int w = 0; w < W; ++w) top = top_of<HALF>(top, m[r][w]);
+    return top_value<HALF>(top);
+}
+// Half-range sums (65534 at most; kHalfInf or more: INF) as full-range values.
 __device__ __forceinline__ uint32_t half_to_full(uint32_t w) {
-    const uint32_t lo = w & 0xffffu, hi = w >> 16;
-    return (lo >= kHalfInf ? (uint32_t)INF : lo) | ((hi >= kHalfInf ? (uint32_t)INF : hi) << 16);
-}
-// Largest value below kHalfInf of a tile.
-template <int CW>
-__device__ __forceinline__ int half_max(const uint32_t (&m)[4][CW]) {
-    uint32_t mx = 0;
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int w = 0; w < CW; ++w) {
-            const uint32_t lo = m[r][w] & 0xffffu, hi = m[r][w] >> 16;
-            if (lo < kHalfInf) mx = max(mx, lo);
-            if (hi < kHalfInf) mx = max(mx, hi);
-        }
-    return (int)mx;
+    const uint32_t inf = (w + 0x00010001u) & 0x80008000u;  // the top bit of a half that is INF ..
+    return min2(w | (2 * inf - (inf >> 15)), INF2);         // .. -> all its bits
 }
 
 // The whole of it for the tile in F.M (synchronised; raw values, INF = 60000):
 // with Q, first M = min(M, Q_T^T (x) Q) (a 64 x 32 CW panel of the round before).
-// m receives the closed tile with INF = 60000.  Returns false when the half range
-// turned out too small (F is used up; call again on fresh copies with half
-// off).  A finite distance of kHalfInf or more would have a prefix, itself a
-// distance between pivots, within one entry of M of kHalfInf: none is there when
+// m receives the closed tile with INF = 60000.  The half range is tried with Q, whose
+// product is most of the work; without it the checks cost more than the clamps.
+// Returns false when the half range turned out too small (Q is used up; call again on
+// fresh copies with half off).  A finite distance of kHalfInf or more would have a
+// prefix, itself a distance between pivots, within one entry of M of kHalfInf: none is there when
 // the largest finite result and the largest finite entry add up to less.
 template <int CW>
 __device__ __forceinline__ bool fw_panel(FwSmem<CW>& F, uint16_t* Q, int mk, bool try_half, uint32_t (&m)[4][CW]) {
     constexpr int LD = FwSmem<CW>::LD;
     const int tid = threadIdx.x, rg = tid >> 4, cg = tid & 15;
-    bool ok = try_half;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        ld_words<CW>(&F.M[4 * rg + r][2 * CW * cg], m[r]);
-#pragma unroll
-        for (int w = 0; w < CW; ++w) ok &= half_ok(m[r][w]);
-    }
+    for (int r = 0; r < 4; ++r) ld_words<CW>(&F.M[4 * rg + r][2 * CW * cg], m[r]);
+    bool half = false;
     if (Q) {
+        uint32_t q[4][CW];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            uint32_t q[CW];
-            ld_words<CW>(Q + (4 * rg + r) * LD + 2 * CW * cg, q);
-#pragma unroll
-            for (int w = 0; w < CW; ++w) ok &= half_ok(q[w]);
-        }
+        for (int r = 0; r < 4; ++r) ld_words<CW>(Q + (4 * rg + r) * LD + 2 * CW * cg, q[r]);
+        if (tid < 2) F.mx[tid] = 0;
+        half = __syncthreads_and(try_half && max(tile_top<false>(m), tile_top<false>(q)) <= kHalfMax);
     }
-    if (tid < 2) F.mx[tid] = 0;
-    if (!__syncthreads_and(ok)) {
-        if (Q) {
-            fw_product<CW, false, 64>(Q, m);
-#pragma unroll
-            for (int r = 0; r < 4; ++r) st_words<CW>(&F.M[4 * rg + r][2 * CW * cg], m[r]);
-            __syncthreads();
-        }
+    if (!half) {
+        if (Q) fw_product<CW, false>(Q, m);
         fw_close<CW, false>(F, mk, m);
         return true;
     }
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 4; ++r) {
+        uint32_t q[CW];
+        uint16_t* p = Q + (4 * rg + r) * LD + 2 * CW * cg;
+        ld_words<CW>(p, q);
 #pragma unroll
-        for (int w = 0; w < CW; ++w) m[r][w] = min2(m[r][w], kHalfInf2);
-    if (Q) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            uint32_t q[CW];
-            uint16_t* p = Q + (4 * rg + r) * LD + 2 * CW * cg;
-            ld_words<CW>(p, q);
-#pragma unroll
-            for (int w = 0; w < CW; ++w) q[w] = min2(q[w], kHalfInf2);
-            st_words<CW>(p, q);
+        for (int w = 0; w < CW; ++w) {
+            m[r][w] = min2(m[r][w], kHalfInf2);
+            q[w] = min2(q[w], kHalfInf2);
         }
-        __syncthreads();
-        fw_product<CW, true, 64>(Q, m);
+        st_words<CW>(p, q);
     }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) st_words<CW>(&F.M[4 * rg + r][2 * CW * cg], m[r]);
-    const int m0 = half_max<CW>(m);
     __syncthreads();
+    fw_product<CW, true>(Q, m);
+    const int m0 = tile_top<true>(m);
     fw_close<CW, true>(F, mk, m);
-    const int a = __reduce_max_sync(0xffffffffu, m0), z = __reduce_max_sync(0xffffffffu, half_max<CW>(m));
+    const int a = __reduce_max_sync(0xffffffffu, m0), z = __reduce_max_sync(0xffffffffu, tile_top<true>(m));
     if ((tid & 31) == 0) {
         atomicMax(&F.mx[0], a);
         atomicMax(&F.mx[1], z);

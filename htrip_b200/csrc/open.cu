@@ -19,7 +19,7 @@
 //   compact(l) pivot flags -> sorted pivot list per matrix.
 //   rounds     blocked pivot-set Kleene closure, kOpenB pivots per round:
 //              panel: every CTA of a column tile closes the round's pivot
-//                block T = D[K, K] itself (16 pivots a step in shared memory)
+//                block T = D[K, K] itself (Floyd-Warshall in registers)
 //                and computes P[:, tile] = T* (x) D[K, tile];
 //              update: D = min(D, P^T (x) P) over upper-triangle tiles, each
 //                also written transposed (D is symmetric), and only where an
@@ -492,7 +492,8 @@ __device__ void panel_unit(const OpenLaunch& L, int l, int s, int j0, int r, uns
     }
     uint16_t* P = panel_of(L, r, s, NP);
     const int rg = tid >> 4, cg = tid & 15;
-    bool any = false, wide = false;
+    bool any = false;
+    uint32_t top = 0;
     if (cg >= 8) {  // the tile's columns
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
@@ -502,9 +503,10 @@ __device__ void panel_unit(const OpenLaunch& L, int l, int s, int j0, int r, uns
                 make_uint4(m[x][0], m[x][1], m[x][2], m[x][3]);
             any |= m[x][0] != INF2 || m[x][1] != INF2 || m[x][2] != INF2 || m[x][3] != INF2;
 #pragma unroll
-            for (int w = 0; w < 4; ++w) wide |= !half_ok(m[x][w]);
+            for (int w = 0; w < 4; ++w) top = top_of<false>(top, m[x][w]);
         }
     }
+    const bool wide = top_value<false>(top) > kHalfMax;
     const int flag = (__syncthreads_or(any) ? 1 : 0) | (__syncthreads_or(wide) ? 2 : 0);
     if (tid == 0) pflags_of(L, r, s, NP)[j0 / 64] = (uint8_t)flag;
 }
@@ -804,19 +806,7 @@ __device__ __forceinline__ bool close_small(const uint16_t* Dm, const int* kl, i
     constexpr int TR = NP / 16, TW = TR / 2;
     static_assert(TW == 4 || TW == 2, "NP is 128 or 64");
     const int tid = threadIdx.x, rg = tid >> 4, cg = tid & 15;
-    uint32_t m0 = 0;
-    auto top = [&] {
-        uint32_t m = 0;
-#pragma unroll
-        for (int r = 0; r < TR; ++r)
-#pragma unroll
-            for (int w = 0; w < TW; ++w) {
-                const uint32_t lo = d[r][w] & 0xffffu, hi = d[r][w] >> 16;
-                if (lo < kHalfInf) m = max(m, lo);
-                if (hi < kHalfInf) m = max(m, hi);
-            }
-        return __reduce_max_sync(FULL, m);
-    };
+    int m0 = 0;
     auto publish = [&](int s) {  // pivot s's row
         const int row = kl[s];
         if (row / TR != rg) return;
@@ -842,7 +832,7 @@ __device__ __forceinline__ bool close_small(const uint16_t* Dm, const int* kl, i
 #pragma unroll
             for (int w = 0; w < TW; ++w) d[r][w] = min2(d[r][w], kHalfInf2);
     }
-    if constexpr (HALF) m0 = top();
+    if constexpr (HALF) m0 = __reduce_max_sync(FULL, tile_top<true>(d));
     if (k > 0) publish(0);
     __syncthreads();
 #pragma unroll 1
@@ -860,10 +850,10 @@ __device__ __forceinline__ bool close_small(const uint16_t* Dm, const int* kl, i
         __syncthreads();
     }
     if constexpr (HALF) {
-        const uint32_t z = top();
+        const int z = __reduce_max_sync(FULL, tile_top<true>(d));
         if ((tid & 31) == 0) {
-            atomicMax(mx, (int)m0);
-            atomicMax(mx + 1, (int)z);
+            atomicMax(mx, m0);
+            atomicMax(mx + 1, z);
         }
         __syncthreads();
         if (mx[0] + mx[1] >= (int)kHalfInf) return false;
@@ -997,16 +987,16 @@ __device__ void small_unit(const OpenLaunch& L, int l, int s, unsigned char* sme
     }
     uint32_t d[TR][TW];
     const int rg = tid >> 4, cg = tid & 15;
-    bool ok = true;
+    uint32_t top = 0;
 #pragma unroll
     for (int r = 0; r < TR; ++r) {
         uint32_t w[TW];
         ld_words<TW>(Dm + (TR * rg + r) * NP + TR * cg, w);
 #pragma unroll
-        for (int x = 0; x < TW; ++x) ok &= half_ok(w[x]);
+        for (int x = 0; x < TW; ++x) top = top_of<false>(top, w[x]);
     }
     bool done = false;
-    if (__syncthreads_and(ok)) {
+    if (__syncthreads_and(top_value<false>(top) <= kHalfMax)) {
         done = close_small<NP, true>(Dm, kl, k, Pr, s_mx, d);
         __syncthreads();  // the pivot row buffers are free
     }
