@@ -44,6 +44,7 @@
 #include "kernels.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace hb {
 
@@ -523,6 +524,10 @@ __device__ void panel_unit(const OpenLaunch& L, int l, int s, int j0, int r, uns
 // with the panel: 0 all INF (skip), 1 all <= INF_HEADROOM (2-op form, no
 // wrap), 2 otherwise (3-op clamped form).  Panel blocks without a value beyond the half
 // range (their flag's second bit) take the 2-op form throughout, INF as kHalfInf.
+// Each form has a loop of its own: in one loop with the form chosen inside, the range's
+// branch and its unrolled copies cost registers and instruction fetches (kernel, 1024 x 1024
+// street map, b = 8, 256 cells: 4137 -> 3600 us; one cell on a 256 x 256 open map, b = 16:
+// 115 -> 111).
 // ---------------------------------------------------------------------------
 template <int RW, int CP>
 __device__ void update_unit(const OpenLaunch& L, int l, int s, int I, int J, int r, unsigned char* smem) {
@@ -587,7 +592,44 @@ __device__ void update_unit(const OpenLaunch& L, int l, int s, int I, int J, int
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
     __syncthreads();
-    if (!half) {
+    uint32_t acc[RW][CP];
+#pragma unroll
+    for (int rr = 0; rr < RW; ++rr)
+#pragma unroll
+        for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = INF2;
+    auto step = [&](int k, auto mode) {
+        constexpr int M = decltype(mode)::value;  // 0 half range, 1 unclamped, 2 clamped
+        uint32_t bv[CP];
+#pragma unroll
+        for (int cc = 0; cc < CP; ++cc) {
+            bv[cc] = reinterpret_cast<const uint32_t*>(Bs + k * TT + lane * 2 * CP)[cc];
+            if constexpr (M == 0) bv[cc] = min2(bv[cc], kHalfInf2);
+        }
+        const uint32_t* ar = As + k * TT + warp * RW;
+        uint32_t av[RW];
+#pragma unroll
+        for (int q = 0; q < RW / 4; ++q) {
+            const uint4 x = reinterpret_cast<const uint4*>(ar)[q];
+            av[4 * q] = x.x; av[4 * q + 1] = x.y; av[4 * q + 2] = x.z; av[4 * q + 3] = x.w;
+        }
+#pragma unroll
+        for (int rr = 0; rr < RW; ++rr) {
+            const uint32_t tt = INF2 - av[rr];
+#pragma unroll
+            for (int cc = 0; cc < CP; ++cc) {
+                if constexpr (M == 2) acc[rr][cc] = acc_clamp(acc[rr][cc], bv[cc], av[rr], tt);
+                else acc[rr][cc] = acc_fast(acc[rr][cc], bv[cc], av[rr]);
+            }
+        }
+    };
+    if (half) {
+#pragma unroll 1
+        for (int k = 0; k < mk; ++k) step(k, std::integral_constant<int, 0>());
+#pragma unroll
+        for (int rr = 0; rr < RW; ++rr)  // sums of kHalfInf or more: INF
+#pragma unroll
+            for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = half_to_full(acc[rr][cc]);
+    } else {
         for (int idx = tid; idx < mk * kWarps; idx += kThreads) {
             const int a = idx / kWarps, w = idx % kWarps;
             const uint32_t* ar = As + a * TT + w * RW;
@@ -601,48 +643,13 @@ __device__ void update_unit(const OpenLaunch& L, int l, int s, int I, int J, int
             cls[idx] = mn >= INF ? 0 : (mx <= INF_HEADROOM ? 1 : 2);
         }
         __syncthreads();
-    }
-    uint32_t acc[RW][CP];
-#pragma unroll
-    for (int rr = 0; rr < RW; ++rr)
-#pragma unroll
-        for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = INF2;
-#pragma unroll 2
-    for (int k = 0; k < mk; ++k) {
-        const int c = half ? 1 : cls[k * kWarps + warp];
-        if (c == 0) continue;  // uniform over the warp
-        uint32_t bv[CP];
-#pragma unroll
-        for (int cc = 0; cc < CP; ++cc) {
-            bv[cc] = reinterpret_cast<const uint32_t*>(Bs + k * TT + lane * 2 * CP)[cc];
-            if (half) bv[cc] = min2(bv[cc], kHalfInf2);
+#pragma unroll 1
+        for (int k = 0; k < mk; ++k) {
+            const int c = cls[k * kWarps + warp];
+            if (c == 0) continue;  // uniform over the warp
+            if (c == 1) step(k, std::integral_constant<int, 1>());
+            else step(k, std::integral_constant<int, 2>());
         }
-        const uint32_t* ar = As + k * TT + warp * RW;
-        uint32_t av[RW];
-#pragma unroll
-        for (int q = 0; q < RW / 4; ++q) {
-            const uint4 x = reinterpret_cast<const uint4*>(ar)[q];
-            av[4 * q] = x.x; av[4 * q + 1] = x.y; av[4 * q + 2] = x.z; av[4 * q + 3] = x.w;
-        }
-        if (c == 1) {
-#pragma unroll
-            for (int rr = 0; rr < RW; ++rr)
-#pragma unroll
-                for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = acc_fast(acc[rr][cc], bv[cc], av[rr]);
-        } else {
-#pragma unroll
-            for (int rr = 0; rr < RW; ++rr) {
-                const uint32_t tt = INF2 - av[rr];
-#pragma unroll
-                for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = acc_clamp(acc[rr][cc], bv[cc], av[rr], tt);
-            }
-        }
-    }
-    if (half) {  // sums of kHalfInf or more: INF
-#pragma unroll
-        for (int rr = 0; rr < RW; ++rr)
-#pragma unroll
-            for (int cc = 0; cc < CP; ++cc) acc[rr][cc] = half_to_full(acc[rr][cc]);
     }
     // epilogue: new = min(acc, old); changed entries are written
     const int col = jb + lane * 2 * CP;
