@@ -746,7 +746,8 @@ struct BuildSet {
 // Scratch of one launch of the general node build (bounds the nodes a launch takes).
 constexpr size_t kNodeScratch = (size_t)192 << 20;
 
-// Everything is issued on the index's stream and not waited for.
+// Everything is issued on the index's stream; with `track` the host waits once for the lowest
+// levels' flags, and weighted leaves of padded order above 64 for their pivot counts.
 void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int rows, int cols) {
     cudaStream_t st = h->stream;
     UpdateArena& A = h->u;
@@ -854,7 +855,19 @@ void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int 
     }
     // for the call alone: 0.2 GB for the root of a 2048 x 2048 map, which an index at rest has no use for
     CallScratch work(scratch, st);
-    for (int l = 1; l <= H; ++l)
+    bool asked = !bs.track;
+    for (int l = 1; l <= H; ++l) {
+        if (!asked && l >= 2 && !hb::node_build_small(nb[l])) {
+            // Did the lowest levels change anything?  If not, each level above would be a dozen
+            // launches that return at once (30 us); the wait costs a call that goes on about 8 us.
+            // Further up there is none: a level that was built saved more than its parents' launches.
+            ck(cudaMemcpyAsync(hs + o_active[l], ds + o_active[l], bs.nodes[l].size(), cudaMemcpyDeviceToHost, st),
+               "changed nodes");
+            ck(cudaStreamSynchronize(st), "changed nodes");
+            const unsigned char* f = hs + o_active[l];
+            if (std::find(f, f + bs.nodes[l].size(), 1) == f + bs.nodes[l].size()) break;
+            asked = true;
+        }
         for (int c0 = 0; c0 < count(l); c0 += chunk[l]) {
             hb::NodeBuild P = nb[l];
             const int n = std::min(chunk[l], count(l) - c0);
@@ -866,6 +879,7 @@ void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int 
             hb::launch_node_build(P, n, st);
             ck(cudaGetLastError(), "node build");
         }
+    }
 }
 
 // ---------------------------------------------------------------------------
