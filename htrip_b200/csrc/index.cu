@@ -1738,6 +1738,12 @@ int query_split_items(const htrip_index* h) {
     return it->second;
 }
 
+// Whether a level's project and meet items pick the ports on a seam: where at least a
+// quarter of the ports (about 1 / g) lie on none.  Query kernel, seam ports / all ports:
+// g = 2, 1024 x 1024 street map, b = 16, k = 509: 498 / 631 us; g = 4, 512 x 512, b = 8, k = 160:
+// 147 / 151; g = 8, 256 x 256, b = 4, k = 160: 75 / 73; g = 16, b = 16, k = 512: 334 / 317.
+int query_seam_rows(const Level& Lv) { return 4 * Lv.nExt >= Lv.n; }
+
 // Levels lifted viewpoint by viewpoint (QueryParams::chain): from the leaves
 // up, matrices of padded order <= 1024 (a viewpoint's rows are at most 0.5 MB,
 // read by one CTA in a few microseconds) while a child holds at most about 4
@@ -2090,6 +2096,7 @@ hb::QueryParams make_params(const htrip_index* h, const QueryPlan& P, unsigned c
         q.NP = Lv.NP;
         q.nP = Lv.nP;
         q.cols = Lv.d_cols.p;
+        q.seam_rows = query_seam_rows(Lv);
         q.groups = plan + PL.o_groups;
         q.flags = flags + PL.flags_off;
         q.items = plan + PL.o_items;
@@ -2540,6 +2547,7 @@ int run_devplan(htrip_index* h, int k, int cfg, const int32_t* vps_host, const u
         T.lv[l].NP = Lv.NP;
         T.lv[l].nP = Lv.nP;
         T.lv[l].cols = Lv.d_cols.p;
+        T.lv[l].seam_rows = query_seam_rows(Lv);
         T.lv[l].store_y = 1;
         T.lv[l].split = l == h->H ? D.root_split : 1;
         if (T.lv[l].split > 1) {

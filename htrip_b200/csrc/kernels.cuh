@@ -255,6 +255,7 @@ struct QueryLevel {
     uint8_t* flags;         // [group][nP] finite-port flags of X_{l-1}
     const int* items;       // project items {group, m0, n0}
     int n_items;
+    int seam_rows;          // only ports on a seam are operand rows (query_seam_rows)
     const int* meet;        // meet items {i0, j0, nj, group, coloff, kb, ke}
     int n_meet;
     const int* s2v;         // level-l slot -> sorted viewpoint or -1

@@ -249,6 +249,7 @@ plan_query_kernel(const int32_t* __restrict__ vps, const uint8_t* __restrict__ p
             lv.NP = tmpl.lv[l].NP;
             lv.nP = tmpl.lv[l].nP;
             lv.cols = tmpl.lv[l].cols;
+            lv.seam_rows = tmpl.lv[l].seam_rows;
             lv.store_y = tmpl.lv[l].store_y;
             lv.part = tmpl.lv[l].part;
             lv.ticket = tmpl.lv[l].ticket;

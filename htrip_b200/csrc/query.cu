@@ -232,7 +232,7 @@ __device__ __forceinline__ void count_work(unsigned long long* work, int n, int 
 }
 
 // Compacts the rows of a child (n ports) whose flag is set and that lie on a seam
-// (`cols`: the child's part of QueryLevel::cols) into kl (ascending); returns the
+// (`cols`: the child's part of QueryLevel::cols, or null: all) into kl (ascending); returns the
 // count (block-wide scan; every thread gets the total).
 __device__ __forceinline__ int compact_flags(const uint8_t* __restrict__ flags, const int* __restrict__ cols, int n,
                                              int* kl, int* wsum) {
@@ -243,7 +243,7 @@ __device__ __forceinline__ int compact_flags(const uint8_t* __restrict__ flags, 
     uint32_t mask = 0;
 #pragma unroll 4
     for (int j = 0; j < per; ++j)
-        if (p0 + j < p1) mask |= (uint32_t)((__ldcg(flags + p0 + j) != 0) & __ldg(cols + p0 + j)) << j;
+        if (p0 + j < p1) mask |= (uint32_t)((__ldcg(flags + p0 + j) != 0) & (cols ? __ldg(cols + p0 + j) : 1)) << j;
     const int cntl = __popc(mask);
     int incl = cntl;
 #pragma unroll
@@ -610,12 +610,12 @@ __device__ bool do_project(const QueryParams& P, const QueryLevel& L, const Quer
         for (int r = 0; r < min(RW, G[3] - m0); ++r) any |= dirty_at(P.dirty, G[4] + m0 + r, l);
         if (!any) return L.split <= 1 || part == 0;  // a skipped item counts once
     }
-    if (!Ln) {  // the root lifts nothing: only seam columns are read
+    if (!Ln && L.seam_rows) {  // the root lifts nothing: only seam columns are read
         int any = 0;
         for (int c = n0 + threadIdx.x; c < min(n0 + 64 * CP, L.NP); c += kThreads) any |= __ldg(L.cols + c) & 1;
         if (!__syncthreads_or(any)) return L.split <= 1 || part == 0;
     }
-    const int nA = compact_flags(L.flags + (size_t)gi * L.nP, L.cols + q * L.nP, L.nP, kl, wsum);
+    const int nA = compact_flags(L.flags + (size_t)gi * L.nP, L.seam_rows ? L.cols + q * L.nP : nullptr, L.nP, kl, wsum);
     const int kb = (int)((long)nA * part / L.split), ke = (int)((long)nA * (part + 1) / L.split);
     const uint16_t* D = L.D + (size_t)node * L.NP * L.NP + (size_t)q * L.nP * L.NP;
     const int col = n0 + lane * 2 * CP;
@@ -706,7 +706,7 @@ __device__ void do_meet(const QueryParams& P, const QueryLevel& L, int item, int
     }
     // the item's share of the rows that count: seam ports lie side by side, so equal
     // ranges of ports would be unequal work
-    const int nL = compact_flags(L.flags + (size_t)g2 * L.nP, L.cols + coloff, L.nP, kl, wsum);
+    const int nL = compact_flags(L.flags + (size_t)g2 * L.nP, L.seam_rows ? L.cols + coloff : nullptr, L.nP, kl, wsum);
     const int k0 = (int)((long)nL * kb / L.nP), nA = (int)((long)nL * ke / L.nP) - k0;
     const uint16_t* Xp = P.X[l - 1] + j0;
     const uint16_t* Y = P.Y[l] + (size_t)coloff * P.ldv + i0;
