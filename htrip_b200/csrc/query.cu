@@ -241,9 +241,15 @@ __device__ __forceinline__ int compact_flags(const uint8_t* __restrict__ flags, 
     const int p0 = tid * per, p1 = min(n, p0 + per);
     // the thread's flags are read once, all loads in flight together
     uint32_t mask = 0;
+    if (cols) {
 #pragma unroll 4
-    for (int j = 0; j < per; ++j)
-        if (p0 + j < p1) mask |= (uint32_t)((__ldcg(flags + p0 + j) != 0) & (cols ? __ldg(cols + p0 + j) : 1)) << j;
+        for (int j = 0; j < per; ++j)
+            if (p0 + j < p1) mask |= (uint32_t)((__ldcg(flags + p0 + j) != 0) & __ldg(cols + p0 + j)) << j;
+    } else {
+#pragma unroll 1
+        for (int j = 0; j < per; ++j)
+            if (p0 + j < p1) mask |= (uint32_t)(__ldcg(flags + p0 + j) != 0) << j;
+    }
     const int cntl = __popc(mask);
     int incl = cntl;
 #pragma unroll
