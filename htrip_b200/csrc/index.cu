@@ -213,6 +213,7 @@ inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 // for an event recorded after the previous one.  Each such grid takes every
 // SM, so running two at once gains nothing, and ordering them keeps two
 // grids that wait on their own CTAs from holding parts of the GPU at once.
+// (Two openings side by side are one link: their grids fit the GPU together.)
 // The host only takes a short lock; nothing waits on the host.
 constexpr int kCoopMaxDevices = 64;
 struct CoopChain {
@@ -832,7 +833,10 @@ void build_matrices(htrip_index* h, const BuildSet& bs, const uint8_t* obs, int 
         }
     }
     // leaves: bit-parallel BFS, then, for leaves with non-unit weights, the
-    // weighted adjacency closed over its passable cells
+    // weighted adjacency closed over its passable cells: padded order 64 in one
+    // kernel, larger ones by the general closure with a wait for its pivot counts (there is
+    // no kernel of their own; one weight changed on a 256 x 256 map, whole call: b = 8
+    // 375 us, b = 16 660, b = 32 1060)
     if (count(0))
         hb::launch_leaf_bfs(h->pass.p, h->S, h->b, h->leaves_x, count(0), h->L[0].ms(), st,
                             bs.all ? nullptr : reinterpret_cast<const int*>(ds + o_leaves));
@@ -1003,7 +1007,7 @@ void do_lift_root(htrip_index* h, const uint8_t* observed, int rows, int cols) {
 // and onBatchLeavesChanged, :507-527 with propagateBatchUpward, :427-505):
 // the listed leaves are rebuilt from the grid (leaf BFS) and every ancestor of
 // a rebuilt tile is rebuilt from its children's summaries and its seams
-// (node init + seams + closure), level by level up to the root.  Each rebuilt
+// (node_build.cu), level by level up to the root.  Each rebuilt
 // matrix is the unique closure of its region, so the index equals the one a
 // full build of the same grid gives on those tiles.
 // ---------------------------------------------------------------------------
@@ -1750,10 +1754,13 @@ int query_split_items(const htrip_index* h) {
 int query_seam_rows(const Level& Lv) { return 4 * Lv.nExt >= Lv.n; }
 
 // Levels lifted viewpoint by viewpoint (QueryParams::chain): from the leaves
-// up, matrices of padded order <= 1024 (a viewpoint's rows are at most 0.5 MB,
-// read by one CTA in a few microseconds) while a child holds at most about 4
-// viewpoints: with more, the tiled project items read a matrix row once for RW
-// viewpoints.
+// up, at most four, matrices of padded order <= 1024 (a viewpoint's rows are at most 0.5 MB,
+// read by one CTA in a few microseconds) while a child holds at most 4 viewpoints on
+// average: with more, the tiled project items read a matrix row once for RW viewpoints.
+// Query kernel in us, at most 0 (no chain) / 1 / 2 / 4 / 8 / 16 viewpoints a child: 512 x 512
+// maze, b = 8, k = 256: 115 / 84 / 84 / 76 / 76 / 76; 256 x 256 street map, b = 16, k = 128:
+// 78 / 70 / 64 / 64 / 59 / 59, k = 1024: 182 / 183 / 182 / 180 / 180 / 178.  Up to 2 / 3 / 4 levels,
+// 1024 x 1024 street map, b = 8, k = 256: 426 / 397 / 350.  Order up to 512 / 1024: 396 / 350 there.
 int query_chain(const htrip_index* h, int k) {
     int c = 0;
     while (c < std::min(h->H, hb::kMaxChain) && h->L[c + 1].NP <= hb::kMaxChainNP &&

@@ -154,7 +154,7 @@ __global__ void leaf_weight_init_kernel(const uint8_t* __restrict__ pass, const 
 // The same for leaves of padded order 64 (b <= 8), closed in place: Floyd-Warshall
 // over the passable cells on the whole matrix in shared memory, one CTA per
 // leaf (init, compaction and one closure round of three kernels took 72 us for one leaf,
-// this 13 us).
+// this 13 us).  Order 64 is what close_pivot_block's 256 threads hold.
 __global__ void __launch_bounds__(kThreads)
 leaf_weight_close_kernel(const uint8_t* __restrict__ pass, const uint16_t* __restrict__ wts, int S, int b, int leaves_x,
                          MatSet L, const int* __restrict__ list) {

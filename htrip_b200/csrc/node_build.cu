@@ -868,8 +868,10 @@ void launch_products(const NodeBuild& P, int n, cudaStream_t st) {
         <<<dim3(g2 * nt * (nt + 1) / 2 + g2 * (g2 - 1) / 2 * nt * nt, n), 32 * W * KS, smem, st>>>(P);
 }
 
-// Fewer 128 x 128 tiles than this leave SMs idle or with one CTA (8 warps), whose
-// latencies show.
+// Fewer 128 x 128 tiles than two per SM (148 of them) leave SMs idle or with one CTA (8 warps),
+// whose latencies show.  Whole builds, 128 x 128 tiles always / from one per SM / from two /
+// from four / never: 256 x 256, b = 8: 472 / 457 / 453 / 453 / 451 us; 512 x 512:
+// 1096 / 1097 / 1100 / 1134 / 1142; 1024 x 1024: 4729 / 4729 / 4731 / 4722 / 5440.
 constexpr size_t kWideTiles = 2 * 148;
 
 }  // namespace

@@ -24,10 +24,10 @@
 //            The lowest levels have few viewpoints per child (mostly one), so
 //            a tile of RW viewpoint rows is mostly padding there, and
 //            handing a level on to the next through L2 (fence, count, poll, flags)
-//            costs 7-10 us.  Measured, query kernel before and after (B200): 256 x 256
-//            street map, b = 16 (three of four levels in the chain), k = 2: 57 -> 41 us,
-//            k = 16: 62 -> 50 us; 512 x 512 maze, k = 256: 168 -> 123 us; 1000 x 1013
-//            street map, k = 509: 797 -> 655 us.  About half of a unit's time goes to
+//            costs 7-10 us.  Query kernel without and with a chain (B200): 256 x 256
+//            street map, b = 16 (three of four levels in the chain), k = 2: 59 -> 42 us,
+//            k = 16: 59 -> 46 us; 512 x 512 maze, b = 16, k = 256: 111 -> 74 us; 1024 x 1024
+//            street map, b = 8, k = 512: 661 -> 514 us.  About half of a unit's time goes to
 //            fetching its instructions (each CTA runs most of them once): loops here
 //            stay rolled, and a deeper copy ring measured slower.
 //   level 0  (no chain) X0[p][s] = leaf D[u][port p] for every viewpoint (+ finite-port
@@ -44,9 +44,10 @@
 //            X_{l-1} itself, which the epilogue takes for the child's own
 //            columns and the level below for its pairs.  At the root only
 //            seam columns are read, so tiles without one are left out.  The same
-//            holds in the chain and in meet.  Whole calls, all ports / seam ports:
-//            512 x 512 maze k = 256 199 -> 154 us, the same with corridors of 16 and
-//            k = 64 139 -> 103, 1000 x 1013 street map k = 509 666 -> 523.
+//            holds in the chain and in meet.  Query kernel, all ports / seam ports:
+//            512 x 512 maze, b = 16, k = 256 82 -> 72 us, 512 x 512 street map, k = 64
+//            102 -> 93, 1024 x 1024 street map, k = 509 631 -> 498.  Where nearly
+//            every port is on a seam all of them are rows (query_seam_rows, index.cu).
 //   meet     M[i][j] = min(M[i][j], min_p Yt_l[q_j*nP + p][i] (+) X_{l-1}[p][j])
 //            for i < j in one node: the inter-child meets (:1157-1326) and the
 //            intra-child shortcut (:1328-1411) are one formula.  Split-K items

@@ -408,8 +408,9 @@ htrip_status htrip_last_open_levels(const htrip_index* h, int64_t* out, int32_t 
 
 /* Phase trace of the last query launch of an index / a batch: ns[i] =
  * global-timer nanoseconds of phase i of the persistent query kernel
- * (0: level-0 gathers; 1..H+1: projections of level i with the meets of
- * level i-1; H+2: output).  Barrier schedule (HTRIP_QUERY_DATAFLOW=0): the
+ * (0: the lowest levels lifted viewpoint by viewpoint, or level-0 gathers;
+ * 1..H+1: projections of level i above those with the meets of level i-1;
+ * H+2: output).  Barrier schedule (HTRIP_QUERY_DATAFLOW=0): the
  * phase as its first CTA sees it; with max_n >= 2 * phases, ns[phases + i]
  * is the part of phase i until its last CTA finished its work (the rest is
  * the grid-barrier wait).  Dataflow schedule (default; phases overlap): the
