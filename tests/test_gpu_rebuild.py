@@ -178,7 +178,9 @@ def test_one_handle_built_again_and_again(gpu, b, g, sizes):
 @pytest.mark.parametrize("side,b,g", [(64, 4, 2), (96, 8, 2), (100, 9, 2), (128, 16, 2), (128, 32, 2), (54, 6, 3)])
 def test_leaves_and_weights_changed(gpu, side, b, g):
     """onBatchLeavesChanged (the parents to rebuild are chosen on the device),
-    onCellWeightChanged and onTileWeightsChanged against a build of the changed map."""
+    onCellWeightChanged and onTileWeightsChanged against a build of the changed map (the
+    two agree here; in general an unchanged exterior hides a changed seam higher up, as in
+    the reference)."""
     from htrip_b200.minplus_oracle import GridMap, HierarchyConfig, MinPlusOracle
     rng = np.random.default_rng(side + b)
     grid = make_grid("street", side, side, b)
